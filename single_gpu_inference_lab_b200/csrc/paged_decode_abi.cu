@@ -618,6 +618,37 @@ int decode_impl(const pfd_decode_args* args, int slot_offset, const GroupedRows*
   return bf16 ? launch_decode<64, true>(a, kp, num_splits) : launch_decode<64, false>(a, kp, num_splits);
 }
 
+int log2_or_none(int x) { return x > 0 && (x & (x - 1)) == 0 ? __builtin_ctz(static_cast<unsigned>(x)) : -1; }
+
+// Threads per token: as many as still let all CTAs of 256 threads run at once (four to an SM), which
+// gives a small call the shortest chains; beyond that a warp, which does the least work per token.
+// us at 256 / 128 / 64 / 32 threads per token, 28 + 4 heads of 128, FP8 cache, 148 SMs:
+//   512 tokens 4.1 / 4.2 / 5.4 / 7.7    1024: 6.2 / 5.5 / 6.2 / 7.9    2048: 10.2 / 8.8 / 8.6 / 8.9
+//   4096: 17.5 / 14.8 / 14.0 / 13.9     8192: 40.1 / 32.4 / 29.1 / 27.2 (28.4 as it stands)
+// A token's threads have to cover the rotation tasks of one head (16 elements each).
+constexpr int kRopeMaxRotary = 16 * 32;
+template <bool BF16, bool NEOX>
+cudaError_t launch_rope_vec(const pfd::RopeParams& p, int sms, cudaStream_t stream) {
+  const auto launch = [&](auto kernel, int threads_per_token) {
+    const int per_cta = pfd::kRopeThreads / threads_per_token;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(static_cast<unsigned>((p.num_tokens + per_cta - 1) / per_cta));
+    cfg.blockDim = dim3(pfd::kRopeThreads);
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, p);
+  };
+  const int64_t ctas = 4LL * sms;
+  if (p.num_tokens <= ctas) return launch(pfd::rope_quant_append_vec_kernel<BF16, NEOX, 256>, 256);
+  if (p.num_tokens <= 2 * ctas) return launch(pfd::rope_quant_append_vec_kernel<BF16, NEOX, 128>, 128);
+  if (p.num_tokens <= 4 * ctas) return launch(pfd::rope_quant_append_vec_kernel<BF16, NEOX, 64>, 64);
+  return launch(pfd::rope_quant_append_vec_kernel<BF16, NEOX, 32>, 32);
+}
+
 template <bool QBF16>
 int launch_prefix(const pfd_decode_args& a, int prefix_len, int chunks, bool suffix_beside,
                   const int32_t* groups = nullptr, int max_groups = 0) {
@@ -1037,12 +1068,16 @@ int pfd_rope_quant_append(const pfd_rope_args* args) {
   p.is_neox = a.is_neox ? 1 : 0;
   p.cos_sin_f32 = a.cos_sin_dtype == PFD_DTYPE_F32 ? 1 : 0;
   p.cache_fp8 = a.cache_dtype == PFD_DTYPE_E4M3 ? 1 : 0;
+  p.block_shift = log2_or_none(a.block_size);
+  p.chunk_shift = log2_or_none(a.head_dim / 8);
+  p.task_shift = log2_or_none(a.rotary_dim / 16);
+  p.neg_zeros = 0x8000000080000000ull;
   cudaStream_t stream = static_cast<cudaStream_t>(a.stream);
-  // The vectorised kernel: NeoX pairs over the whole head, rows and caches 16-byte aligned.
+  // The kernel of 16-byte chunks: rotary_dim a multiple of 16, rows and caches aligned for it.
   const auto al = [](const void* ptr, int64_t bytes) { return (reinterpret_cast<uintptr_t>(ptr) & (uintptr_t)(bytes - 1)) == 0; };
   const auto m8 = [](int64_t x) { return x % 8 == 0; };
   const int cache_elem = p.cache_fp8 ? 1 : 2;
-  const bool vec = p.is_neox && a.rotary_dim == a.head_dim && a.head_dim % 16 == 0 &&
+  const bool vec = a.rotary_dim % 16 == 0 && a.rotary_dim <= kRopeMaxRotary && a.head_dim % 8 == 0 &&
                    al(a.query, 16) && al(a.key, 16) && al(a.value, 16) && al(a.cos_sin_cache, 16) &&
                    m8(a.q_stride_t) && m8(a.q_stride_h) && m8(a.k_stride_t) && m8(a.k_stride_h) && m8(a.v_stride_t) &&
                    m8(a.v_stride_h) && (p.cos_sin_f32 ? a.cos_sin_stride % 4 == 0 : m8(a.cos_sin_stride)) &&
@@ -1050,8 +1085,12 @@ int pfd_rope_quant_append(const pfd_rope_args* args) {
                    m8(a.kc_stride_token) && m8(a.kc_stride_head) && m8(a.vc_stride_block) && m8(a.vc_stride_token) &&
                    m8(a.vc_stride_head);
   if (vec) {
-    if (a.query_dtype == PFD_DTYPE_BF16) pfd::rope_quant_append_vec_kernel<true><<<a.num_tokens, 256, 0, stream>>>(p);
-    else pfd::rope_quant_append_vec_kernel<false><<<a.num_tokens, 256, 0, stream>>>(p);
+    if (int rc = enter_call()) return rc;
+    const int sms = t_device->sms;
+    const bool bf16 = a.query_dtype == PFD_DTYPE_BF16;
+    const cudaError_t e = p.is_neox ? (bf16 ? launch_rope_vec<true, true>(p, sms, stream) : launch_rope_vec<false, true>(p, sms, stream))
+                                    : (bf16 ? launch_rope_vec<true, false>(p, sms, stream) : launch_rope_vec<false, false>(p, sms, stream));
+    if (e != cudaSuccess) return fail(PFD_ERR_CUDA, "rope + append kernel (vectorised) launch failed: %s", cudaGetErrorString(e));
     return check_launch("rope + append kernel (vectorised)");
   }
   if (a.query_dtype == PFD_DTYPE_BF16) pfd::rope_quant_append_kernel<true><<<a.num_tokens, 256, 0, stream>>>(p);

@@ -222,3 +222,40 @@ def test_wrapper_argument_errors_without_a_gpu():
         l20_rope_kv.l20_rope_and_cache(q, q, q, torch.zeros(2, dtype=torch.long), torch.zeros(8, 128), True,
                                        torch.zeros(1, 16, 4, 128, dtype=torch.bfloat16),
                                        torch.zeros(1, 16, 4, 128, dtype=torch.bfloat16), torch.zeros(2, dtype=torch.long))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("is_neox", [True, False])
+@pytest.mark.parametrize("cache", ["same", "fp8"])
+def test_chunk_kernel_edges_bit_for_bit(built_libs, is_neox, cache):
+    """The kernel of 16-byte chunks where it can go wrong: every number of threads per token with a ragged last CTA,
+    partial rotation, frequency groups that do not divide a token's threads, more heads than the threads take at once,
+    scales that are powers of two (ties) and that are not; and rotary_dim 24, which the scalar kernel takes."""
+    from single_gpu_inference_lab_b200 import l20_rope_kv
+
+    for seed, (tokens, hq, hkv, d, rot, dtype, table_dtype) in enumerate([
+        (256, 5, 1, 128, 64, torch.bfloat16, torch.float32),
+        (257, 28, 4, 128, 128, torch.bfloat16, torch.bfloat16),
+        (1027, 3, 3, 80, 48, torch.float16, torch.float32),
+        (1030, 40, 8, 64, 16, torch.bfloat16, torch.float32),
+        (2, 71, 9, 128, 96, torch.float16, torch.float16),
+        (1201, 16, 2, 128, 128, torch.bfloat16, torch.float32),
+        (2401, 6, 2, 64, 64, torch.float16, torch.float32),
+        (301, 14, 2, 256, 256, torch.bfloat16, torch.float32),
+        (300, 4, 2, 64, 24, torch.bfloat16, torch.float32),
+    ]):
+        cache_dtype = torch.float8_e4m3fn if cache == "fp8" else dtype
+        q, k, v, pos, cs, kc, vc, slots, ks, vs = make_step(100 + seed, tokens, hq, hkv, d, rot, dtype, cache_dtype, table_dtype)
+        if ks is not None and seed % 2:
+            ks, vs = torch.full_like(ks, 0.25), torch.full_like(vs, 2.0)
+        want = oracle.rope_and_cache(q, k, v, pos, cs, is_neox, kc, vc, slots, ks, vs)
+        # rows of one projection output, as an engine hands them on
+        rows = torch.cat([q, k, v], 1).to(DEV)
+        gq, gk, gv = rows[:, :hq], rows[:, hq:hq + hkv], rows[:, hq + hkv:]
+        gkc, gvc = kc.to(DEV), vc.to(DEV)
+        l20_rope_kv.l20_rope_and_cache(gq, gk, gv, pos.to(DEV), cs.to(DEV), is_neox, gkc, gvc, slots.to(DEV),
+                                       k_scale=None if ks is None else ks.to(DEV), v_scale=None if vs is None else vs.to(DEV))
+        as_bytes = lambda t: t.cpu().contiguous().view(torch.uint8)
+        for name, got, exp in zip(("query", "key", "key cache", "value cache"), (gq, gk, gkc, gvc), want):
+            assert torch.equal(as_bytes(got), as_bytes(exp)), f"{name}: case {seed} neox={is_neox} cache={cache}"
+        assert torch.equal(as_bytes(gv), as_bytes(v))
