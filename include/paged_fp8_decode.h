@@ -370,8 +370,10 @@ int pfd_group_shared_prefixes(const int32_t* block_table, int64_t bt_stride_b, i
  * max_seq_len); what lies beyond goes through the split-KV pass, so any bound is safe and a
  * tight one saves idle CTAs.  Every member of a group must be at least as long as the group's
  * prefix.  max_suffix_len bounds what a request IN a group has behind its prefix (0 = unknown: the
- * whole context); the split-KV grid is sized for it, ceil(max_suffix_len / split_size) splits, and
- * a request in no group covers its whole context with as many, longer, splits.  A member whose
+ * whole context); the split-KV grid is sized for it, ceil(max_suffix_len / split_size) splits.  A
+ * request in no group covers its whole context with as many splits as all its slots allow, of 256
+ * tokens or more, taken by CTAs of their own (under PFD_FLAG_ALL_IN_GROUPS, or with a cache that TMA
+ * cannot describe: with as many splits as the others' suffixes, longer ones).  A member whose
  * suffix exceeds the bound would be attended only up to it (device status 5 reports it): give a true bound (max_seq_len minus
  * the smallest prefix a group can have, i.e. the min_prefix_len of the grouping call).  The
  * workspace needs ceil(min(max_prefix_len, max_seq_len) / 256) +

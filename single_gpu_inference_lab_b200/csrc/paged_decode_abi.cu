@@ -228,7 +228,7 @@ bool tma_eligible(const pfd_decode_args& a) {
 
 // kWarpsT = 2, kStagesT = 1 beside the dense prefix pass: two CTAs of two warps, 165 registers
 // and 18 KB fit on an SM next to a CTA of the slim prefix kernel (see suffix_beside_prefix).
-template <bool QBF16, int kWarpsT = kWarps, int kStagesT = kStages>
+template <bool QBF16, int kWarpsT = kWarps, int kStagesT = kStages, bool LONERS = false>
 int launch_partial_tma(const pfd_decode_args& a, const pfd::KernelParams& kp, dim3 grid, cudaStream_t stream) {
   CUtensorMap mk, mv;
   if (int rc = get_tensor_map(a.key_cache, a.k_stride_page, a.k_stride_token, a.k_stride_head, a.num_pages,
@@ -241,8 +241,9 @@ int launch_partial_tma(const pfd_decode_args& a, const pfd::KernelParams& kp, di
   tp.head_is_dim1 = head_is_dim1(a.k_stride_token, a.k_stride_head) ? 1 : 0;
   if (int rc = status_pointer(&tp.status)) return rc;
   tp.wait_limit_ns = g_wait_limit_ns.load(std::memory_order_relaxed);
-  auto kernel = pfd::paged_decode_fp8_partial_tma_kernel<QBF16, kWarpsT, kStagesT>;
-  constexpr int smem = 1024 + kWarpsT * kStagesT * 8192 + kWarpsT * kStagesT * 8 + 2 * kWarpsT * 16 * 4;
+  auto kernel = pfd::paged_decode_fp8_partial_tma_kernel<QBF16, kWarpsT, kStagesT, LONERS>;
+  constexpr int smem = 1024 + kWarpsT * kStagesT * 8192 + kWarpsT * kStagesT * 8 + 2 * kWarpsT * 16 * 4 +
+                       (LONERS ? kWarpsT * 4 + pfd::kGroupedMaxBatch * 2 : 0);
   static std::atomic<bool> configured[kMaxDevices];  // (one array per instantiation)
   if (int rc = configure_smem(configured, kernel, smem, kWarpsT != kWarps)) return rc;
   {
@@ -431,7 +432,9 @@ int launch_decode(const pfd_decode_args& a, const pfd::KernelParams& kp, int num
   const dim3 grid(num_splits, a.num_kv_heads, a.batch);
   if (D == 128 && tma_eligible(a)) {
     g_last_path = PFD_PATH_FIXED_TMA;
-    if (int rc = suffix_beside_prefix(a, kp.slot_offset, num_splits, kp.row_kv_start != nullptr)
+    const dim3 grid_with_loners(num_splits, a.num_kv_heads, a.batch + kp.loner_rows);
+    if (int rc = kp.loner_rows > 0 ? launch_partial_tma<QBF16, kWarps, kStages, true>(a, kp, grid_with_loners, stream)
+                 : suffix_beside_prefix(a, kp.slot_offset, num_splits, kp.row_kv_start != nullptr)
                      ? launch_partial_tma<QBF16, 2, 1>(a, kp, grid, stream)
                      : launch_partial_tma<QBF16>(a, kp, grid, stream))
       return rc;
@@ -457,8 +460,12 @@ int launch_decode(const pfd_decode_args& a, const pfd::KernelParams& kp, int num
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     const int batch = a.batch;
-    const cudaError_t e = wide ? cudaLaunchKernelEx(&cfg, pfd::paged_decode_merge_kernel<D, QBF16, 4>, kp, batch)
-                               : cudaLaunchKernelEx(&cfg, pfd::paged_decode_merge_kernel<D, QBF16, 1>, kp, batch);
+    auto kernel = wide ? pfd::paged_decode_merge_kernel<D, QBF16, 4, false> : pfd::paged_decode_merge_kernel<D, QBF16, 1, false>;
+    if constexpr (D == 128) {  // (a grouped decode has head_dim 128)
+      if (kp.row_kv_start != nullptr)
+        kernel = wide ? pfd::paged_decode_merge_kernel<D, QBF16, 4, true> : pfd::paged_decode_merge_kernel<D, QBF16, 1, true>;
+    }
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, kp, batch);
     if (e != cudaSuccess) return fail(PFD_ERR_CUDA, "merge kernel launch failed: %s", cudaGetErrorString(e));
     if (int rc = check_launch("merge kernel")) return rc;
   }
@@ -478,6 +485,8 @@ int64_t pfd_launch_count(void) { return g_launches.load(std::memory_order_relaxe
 }  // extern "C"
 
 namespace {
+constexpr int kLonerSplit = 256;  // tokens of a request in no group to an item, at least (two page pairs for each of four warps)
+static_assert(pfd::kGroupedMaxBatch == pfd::kGroupsMaxBatch, "batch of a grouped decode");
 // What the grouped shared-prefix entry adds to a split-KV pass: per-request attend starts read on
 // the device, their cap, the split size of requests in no group, and the grid's split count.
 struct GroupedRows {
@@ -485,6 +494,8 @@ struct GroupedRows {
   int row_kv_cap = 0;
   int split_size_loner = 0;
   int num_splits = 0;
+  int loner_rows = 0, loner_splits = 0, loner_share = 0;  // see pfd::KernelParams
+  const int32_t* grouped_count = nullptr;
 };
 
 pfd::KernelParams fill_params(const pfd_decode_args& a, int group, bool direct_ok, int slot_offset,
@@ -522,6 +533,12 @@ pfd::KernelParams fill_params(const pfd_decode_args& a, int group, bool direct_o
     kp.row_kv_start = grouped->row_kv_start;
     kp.row_kv_cap = grouped->row_kv_cap;
     kp.split_size_loner = grouped->split_size_loner;
+    kp.loner_rows = grouped->loner_rows;
+    kp.loner_grid_row = grouped->num_splits * a.num_kv_heads;
+    kp.loner_splits = grouped->loner_splits;
+    kp.loner_share = grouped->loner_share;
+    kp.grouped_count = grouped->grouped_count;
+    kp.batch = a.batch;
   }
   kp.early_metadata = (a.flags & PFD_FLAG_EARLY_METADATA) ? 1 : 0;
   kp.early_kv = (kp.early_metadata && (a.flags & PFD_FLAG_EARLY_KV)) ? 1 : 0;
@@ -957,6 +974,17 @@ int pfd_shared_prefix_decode_grouped_fp8_e4m3(const pfd_decode_args* args, const
   rows.row_kv_start = g + pfd::groups_row_prefix_off();
   rows.row_kv_cap = cap;
   rows.split_size_loner = split_loner;
+  if (tma_eligible(a) && !(a.flags & PFD_FLAG_ALL_IN_GROUPS)) {
+    // Requests in no group get CTAs of their own, one wave of them, and all the slots of their rows
+    // (chunks + ns: the prefix chunks are none of theirs), kLonerSplit tokens or more to a slot.
+    const int slots = chunks + ns;
+    rows.split_size_loner = std::max(((a.max_seq_len + slots - 1) / slots + 15) / 16 * 16, kLonerSplit);
+    rows.loner_splits = std::max((a.max_seq_len + rows.split_size_loner - 1) / rows.split_size_loner, 1);
+    rows.loner_rows = (3 * t_device->sms + ns * a.num_kv_heads - 1) / (ns * a.num_kv_heads);
+    const int64_t ctas = (int64_t)rows.loner_rows * ns * a.num_kv_heads;
+    rows.loner_share = static_cast<int>(std::min<int64_t>(a.max_seq_len * (int64_t)a.num_kv_heads / ctas, 1 << 19));
+    rows.grouped_count = g + 4;
+  }
   rows.num_splits = ns;
   return decode_impl(&a, chunks, &rows);
 }

@@ -26,6 +26,7 @@
 namespace pfd {
 
 constexpr int kPage = 16;
+constexpr int kGroupedMaxBatch = 2048;  // requests of a grouped shared-prefix decode
 constexpr float kLog2e = 1.4426950408889634f;
 constexpr float kLn2 = 0.6931471805599453f;
 
@@ -61,6 +62,13 @@ struct KernelParams {
   const int32_t* row_kv_start;
   int32_t row_kv_cap;  // upper bound applied to row_kv_start (a multiple of 16): the slots in front cover no more
   int32_t split_size_loner;  // grouped decode: split size of a request in no group (it attends from 0); 0 = split_size
+  // Grouped decode, requests in no group shared out over CTAs of their own (loner_rows > 0): that many
+  // grid rows in front of the batch's take their (request, kv head, split) items in turns, at most
+  // loner_splits to a request, of split_size_loner tokens or more (split_size_of); their partials fill
+  // the request's slots from 0 on, since it has no prefix chunks.
+  // (loner_grid_row: CTAs of one grid row; loner_share: tokens of one such request, as long as any, for each of those CTAs)
+  int32_t loner_rows, loner_grid_row, loner_splits, loner_share, batch;
+  const int32_t* grouped_count;  // device word: requests of the batch that are in groups
   int32_t early_metadata;  // 1: seq_lens and block_table may be read before the preceding kernel has completed
   int32_t early_kv;        // 1: so may K/V pages, except each sequence's last (balanced kernel with a plan)
   int32_t kv_evict_first;  // 1: K/V tiles are loaded with the L2 evict-first hint
@@ -122,10 +130,14 @@ __device__ __forceinline__ int kv_start_of(const KernelParams& p, int b) {
   return p.row_kv_start != nullptr ? min(__ldg(p.row_kv_start + b) & ~15, p.row_kv_cap) : p.kv_start;
 }
 
-// Split size of sequence b, whose first attended token is kv0: in a grouped decode a request in
-// no group has the whole context to cover with the same number of splits as the others' suffixes.
+// Split size of a sequence whose first attended token is kv0: in a grouped decode a request in no
+// group has the whole context to cover.  Shared out over CTAs of their own, such requests get as many
+// items as those CTAs can take at once, of no less than the size that their slots allow.
 __device__ __forceinline__ int split_size_of(const KernelParams& p, int kv0) {
-  return (p.row_kv_start != nullptr && kv0 == 0 && p.split_size_loner > 0) ? p.split_size_loner : p.split_size;
+  if (p.row_kv_start == nullptr || kv0 != 0 || p.split_size_loner <= 0) return p.split_size;
+  if (p.loner_rows == 0) return p.split_size_loner;
+  const int loners = p.batch - __ldg(p.grouped_count);
+  return max(p.split_size_loner, (loners * p.loner_share + 63) & ~63);
 }
 
 __device__ __forceinline__ int32_t page_of(const int32_t* __restrict__ block_table,
@@ -409,7 +421,7 @@ __device__ __forceinline__ void store_out_elem4(void* base, int64_t idx, float4 
 //   sm_m/sm_l : [NWARPS][16], sm_o : [NWARPS][16][D] floats.
 template <int D, bool QBF16, int NWARPS>
 __device__ __forceinline__ void cta_merge_and_store(WarpState<D>& st, const KernelParams& p, int b,
-                                                    int kvh, int split, int nsplits_seq,
+                                                    int kvh, int slot, int nsplits_seq,
                                                     float v_scale, float* sm_m, float* sm_l,
                                                     float* sm_o) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, i = lane >> 2, j = lane & 3;
@@ -486,7 +498,7 @@ __device__ __forceinline__ void cta_merge_and_store(WarpState<D>& st, const Kern
       }
     } else {
       const int64_t pidx = (int64_t)b * p.partial_stride_b + (int64_t)hq * p.partial_stride_h +
-                           (int64_t)(split + p.slot_offset) * p.partial_stride_s;
+                           (int64_t)slot * p.partial_stride_s;
       store_partial_elem4(p.partial_output, p.partial_dtype, pidx * D + c4, acc);
       if (c4 == 0) {
         p.partial_max[pidx] = big_row * kLn2;
@@ -570,7 +582,7 @@ paged_decode_fp8_partial_ldg_kernel(const KernelParams p) {
     consume_tile<D>(st, cur, qa, scale_log2, pg * kPage, lo, hi, j);
     cur = nxt;
   }
-  cta_merge_and_store<D, QBF16, NWARPS>(st, p, b, kvh, split, nsplits_seq, vs, sm_m, sm_l, sm_o);
+  cta_merge_and_store<D, QBF16, NWARPS>(st, p, b, kvh, split + p.slot_offset, nsplits_seq, vs, sm_m, sm_l, sm_o);
   pdl_wait();  // see the TMA kernel
 }
 
@@ -753,7 +765,14 @@ __global__ void bounded_wait_selftest_kernel(int32_t* status, unsigned long long
 // each other inside the loop, and the bytes in flight do not cost registers.  Two pages per
 // step give four independent QK^T accumulator chains and halve the per-token cost of the
 // softmax bookkeeping (shuffles, rescale).
-template <bool QBF16, int NWARPS, int NSTAGE>
+//
+// LONERS: a grouped shared-prefix decode whose requests in no group are shared out over CTAs of
+// their own (KernelParams::loner_rows).  A request in no group has some ten times the tokens of
+// another's suffix; cut into as many splits as those, it is one chain of a dozen page pairs per
+// warp that the whole step waits for: with 64 requests, two groups behind 4096 and 5120 tokens and 8
+// requests of 4.3 K tokens in none, 2 kv heads, this pass took 29 us and a step of eight layers
+// 357 us that way, and 260 us with 256 tokens to an item (128: 260, 512: 266).
+template <bool QBF16, int NWARPS, int NSTAGE, bool LONERS = false>
 __global__ void __launch_bounds__(NWARPS * 32, NWARPS <= 12 ? 12 / NWARPS : 1)  // twelve warps per SM: at most 168 registers
 paged_decode_fp8_partial_tma_kernel(const KernelParams p, const TmaParams tp,
                                     const __grid_constant__ CUtensorMap tmap_k,
@@ -774,8 +793,71 @@ paged_decode_fp8_partial_tma_kernel(const KernelParams p, const TmaParams tp,
   // With early_metadata the caller vouches that seq_lens and block_table are not written by
   // that kernel: their reads below are then allowed to come first.
   if (p.slot_offset == 0 && !p.early_metadata) pdl_wait();
-  const int split = blockIdx.x, kvh = blockIdx.y, b = blockIdx.z;
+  int split = blockIdx.x, kvh = blockIdx.y, b = blockIdx.z;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, i = lane >> 2, j = lane & 3;
+  // A CTA of the rows in front takes the items of the requests in no group in turns: item
+  // (request, kv head, split) number blockIdx, + CTAs of those rows, ...; the others have one item.
+  int item = 0, n_items = 0;
+  const bool takes_turns = LONERS && (int)blockIdx.z < p.loner_rows;
+  extern __shared__ uint8_t smem_raw[];
+  const uint32_t ring = (smem_u32(smem_raw) + 1023u) & ~1023u;
+  uint8_t* ring_ptr = smem_raw + (ring - smem_u32(smem_raw));
+  // after the ring: mbarriers, then the small merge arrays; sm_o aliases the ring at the end
+  const uint32_t bars = ring + NWARPS * NSTAGE * kStageBytes;
+  float* sm_m = reinterpret_cast<float*>(ring_ptr + NWARPS * NSTAGE * kStageBytes + NWARPS * NSTAGE * 8);
+  float* sm_l = sm_m + NWARPS * 16;
+  float* sm_o = reinterpret_cast<float*>(ring_ptr);
+  static_assert(NSTAGE * kStageBytes >= 16 * D * 4, "merge buffer must fit in the ring");
+  // LONERS only: counts of the scan below, then the requests in no group, ascending
+  int* sm_count = reinterpret_cast<int*>(sm_l + NWARPS * 16);
+  uint16_t* sm_loners = reinterpret_cast<uint16_t*>(sm_count + NWARPS);
+  if constexpr (LONERS) {
+    if (takes_turns) {
+      int n_loners = 0;
+      for (int b0 = 0; b0 < p.batch; b0 += NWARPS * 32) {
+        const int r = b0 + (int)threadIdx.x;
+        const bool mine = r < p.batch && kv_start_of(p, r) == 0;
+        const unsigned votes = __ballot_sync(0xffffffffu, mine);
+        if (lane == 0) sm_count[warp] = __popc(votes);
+        __syncthreads();
+        int before = n_loners;
+        for (int w = 0; w < NWARPS; ++w) {
+          if (w < warp) before += sm_count[w];
+          n_loners += sm_count[w];
+        }
+        if (mine) sm_loners[before + __popc(votes & ((1u << lane) - 1u))] = (uint16_t)r;
+        __syncthreads();
+      }
+      n_items = n_loners * p.num_kv_heads * p.loner_splits;
+      item = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z);
+    } else {
+      b -= p.loner_rows;
+    }
+  }
+  // Behind the dense prefix pass (slot_offset > 0) this grid reads nothing of that pass, but it must
+  // not COMPLETE before it: the merge kernel waits for this grid only.  One CTA that waits before
+  // it exits is enough for that, and the others give their place on the SM to the next CTA.
+  const bool waits_at_exit = p.slot_offset == 0 || (blockIdx.x | blockIdx.y | blockIdx.z) == 0;
+  int tbase = 0;  // page pairs that went through this warp's ring for earlier items
+  bool ok = true;
+  for (bool first_item = true;; first_item = false) {
+  if constexpr (LONERS) {
+    if (takes_turns) {
+      // splits of a request side by side; those behind its end are passed over
+      for (;; item += p.loner_rows * p.loner_grid_row) {
+        if (item >= n_items) break;
+        split = item % p.loner_splits;
+        const int rest = item / p.loner_splits;
+        kvh = rest % p.num_kv_heads;
+        b = sm_loners[rest / p.num_kv_heads];
+        if (split * split_size_of(p, 0) < p.seq_lens[b]) break;
+      }
+      if (item >= n_items) {
+        if (waits_at_exit) pdl_wait();
+        return;
+      }
+    }
+  }
   const int kv0 = kv_start_of(p, b);
   const int split_sz = split_size_of(p, kv0);
   const int lo = kv0 + split * split_sz;
@@ -794,14 +876,11 @@ paged_decode_fp8_partial_tma_kernel(const KernelParams p, const TmaParams tp,
   const int hi = min(lo + split_sz, seq_len);
   // grouped decode: the grid was sized from the caller's bound on the suffixes; a request that
   // needs more splits than the grid has would lose its tail silently, so it is reported instead
-  if (p.row_kv_start != nullptr && split == 0 && kvh == 0 && threadIdx.x == 0 &&
-      seq_len - kv0 > (int)gridDim.x * split_sz)
+  const bool not_mine = LONERS && !takes_turns && kv0 == 0;  // a request in no group
+  if (p.row_kv_start != nullptr && !not_mine && split == 0 && kvh == 0 && threadIdx.x == 0 &&
+      seq_len - kv0 > (takes_turns ? p.loner_splits : (int)gridDim.x) * (int64_t)split_sz)
     atomicExch(tp.status, kErrSuffixBound);
-  // Behind the dense prefix pass (slot_offset > 0) this grid reads nothing of that pass, but it must
-  // not COMPLETE before it: the merge kernel waits for this grid only.  One CTA that waits before
-  // it exits is enough for that, and the others give their place on the SM to the next CTA.
-  const bool waits_at_exit = p.slot_offset == 0 || (blockIdx.x | blockIdx.y | blockIdx.z) == 0;
-  if (lo >= hi) {
+  if (lo >= hi || not_mine) {
     if (waits_at_exit) pdl_wait();
     if (split == 0 && gridDim.x == 1 && p.direct_out) write_empty_rows<D>(p, b, kvh);
     return;
@@ -810,19 +889,9 @@ paged_decode_fp8_partial_tma_kernel(const KernelParams p, const TmaParams tp,
   dbg_mark(dbg_slot, 6, threadIdx.x == 0);  // sequence length known
   const int nsplits_seq = (seq_len - kv0 + split_sz - 1) / split_sz;
 
-  extern __shared__ uint8_t smem_raw[];
-  const uint32_t ring = (smem_u32(smem_raw) + 1023u) & ~1023u;
-  uint8_t* ring_ptr = smem_raw + (ring - smem_u32(smem_raw));
-  // after the ring: mbarriers, then the small merge arrays; sm_o aliases the ring at the end
-  const uint32_t bars = ring + NWARPS * NSTAGE * kStageBytes;
-  float* sm_m = reinterpret_cast<float*>(ring_ptr + NWARPS * NSTAGE * kStageBytes + NWARPS * NSTAGE * 8);
-  float* sm_l = sm_m + NWARPS * 16;
-  float* sm_o = reinterpret_cast<float*>(ring_ptr);
-  static_assert(NSTAGE * kStageBytes >= 16 * D * 4, "merge buffer must fit in the ring");
-
   const uint32_t my_ring = ring + warp * NSTAGE * kStageBytes;
   const uint32_t my_bars = bars + warp * NSTAGE * 8;
-  if (lane == 0) {
+  if (first_item && lane == 0) {
 #pragma unroll
     for (int s = 0; s < NSTAGE; ++s) mbar_init(my_bars + 8 * s, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -835,7 +904,7 @@ paged_decode_fp8_partial_tma_kernel(const KernelParams p, const TmaParams tp,
   const int n_pairs = (n_pairs_cta - warp + NWARPS - 1) / NWARPS;  // pairs warp, warp+NWARPS, ...
 
   auto issue = [&](int t, int32_t phys0, int32_t phys1) {  // lane 0 only
-    const int s = t % NSTAGE;
+    const int s = (tbase + t) % NSTAGE;
     const uint32_t bar = my_bars + 8 * s;
     const uint32_t dst = my_ring + s * kStageBytes;
     const bool two = my_page(t, 1) <= page_last;
@@ -892,11 +961,10 @@ paged_decode_fp8_partial_tma_kernel(const KernelParams p, const TmaParams tp,
     v_off[r] = row * D + ((i ^ (row & 7)) << 4);
   }
 
-  bool ok = true;
   int t = 0;
   for (; t < n_pairs; ++t) {
-    const int s = t % NSTAGE;
-    const uint32_t parity = (t / NSTAGE) & 1;
+    const int s = (tbase + t) % NSTAGE;
+    const uint32_t parity = ((tbase + t) / NSTAGE) & 1;
     if (!mbar_wait_bounded(my_bars + 8 * s, parity, tp.wait_limit_ns)) { ok = false; break; }
     if (t == 0) dbg_mark(dbg_slot, 4, threadIdx.x == 0);  // first pair arrived
     const uint32_t stage = my_ring + s * kStageBytes;
@@ -954,13 +1022,21 @@ paged_decode_fp8_partial_tma_kernel(const KernelParams p, const TmaParams tp,
     if (lane == 0) {
       atomicExch(tp.status, kErrTmaTimeout);
       const int issued = min(n_pairs, t + NSTAGE);
-      for (int u = t + 1; u < issued; ++u) mbar_wait_bounded(my_bars + 8 * (u % NSTAGE), (u / NSTAGE) & 1, tp.wait_limit_ns);
+      for (int u = t + 1; u < issued; ++u) mbar_wait_bounded(my_bars + 8 * ((tbase + u) % NSTAGE), ((tbase + u) / NSTAGE) & 1, tp.wait_limit_ns);
     }
     __syncwarp();
   }
   __syncthreads();  // every warp is done with its ring: sm_o may alias it
-  cta_merge_and_store<D, QBF16, NWARPS>(st, p, b, kvh, split, nsplits_seq, vs, sm_m, sm_l, sm_o);
+  cta_merge_and_store<D, QBF16, NWARPS>(st, p, b, kvh, takes_turns ? split : split + p.slot_offset, nsplits_seq, vs, sm_m,
+                                        sm_l, sm_o);
   dbg_mark(dbg_slot, 1, threadIdx.x == 0);
+  if (!takes_turns) break;
+  tbase += n_pairs;
+  item += p.loner_rows * p.loner_grid_row;
+  // the next item's copies and merge reuse what the merge above reads (no next item after a copy that never landed)
+  if (__syncthreads_or(!ok)) break;
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  }
   // (see waits_at_exit; a no-op for an ordinary launch, which has waited before its first access)
   if (waits_at_exit) pdl_wait();
   dbg_mark(dbg_slot, 2, threadIdx.x == 0);
@@ -970,8 +1046,11 @@ paged_decode_fp8_partial_tma_kernel(const KernelParams p, const TmaParams tp,
 // rows per CTA; WPR = 4 (few rows, many splits): the four warps of a CTA share one row, warp w
 // taking splits w, w + 4, ..., and combine through shared memory.
 // Same maths as _paged_split_kv_reduce (integrations/vllm/l20_paged_split_kv.py:459-488).
-template <int D, bool QBF16, int WPR = 1>
-__global__ void __launch_bounds__(128)
+// GROUPED: rows start where their group's prefix ends (KernelParams::row_kv_start).  An instantiation of
+// its own because it needs more registers: at 72 or less seven CTAs fit an SM, and the 1024 rows of a
+// batch of 64 with 16 heads are resident together (at 75: 18.7 instead of 17.9 us a shared-prefix layer).
+template <int D, bool QBF16, int WPR, bool GROUPED>
+__global__ void __launch_bounds__(128, WPR == 4 ? 7 : 1)
 paged_decode_merge_kernel(const KernelParams p, int batch) {
   static_assert(WPR == 1 || WPR == 4, "one or four warps per row");
   pdl_launch_dependents();
@@ -990,12 +1069,13 @@ paged_decode_merge_kernel(const KernelParams p, int batch) {
   }
   const int b = row / p.num_q_heads, hq = row % p.num_q_heads;
   const int seq_len = p.seq_lens[b];
-  const int kv0 = kv_start_of(p, b);
+  const int kv0 = GROUPED ? kv_start_of(p, b) : p.kv_start;
   const int live = seq_len - kv0;
   // slots in front of the splits: all slot_offset of them, or (grouped) those of this row's prefix
-  const int pre = p.row_kv_start != nullptr ? (kv0 + 255) / 256 : p.slot_offset;
-  const int skip = p.slot_offset - pre;  // unused slots between the row's prefix chunks and its splits
-  const int split_sz = split_size_of(p, kv0);
+  const int pre = GROUPED ? (kv0 + 255) / 256 : p.slot_offset;
+  // unused slots between the row's prefix chunks and its splits
+  const int skip = !GROUPED || (p.loner_rows > 0 && kv0 == 0) ? 0 : p.slot_offset - pre;
+  const int split_sz = GROUPED ? split_size_of(p, kv0) : p.split_size;
   const int ns = (live > 0 ? (live + split_sz - 1) / split_sz : 0) + pre;
   constexpr int E = D / 32;  // elements per lane
   float acc[E];
@@ -1010,6 +1090,10 @@ paged_decode_merge_kernel(const KernelParams p, int batch) {
   dbg_mark(4096 + blockIdx.x, 1, threadIdx.x == 0);
   if (ns > 0) {
     const int64_t base = (int64_t)b * p.partial_stride_b + (int64_t)hq * p.partial_stride_h;
+    const float* const row_max = p.partial_max + base;
+    const float* const row_sum = p.partial_sum + base;
+    // (32 bits: a slot that lies 2^31 rows off would be beyond any memory, rows being 128 bytes or more)
+    const int32_t stride = (int32_t)p.partial_stride_s;
     // One pass with a running maximum; eight splits per round trip, their maxima, sums and data
     // requested together.
     for (int s0 = part; s0 < ns; s0 += 8 * WPR) {
@@ -1018,11 +1102,11 @@ paged_decode_merge_kernel(const KernelParams p, int batch) {
       for (int u = 0; u < 8; ++u) {
         const bool on = s0 + u * WPR < ns;
         const int k = on ? s0 + u * WPR : 0;  // (an idle lane re-reads the row's first live slot: finite data, weight 0)
-        const int64_t pidx = base + (int64_t)(k < pre ? k : k + skip) * p.partial_stride_s;
-        mv[u] = on ? p.partial_max[pidx] : -INFINITY;
-        lv[u] = on ? p.partial_sum[pidx] : 0.f;
+        const int32_t slot = (!GROUPED || k < pre ? k : k + skip) * stride;
+        mv[u] = on ? row_max[slot] : -INFINITY;
+        lv[u] = on ? row_sum[slot] : 0.f;
         if (p.partial_dtype == 0) {
-          const float* src = reinterpret_cast<const float*>(p.partial_output) + pidx * D + lane * E;
+          const float* src = reinterpret_cast<const float*>(p.partial_output) + (base + slot) * D + lane * E;
           if constexpr (E == 4) {
             const float4 x = *reinterpret_cast<const float4*>(src);
             xv[u][0] = x.x; xv[u][1] = x.y; xv[u][2] = x.z; xv[u][3] = x.w;
@@ -1032,7 +1116,7 @@ paged_decode_merge_kernel(const KernelParams p, int batch) {
           }
         } else {
 #pragma unroll
-          for (int e = 0; e < E; ++e) xv[u][e] = load_partial_elem(p.partial_output, p.partial_dtype, pidx * D + lane * E + e);
+          for (int e = 0; e < E; ++e) xv[u][e] = load_partial_elem(p.partial_output, p.partial_dtype, (base + slot) * D + lane * E + e);
         }
       }
       float m_new = big;

@@ -278,7 +278,7 @@ def shared_prefix_decode_grouped_fp8_e4m3(
     split-KV pass from each request's own start, one merge.  ``max_suffix_len`` bounds what a
     request in a group has behind its prefix (``max_seq_len`` minus the grouping's
     ``min_prefix_len`` is always a true bound; ``None`` = the whole context): the split-KV grid is
-    sized for it and requests in no group get as many, longer, splits.  The workspace needs
+    sized for it; requests in no group have CTAs of their own.  The workspace needs
     ``ceil(min(max_prefix_len, max_seq_len) / 256) + ceil(min(max_suffix_len, max_seq_len) /
     split_size)`` slots.  ``all_in_groups`` (``PFD_FLAG_ALL_IN_GROUPS``): the caller has read
     ``groups.buffer[4]`` and it equals the batch; the split-KV pass may then run beside the dense

@@ -451,3 +451,44 @@ def test_grouped_decode_with_more_tiles_than_tile_slots(cabi, hint):
         torch.cuda.synchronize()
         assert cabi.device_status() == 0
         assert_within_gate(out, exp, f"three groups of 17, hint={hint}, step {step}")
+
+
+@pytest.mark.parametrize("batch,hq,hkv,grouped,longest,suffix", [
+    (150, 16, 2, 8, 1500, 40),    # many requests in none: the scan takes two rounds, items are taken in several turns
+    (12, 32, 8, 8, 4000, 16),     # a few long ones: as many splits as their slots allow
+    (40, 8, 8, 0, 700, 100),      # no group at all
+    (16, 28, 4, 15, 900, 300),    # one request in none
+])
+def test_requests_in_no_group_have_ctas_of_their_own(cabi, batch, hq, hkv, grouped, longest, suffix):
+    """Lengths from nothing to the longest (a multiple of the split size, and one more or less) among the requests that
+    the grid rows in front share out, beside a group whose suffixes go the ordinary way."""
+    gen = torch.Generator().manual_seed(batch)
+    prefix_pages, pages, d = 16, 3000, 128
+    from single_gpu_inference_lab_b200.workloads import quantize_per_head
+
+    kc, ks = quantize_per_head(torch.randn(pages, 16, hkv, d, generator=gen))
+    vc, vs = quantize_per_head(torch.randn(pages, 16, hkv, d, generator=gen))
+    table = torch.randint(0, pages, (batch, -(-longest // 16)), generator=gen, dtype=torch.int32)
+    lens = torch.randint(1, longest + 1, (batch,), generator=gen, dtype=torch.int32)
+    table[:grouped, :prefix_pages] = table[:1, :prefix_pages]
+    lens[:grouped] = prefix_pages * 16 + torch.randint(0, suffix + 1, (grouped,), generator=gen, dtype=torch.int32)
+    for r, n in zip(range(grouped, batch), (longest, 0, 256, 257, 255, 512, 1)):
+        lens[r] = n
+    lens[-1] = longest
+    q = torch.randn(batch, hq, d, generator=gen).to(torch.bfloat16)
+    live = lens > 0
+    exp = torch.zeros_like(q)
+    exp[live] = oracle.reference(q[live], kc, vc, table[live].long(), lens[live], ks, vs)
+    gq, gkc, gvc, gt, gl, gks, gvs = (t.to(DEV) for t in (q, kc, vc, table, lens, ks, vs))
+    groups, max_groups = cabi.group_shared_prefixes(gt, seq_lens=gl, min_batch=8, min_prefix_len=256, max_groups=2)
+    split, cap = 64, 256
+    slots = cap // 256 + -(-suffix // split)
+    ws = tuple(torch.full(s, float("nan"), device=DEV) for s in ((batch, hq, slots, d), (batch, hq, slots), (batch, hq, slots)))
+    for step in range(2):
+        out = torch.full_like(gq, float("nan"))
+        cabi.shared_prefix_decode_grouped_fp8_e4m3(
+            gq, gkc, gvc, gt, gl, groups=groups, max_groups=max_groups, max_prefix_len=cap, max_suffix_len=suffix,
+            k_scale=gks, v_scale=gvs, max_seq_len=longest, split_size=split, output=out, workspace=ws)
+        torch.cuda.synchronize()
+        assert cabi.device_status() == 0
+        assert_within_gate(out, exp, f"step {step}")
