@@ -860,8 +860,18 @@ int pfd_plan_decode(const pfd_decode_args* args, int32_t cache_elem_bytes, void*
   pp.max_groups = max_groups;
   pp.piece_cost = kChunkPieceCost;
   pp.plan = static_cast<int32_t*>(plan);
-  const int ctas = std::max(1, std::min(8, (max_groups + 31) / 32));
-  pfd::plan_decode_kernel<<<ctas, 1024, 0, static_cast<cudaStream_t>(a.stream)>>>(pp);
+  constexpr int kPlanWarps = pfd::kPlanThreads / 32;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(static_cast<unsigned>(std::min(2 * t_device->sms, (max_groups + kPlanWarps - 1) / kPlanWarps)));
+  cfg.blockDim = dim3(pfd::kPlanThreads);
+  cfg.stream = static_cast<cudaStream_t>(a.stream);
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, pfd::plan_decode_kernel, pp);
+  if (e != cudaSuccess) return fail(PFD_ERR_CUDA, "plan kernel launch failed: %s", cudaGetErrorString(e));
   return check_launch("plan kernel");
 }
 
