@@ -127,10 +127,11 @@ struct MapKey {
   int32_t heads;
   int32_t promotion;   // L2 promotion in bytes
   int32_t elem_bytes;  // 1: e4m3, 2: fp16 / bf16
+  int32_t head_dim;
   bool operator==(const MapKey& o) const {
     return dev == o.dev && base == o.base && stride_page == o.stride_page && stride_token == o.stride_token &&
            stride_head == o.stride_head && num_pages == o.num_pages && heads == o.heads &&
-           promotion == o.promotion && elem_bytes == o.elem_bytes;
+           promotion == o.promotion && elem_bytes == o.elem_bytes && head_dim == o.head_dim;
   }
 };
 struct MapEntry {
@@ -165,10 +166,13 @@ bool head_is_dim1(int64_t stride_token, int64_t stride_head) { return stride_hea
 // time, so fetching 256 bytes (two heads' rows in the NHD layout) per 128-byte request pays; the
 // balanced grid does not keep kv heads in step, there the second half would be evicted unused.
 // (With 2-byte elements the strides are given in elements and the box is half a row, 64
-// elements = 128 bytes, so that the 128-byte swizzle still applies.)
+// elements = 128 bytes, so that the 128-byte swizzle still applies; head_dim 64, e4m3 only: the rows are
+// 64 bytes, with the 64-byte swizzle.)
 int get_tensor_map(const void* base, int64_t stride_page, int64_t stride_token, int64_t stride_head,
-                   int64_t num_pages, int32_t heads, int32_t promotion, CUtensorMap* out, int32_t elem_bytes = 1) {
-  const MapKey key{t_device->dev, base, stride_page, stride_token, stride_head, num_pages, heads, promotion, elem_bytes};
+                   int64_t num_pages, int32_t heads, int32_t promotion, CUtensorMap* out, int32_t elem_bytes = 1,
+                   int32_t head_dim = 128) {
+  const MapKey key{t_device->dev, base, stride_page, stride_token, stride_head, num_pages, heads, promotion, elem_bytes,
+                   head_dim};
   MapSlot& slot = t_map_slots[map_slot_of(base, elem_bytes)];
   if (slot.used && slot.entry.key == key) {
     *out = slot.entry.map;
@@ -191,12 +195,12 @@ int get_tensor_map(const void* base, int64_t stride_page, int64_t stride_token, 
     g_encode = reinterpret_cast<EncodeTiledFn>(fn);
   }
   const bool h1 = head_is_dim1(stride_token, stride_head);
-  const cuuint64_t dims[4] = {128, (cuuint64_t)(h1 ? heads : 16), (cuuint64_t)(h1 ? 16 : heads),
+  const cuuint64_t dims[4] = {(cuuint64_t)head_dim, (cuuint64_t)(h1 ? heads : 16), (cuuint64_t)(h1 ? 16 : heads),
                               (cuuint64_t)num_pages};
   const cuuint64_t strides[3] = {(cuuint64_t)(h1 ? stride_head : stride_token) * elem_bytes,
                                  (cuuint64_t)(h1 ? stride_token : stride_head) * elem_bytes,
                                  (cuuint64_t)stride_page * elem_bytes};
-  const cuuint32_t box[4] = {(cuuint32_t)(128 / elem_bytes), (cuuint32_t)(h1 ? 1 : 16), (cuuint32_t)(h1 ? 16 : 1), 1};
+  const cuuint32_t box[4] = {(cuuint32_t)(head_dim / elem_bytes), (cuuint32_t)(h1 ? 1 : 16), (cuuint32_t)(h1 ? 16 : 1), 1};
   const cuuint32_t elem[4] = {1, 1, 1, 1};
   MapEntry entry;
   entry.key = key;
@@ -207,7 +211,8 @@ int get_tensor_map(const void* base, int64_t stride_page, int64_t stride_token, 
                                                           : CU_TENSOR_MAP_L2_PROMOTION_L2_256B;
   const CUresult r = g_encode(&entry.map, elem_bytes == 2 ? CU_TENSOR_MAP_DATA_TYPE_UINT16 : CU_TENSOR_MAP_DATA_TYPE_UINT8,
                               4, const_cast<void*>(base), dims, strides,
-                              box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, promo,
+                              box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                              head_dim == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B, promo,
                               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return fail(PFD_ERR_CUDA, "cuTensorMapEncodeTiled failed with CUresult %d", (int)r);
   if (g_maps.size() >= 1024) g_maps.erase(g_maps.begin());
@@ -218,12 +223,14 @@ int get_tensor_map(const void* base, int64_t stride_page, int64_t stride_token, 
   return PFD_OK;
 }
 
-bool tma_eligible(const pfd_decode_args& a) {
-  if (a.head_dim != 128 || (a.flags & PFD_FLAG_NO_TMA)) return false;
+bool tma_describable(const pfd_decode_args& a) {
   // a size-1 dimension may carry any stride; everything else was checked to be 16-byte aligned
   return a.k_stride_page > 0 && a.v_stride_page > 0 && a.k_stride_token > 0 && a.v_stride_token > 0 &&
          a.k_stride_head > 0 && a.v_stride_head > 0 && a.num_pages > 0 &&
          head_is_dim1(a.k_stride_token, a.k_stride_head) == head_is_dim1(a.v_stride_token, a.v_stride_head);
+}
+bool tma_eligible(const pfd_decode_args& a) {
+  return a.head_dim == 128 && !(a.flags & PFD_FLAG_NO_TMA) && tma_describable(a);
 }
 
 // kWarpsT = 2, kStagesT = 1 beside the dense prefix pass: two CTAs of two warps, 165 registers
@@ -333,6 +340,34 @@ bool balanced_eligible(const pfd_decode_args& a, int group, int slot_offset, int
   return rows >= 2LL * (sms * kChunkWarps / a.num_kv_heads) * a.num_q_heads;
 }
 
+// The balanced kernel for head_dim 64 (up to eight query heads per KV head): pages are half as many bytes
+// and a page pair nearly as many instructions as with 128, so sixteen warps share an SM's 192 KiB
+// ring, three 4 KiB stages each (14 + 2 heads, batch 256, 512 .. 4096 tokens, us per call: 8 warps 42.7, 12
+// 37.4, 16 37.2; the fixed-split grid with plain loads 53.3).  It needs slots for three quarters of
+// its warp groups: us balanced / grid, 14 + 2 heads, lengths all alike, uniform, log-uniform to the maximum
+//   room 0.86: 128 x 8192: 53.2 / 77.1, 34.7 / 48.2, 17.0 / 17.9   256 x 4096: 56.2 / 77.1, 37.5 / 51.2, 17.7 / 19.4
+//   room 0.43: 128 x 4096: 40.8 / 43.7, 26.9 / 28.4, 14.3 / 14.0    64 x 8192: 39.8 / 43.6, 25.0 / 23.8, 13.9 / 13.0
+//   room 0.22:  64 x 4096: 34.6 / 20.4, 23.8 / 16.8, 11.6 /  9.9
+// and, since a caller's small split size makes room for any batch, work for them: with 2^17 tokens at
+// most (batch x longest) even eight KV heads leave it nothing to win.
+// Returns the warp groups that its workspace has room for, 0 for the fixed-split grid.
+constexpr int kChunkStages64 = 3, kChunkWarps64 = 16;
+constexpr int64_t kBalanced64MinTokens = 1 << 17;
+int balanced64_groups(const pfd_decode_args& a, int group, int slot_offset, int sms) {
+  if (a.flags & (PFD_FLAG_FIXED_SPLITS | PFD_FLAG_NO_TMA | PFD_FLAG_NO_DIRECT_OUT | PFD_FLAG_PARTIAL_ONLY)) return 0;
+  if (slot_offset != 0 || a.page_indptr != nullptr || a.exchange != nullptr || !tma_describable(a)) return 0;
+  if (group > 8 || a.batch > kChunkMaxBatch || a.num_kv_heads > kChunkWarps64 * sms / 2) return 0;
+  if (!a.partial_output || !a.partial_max || !a.partial_sum || a.partial_dtype != PFD_DTYPE_F32) return 0;
+  if (a.partial_stride_s != 1 || a.partial_stride_h != a.workspace_splits ||
+      a.partial_stride_b != (int64_t)a.num_q_heads * a.workspace_splits)
+    return 0;
+  const int64_t span = std::max(a.max_seq_len - a.kv_start, 0);
+  if (a.batch * span < kBalanced64MinTokens) return 0;
+  const int64_t room = (int64_t)a.batch * a.workspace_splits / 2;  // two slots of num_q_heads rows for a group
+  const int64_t all = (int64_t)sms * kChunkWarps64 / a.num_kv_heads;
+  return 4 * room >= 3 * all ? static_cast<int>(std::min(room, all)) : 0;
+}
+
 // Warps of the balanced grid that take part: all of them, or fewer when the workspace has room
 // for fewer slots (max_groups > 0).  The plan is made for the same number.
 int balanced_num_warps(int sms, int warps_per_cta, int num_kv_heads, int max_groups) {
@@ -342,16 +377,16 @@ int balanced_num_warps(int sms, int warps_per_cta, int num_kv_heads, int max_gro
 }
 
 // max_groups > 0 caps the number of warp groups (a workspace with room for fewer slots).
-template <bool QBF16, int kStagesT, int kWarpsT, bool KV16 = false>
+template <bool QBF16, int kStagesT, int kWarpsT, bool KV16 = false, int D = 128>
 int launch_balanced(const pfd_decode_args& a, const pfd::KernelParams& kp, int sms, cudaStream_t stream,
                     int max_groups = 0) {
   CUtensorMap mk, mv;
   constexpr int kElem = KV16 ? 2 : 1;
   if (int rc = get_tensor_map(a.key_cache, a.k_stride_page, a.k_stride_token, a.k_stride_head, a.num_pages,
-                              a.num_kv_heads, 256, &mk, kElem))
+                              a.num_kv_heads, 256, &mk, kElem, D))
     return rc;
   if (int rc = get_tensor_map(a.value_cache, a.v_stride_page, a.v_stride_token, a.v_stride_head, a.num_pages,
-                              a.num_kv_heads, 256, &mv, kElem))
+                              a.num_kv_heads, 256, &mv, kElem, D))
     return rc;
   pfd::TmaParams tp{};
   tp.head_is_dim1 = head_is_dim1(a.k_stride_token, a.k_stride_head) ? 1 : 0;
@@ -359,19 +394,22 @@ int launch_balanced(const pfd_decode_args& a, const pfd::KernelParams& kp, int s
   tp.wait_limit_ns = g_wait_limit_ns.load(std::memory_order_relaxed);
   tp.phase_times = g_phase_times;
   // A plan needs f32 pieces (its in-kernel merge reads them as such; the merge kernel takes either).
-  const bool planned = a.plan != nullptr && a.partial_dtype == PFD_DTYPE_F32;
+  const bool planned = D == 128 && a.plan != nullptr && a.partial_dtype == PFD_DTYPE_F32;
   const bool fused = planned && (a.flags & PFD_FLAG_SINGLE_LAUNCH) && !(a.flags & PFD_FLAG_PARTIAL_ONLY);
-  auto kernel = fused ? pfd::paged_decode_fp8_chunk_kernel<QBF16, kStagesT, kWarpsT, KV16, true>
-                      : pfd::paged_decode_fp8_chunk_kernel<QBF16, kStagesT, kWarpsT, KV16, false>;
+  auto kernel = pfd::paged_decode_fp8_chunk_kernel<QBF16, kStagesT, kWarpsT, KV16, false, D>;
+  if constexpr (D == 128) {
+    if (fused) kernel = pfd::paged_decode_fp8_chunk_kernel<QBF16, kStagesT, kWarpsT, KV16, true>;
+  }
   constexpr int kThreads = kWarpsT * 32;
   // ring + mbarriers + scan scratch + prefix[B + 1] + lens[B], sized for the largest batch
-  constexpr int smem = 1024 + kWarpsT * kStagesT * 8192 * kElem + kWarpsT * kStagesT * 8 +
+  constexpr int smem = 1024 + kWarpsT * kStagesT * 64 * D * kElem + kWarpsT * kStagesT * 8 +
                        kWarpsT * 4 + (2 * kChunkMaxBatch + 1) * 4 + 16;
   static std::atomic<bool> configured[2][kMaxDevices];  // one array per instantiation of this template
   if (int rc = configure_smem(configured[fused ? 1 : 0], kernel, smem)) return rc;
   pfd::ChunkParams cp{};
   cp.batch = a.batch;
   cp.num_warps = balanced_num_warps(sms, kWarpsT, a.num_kv_heads, max_groups);
+  cp.warps_per_cta = (cp.num_warps + sms - 1) / sms;
   cp.piece_cost = kChunkPieceCost;
   cp.plan = planned ? static_cast<int32_t*>(a.plan) : nullptr;
   cudaLaunchAttribute attr[1];
@@ -402,7 +440,10 @@ int launch_balanced(const pfd_decode_args& a, const pfd::KernelParams& kp, int s
     // (CTAs of a single warp and row, all resident beside the chunk kernel, were measured
     // slower: 21.8 against 19.9 us per step on the batch-64 configuration.)
     const int rows = a.batch * a.num_q_heads;
-    const bool wide = rows <= 8 * sms;  // (one warp per row on the batch-64 configuration: 21.0 against 19.9 us)
+    // (one warp per row on the batch-64 configuration: 21.0 against 19.9 us).  Head_dim 64, whose rows are
+    // half as long, up to sixteen rows per SM where sequences can be long, i.e. have many pieces: batch
+    // 128 x 8192, log-uniform: 20.8 -> 17.0 us per call; batch 256 x 1024, 8 KV heads, would lose (48.5 -> 50.8).
+    const bool wide = rows <= 8 * sms || (D == 64 && rows <= 16 * sms && a.max_seq_len > 4096);
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(wide ? rows : (rows + 3) / 4);
     cfg.blockDim = dim3(128);
@@ -411,8 +452,8 @@ int launch_balanced(const pfd_decode_args& a, const pfd::KernelParams& kp, int s
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     const cudaError_t e =
-        wide ? cudaLaunchKernelEx(&cfg, pfd::paged_decode_chunk_merge_kernel<QBF16, 4, 4, 8>, kp, tp, cp)
-             : cudaLaunchKernelEx(&cfg, pfd::paged_decode_chunk_merge_kernel<QBF16, 1, 16, 4>, kp, tp, cp);
+        wide ? cudaLaunchKernelEx(&cfg, pfd::paged_decode_chunk_merge_kernel<QBF16, 4, 4, 8, D>, kp, tp, cp)
+             : cudaLaunchKernelEx(&cfg, pfd::paged_decode_chunk_merge_kernel<QBF16, 1, 16, 4, D>, kp, tp, cp);
     if (e != cudaSuccess) return fail(PFD_ERR_CUDA, "balanced merge kernel launch failed: %s", cudaGetErrorString(e));
   }
   return check_launch("balanced merge kernel");
@@ -421,9 +462,13 @@ int launch_balanced(const pfd_decode_args& a, const pfd::KernelParams& kp, int s
 template <int D, bool QBF16>
 int launch_decode(const pfd_decode_args& a, const pfd::KernelParams& kp, int num_splits) {
   cudaStream_t stream = static_cast<cudaStream_t>(a.stream);
-  if (D == 128) {
+  if constexpr (D == 128) {
     const int sms = t_device->sms;
     if (balanced_eligible(a, kp.group, kp.slot_offset, sms)) return launch_balanced<QBF16, kChunkStages, kChunkWarps>(a, kp, sms, stream);
+  } else {
+    const int sms = t_device->sms;
+    if (const int groups = balanced64_groups(a, kp.group, kp.slot_offset, sms))
+      return launch_balanced<QBF16, kChunkStages64, kChunkWarps64, false, 64>(a, kp, sms, stream, groups);
   }
   if (a.page_indptr != nullptr)
     return fail(PFD_ERR_UNSUPPORTED,
@@ -553,6 +598,13 @@ pfd::KernelParams fill_params(const pfd_decode_args& a, int group, bool direct_o
     kp.packed_output = static_cast<float*>(x.recv[x.rank]);  // non-NULL selects the packed form; the kernels address through xch_recv
     kp.output = nullptr;
   }
+  // (o, m, l) rows that the caller gets to see, or that are stored in 16 bits, are relative to the true
+  // maximum.  So are fp16 calls': with the largest probabilities at and just below 1 their rounding to
+  // f16 is at its best, and unlike a bf16 output an fp16 one shows it (relative error against 64 bits, 32
+  // + 2 heads, 512 .. 4096 tokens: 2.6e-4 so, 2.8e-4 with a slack of 8; bf16 1.7e-3 either way).
+  kp.max_slack = kp.packed_output != nullptr || a.partial_dtype != PFD_DTYPE_F32 || a.query_dtype == PFD_DTYPE_F16 ||
+                         (a.flags & PFD_FLAG_PARTIAL_ONLY)
+                     ? 0.f : 8.f;
 #ifdef PFD_BOUNDS_CHECK
   kp.dbg_ws_rows = (int64_t)a.batch * a.num_q_heads * a.workspace_splits;
   kp.dbg_batch = a.batch;

@@ -31,6 +31,7 @@ namespace pfd {
 struct ChunkParams {
   int32_t batch;
   int32_t num_warps;   // warps of the whole grid; the merge kernel is told the same number
+  int32_t warps_per_cta;  // (fewer warps than the grid has: every CTA leaves some idle, not some CTAs all)
   int32_t piece_cost;  // what starting a sequence costs a warp, in half page pairs
   int32_t* plan;       // device plan written by plan_decode_kernel, or nullptr
 };
@@ -78,27 +79,27 @@ __device__ __forceinline__ uint32_t movmatrix_trans(uint32_t a) {
 }
 
 // Running state of one warp for the current segment, NH head tiles of 8 heads.
-template <int NH>
+template <int NH, int D>
 struct BalState {
-  float o[NH][8][4];  // [head tile][m-tile mt][c]: d = 16i + 2mt + (c>>1), head = 8h + 2j + (c&1)
+  float o[NH][D / 16][4];  // [head tile][m-tile mt][c]: d = (D / 8) i + 2mt + (c>>1), head = 8h + 2j + (c&1)
   float m[NH][2];     // running max (log2 domain) of heads 2j, 2j+1
   float l[NH][2];     // running sum over this thread's tokens only
 };
 
-template <int NH>
-__device__ __forceinline__ void bal_reset(BalState<NH>& st) {
+template <int NH, int D>
+__device__ __forceinline__ void bal_reset(BalState<NH, D>& st) {
 #pragma unroll
   for (int h = 0; h < NH; ++h) {
 #pragma unroll
-    for (int mt = 0; mt < 8; ++mt) st.o[h][mt][0] = st.o[h][mt][1] = st.o[h][mt][2] = st.o[h][mt][3] = 0.f;
+    for (int mt = 0; mt < D / 16; ++mt) st.o[h][mt][0] = st.o[h][mt][1] = st.o[h][mt][2] = st.o[h][mt][3] = 0.f;
     st.m[h][0] = st.m[h][1] = -INFINITY;
     st.l[h][0] = st.l[h][1] = 0.f;
   }
 }
 
 // Q of head (8h + i) as B-fragments: k-step ks = 4l + w covers d = 16(j+4l) + 4w + {0,1 | 2,3}.
-template <bool QBF16, int NH>
-__device__ __forceinline__ void bal_load_q(uint32_t (&qb)[NH][8][2], const KernelParams& p, int b,
+template <bool QBF16, int NH, int D>
+__device__ __forceinline__ void bal_load_q(uint32_t (&qb)[NH][D / 16][2], const KernelParams& p, int b,
                                            int kvh, int i, int j) {
 #pragma unroll
   for (int h = 0; h < NH; ++h) {
@@ -107,7 +108,7 @@ __device__ __forceinline__ void bal_load_q(uint32_t (&qb)[NH][8][2], const Kerne
     const uint16_t* q = reinterpret_cast<const uint16_t*>(p.query) + (int64_t)b * p.q_stride_b +
                         (int64_t)(kvh * p.group + (live ? head : 0)) * p.q_stride_h;
 #pragma unroll
-    for (int l = 0; l < 2; ++l) {
+    for (int l = 0; l < D / 64; ++l) {
 #pragma unroll
       for (int w = 0; w < 4; ++w) {
         uint2 raw = make_uint2(0u, 0u);
@@ -133,13 +134,73 @@ __device__ __forceinline__ void mma_16816(float (&c)[4], uint32_t a0, uint32_t a
       : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
+// Offset of 16-byte chunk `chunk` of row `row` in a (page, head) tile as TMA leaves it: rows of D bytes,
+// chunks XOR-ed with the row (128-byte swizzle) or with half of it (64-byte swizzle).
+template <int D>
+__device__ __forceinline__ uint32_t bal_chunk(int row, int chunk) {
+  return row * D + ((chunk ^ (D == 128 ? row & 7 : (row >> 1) & 3)) << 4);
+}
+// Row of a page that a thread's V load r reads.  64-byte rows: odd j take the rows of a column pair in the
+// other order, so that the 16 lanes of a load phase read even and odd rows, which lie in different
+// halves of the banks; the byte permutes below put the pair back in order.
+template <int D>
+__device__ __forceinline__ int bal_v_row(int j, int r) { return v_row(j, D == 128 ? r : r ^ (j & 1)); }
+__device__ __forceinline__ uint2 lds_8(uint32_t addr) {
+  uint2 v;
+  asm volatile("ld.shared.v2.u32 {%0,%1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(addr));
+  return v;
+}
+
+// The running maximum of a step's raw scores s[head tile][page][c] (heads 2j + (c & 1)), scaled, brought
+// up to date -- only when some score lies more than `slack` (log2 units) above it: the maximum only has
+// to keep the exponentials in range, and a probability of up to 2^slack against a stale one is as
+// exact, in f16 or two bf16 terms, as one of up to 1.  So after a piece's first step the three
+// shuffles per head, the rescaling factors and the rescaling itself hardly ever run: they were the longest
+// part of a step's chain (a recorded step of eight layers, 16 + 2 heads, batch 64: 160.9 -> 150.7 us;
+// 4 x 131072 tokens: 173.4 -> 162.7).  scale_log2 >= 0 (see the kernel).
+template <int NH, int MT>
+__device__ __forceinline__ void bal_raise_max(float (&m)[NH][2], float (&l)[NH][2], float (&o)[NH][MT][4],
+                                              const float (&s)[NH][2][4], float scale_log2, float slack) {
+  float x[NH][2];
+  bool higher = false;
+#pragma unroll
+  for (int h = 0; h < NH; ++h)
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      x[h][e] = fmaxf(fmaxf(s[h][0][e], s[h][0][2 + e]), fmaxf(s[h][1][e], s[h][1][2 + e])) * scale_log2;
+      higher |= x[h][e] > m[h][e] + slack;
+    }
+  if (!__any_sync(0xffffffffu, higher)) return;
+#pragma unroll
+  for (int h = 0; h < NH; ++h) {
+    float alpha[2];
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      float y = x[h][e];
+      y = fmaxf(y, __shfl_xor_sync(0xffffffffu, y, 4));
+      y = fmaxf(y, __shfl_xor_sync(0xffffffffu, y, 8));
+      y = fmaxf(y, __shfl_xor_sync(0xffffffffu, y, 16));
+      y = fmaxf(m[h][e], y);
+      alpha[e] = exp2f(m[h][e] - y);
+      m[h][e] = y;
+      l[h][e] *= alpha[e];
+    }
+#pragma unroll
+    for (int mt = 0; mt < MT; ++mt) {
+      o[h][mt][0] *= alpha[0]; o[h][mt][1] *= alpha[1];
+      o[h][mt][2] *= alpha[0]; o[h][mt][3] *= alpha[1];
+    }
+  }
+}
+
 // One step = two consecutive pages (32 tokens) of one segment, read from a stage
-// [K0][K1][V0][V1] (2 KiB tiles, 128-byte swizzle).  tok0 = token index of page 0's row 0.
-template <int NH>
-__device__ __forceinline__ void bal_step(BalState<NH>& st, uint32_t stage, const uint32_t (&k_off)[2][2],
-                                         const uint32_t (&v_off)[4], const uint32_t (&qb)[NH][8][2],
-                                         float scale_log2, int tok0, int lo, int hi, int i, int j) {
-  constexpr uint32_t kTile = kPage * 128;
+// [K0][K1][V0][V1] (16 x D-byte tiles, see bal_chunk).  tok0 = token index of page 0's row 0.
+template <int NH, int D>
+__device__ __forceinline__ void bal_step(BalState<NH, D>& st, uint32_t stage, const uint32_t (&k_off)[2][D / 64],
+                                         const uint32_t (&v_off)[4], const uint32_t (&qb)[NH][D / 16][2],
+                                         float scale_log2, float slack, int tok0, int lo, int hi, int i, int j) {
+  constexpr uint32_t kTile = kPage * D;
+  constexpr int KL = D / 64, VW = D / 32;
   const bool edge = (tok0 < lo) | (tok0 + 2 * kPage > hi);
   float s[NH][2][4];
 #pragma unroll
@@ -147,18 +208,18 @@ __device__ __forceinline__ void bal_step(BalState<NH>& st, uint32_t stage, const
 #pragma unroll
     for (int u = 0; u < 2; ++u) s[h][u][0] = s[h][u][1] = s[h][u][2] = s[h][u][3] = 0.f;
   {
-    uint32_t k[2][2][2][4];  // [page][row half][l][word]
+    uint32_t k[2][2][KL][4];  // [page][row half][l][word]
 #pragma unroll
     for (int u = 0; u < 2; ++u)
 #pragma unroll
       for (int half = 0; half < 2; ++half)
 #pragma unroll
-        for (int l = 0; l < 2; ++l) {
+        for (int l = 0; l < KL; ++l) {
           const uint4 x = lds_16(stage + u * kTile + k_off[half][l]);
           k[u][half][l][0] = x.x; k[u][half][l][1] = x.y; k[u][half][l][2] = x.z; k[u][half][l][3] = x.w;
         }
 #pragma unroll
-    for (int l = 0; l < 2; ++l)
+    for (int l = 0; l < KL; ++l)
 #pragma unroll
       for (int w = 0; w < 4; ++w)
 #pragma unroll
@@ -170,74 +231,72 @@ __device__ __forceinline__ void bal_step(BalState<NH>& st, uint32_t stage, const
           for (int h = 0; h < NH; ++h) mma_16816(s[h][u], a0, a1, a2, a3, qb[h][l * 4 + w][0], qb[h][l * 4 + w][1]);
         }
   }
-  // scale + mask: s[h][u][c] is (token 16u + 8(c>>1) + rho(i), head 8h + 2j + (c&1))
+  // mask: s[h][u][c] is (token 16u + 8(c>>1) + rho(i), head 8h + 2j + (c&1))
+  uint32_t dead = 0u;  // bit 4u + c
+  if (edge) {
 #pragma unroll
-  for (int u = 0; u < 2; ++u)
+    for (int u = 0; u < 2; ++u)
 #pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      bool dead = false;
-      if (edge) {
+      for (int c = 0; c < 4; ++c) {
         const int tok = tok0 + u * kPage + 8 * (c >> 1) + rho(i);
-        dead = (tok < lo) | (tok >= hi);
-      }
+        if ((tok < lo) | (tok >= hi)) {
+          dead |= 1u << (4 * u + c);
 #pragma unroll
-      for (int h = 0; h < NH; ++h) s[h][u][c] = dead ? -INFINITY : s[h][u][c] * scale_log2;
-    }
+          for (int h = 0; h < NH; ++h) s[h][u][c] = -INFINITY;
+        }
+      }
+  }
+  bal_raise_max<NH, D / 16>(st.m, st.l, st.o, s, scale_log2, slack);
   uint32_t pb[NH][2][2];  // P^T B-fragments [head tile][page][b0|b1]
 #pragma unroll
   for (int h = 0; h < NH; ++h) {
-    float mx[2], alpha[2];
-#pragma unroll
-    for (int e = 0; e < 2; ++e) {
-      float x = fmaxf(fmaxf(s[h][0][e], s[h][0][2 + e]), fmaxf(s[h][1][e], s[h][1][2 + e]));
-      x = fmaxf(x, __shfl_xor_sync(0xffffffffu, x, 4));
-      x = fmaxf(x, __shfl_xor_sync(0xffffffffu, x, 8));
-      x = fmaxf(x, __shfl_xor_sync(0xffffffffu, x, 16));
-      mx[e] = fmaxf(st.m[h][e], x);
-      alpha[e] = exp2f(st.m[h][e] - mx[e]);
-      st.m[h][e] = mx[e];
-    }
-    float sum[2] = {0.f, 0.f};
 #pragma unroll
     for (int u = 0; u < 2; ++u) {
-      const float p0 = exp2f(s[h][u][0] - mx[0]), p1 = exp2f(s[h][u][1] - mx[1]);
-      const float p2 = exp2f(s[h][u][2] - mx[0]), p3 = exp2f(s[h][u][3] - mx[1]);
-      sum[0] += p0 + p2;
-      sum[1] += p1 + p3;
-      // (token row i, heads 2j, 2j+1) -> transpose -> (tokens rho(2j), rho(2j+1); head i)
-      pb[h][u][0] = movmatrix_trans(pack_f16x2(p0, p1));
-      pb[h][u][1] = movmatrix_trans(pack_f16x2(p2, p3));
-    }
-    st.l[h][0] = st.l[h][0] * alpha[0] + sum[0];
-    st.l[h][1] = st.l[h][1] * alpha[1] + sum[1];
-    if (__any_sync(0xffffffffu, (alpha[0] != 1.f) | (alpha[1] != 1.f))) {
+      float pr[4];
 #pragma unroll
-      for (int mt = 0; mt < 8; ++mt) {
-        st.o[h][mt][0] *= alpha[0]; st.o[h][mt][1] *= alpha[1];
-        st.o[h][mt][2] *= alpha[0]; st.o[h][mt][3] *= alpha[1];
+      for (int c = 0; c < 4; ++c) pr[c] = exp2f(fmaf(s[h][u][c], scale_log2, -st.m[h][c & 1]));
+      if (edge) {
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+          if ((dead >> (4 * u + c)) & 1u) pr[c] = 0.f;
       }
+      st.l[h][0] += pr[0] + pr[2];
+      st.l[h][1] += pr[1] + pr[3];
+      // (token row i, heads 2j, 2j+1) -> transpose -> (tokens rho(2j), rho(2j+1); head i)
+      pb[h][u][0] = movmatrix_trans(pack_f16x2(pr[0], pr[1]));
+      pb[h][u][1] = movmatrix_trans(pack_f16x2(pr[2], pr[3]));
     }
   }
   // O^T += V^T P^T
+  const bool swapped = D == 64 && (j & 1);  // (see bal_v_row)
+  const uint32_t sel01 = swapped ? 0x1504u : 0x5140u, sel23 = swapped ? 0x3726u : 0x7362u;
 #pragma unroll
   for (int u = 0; u < 2; ++u) {
-    uint32_t v[4][4];
+    uint32_t v[4][VW];
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
-      const uint4 x = lds_16(stage + (2 + u) * kTile + v_off[r]);
-      v[r][0] = x.x; v[r][1] = x.y; v[r][2] = x.z; v[r][3] = x.w;
+      if constexpr (D == 128) {
+        const uint4 x = lds_16(stage + (2 + u) * kTile + v_off[r]);
+        v[r][0] = x.x; v[r][1] = x.y; v[r][2] = x.z; v[r][3] = x.w;
+      } else {
+        const uint2 x = lds_8(stage + (2 + u) * kTile + v_off[r]);
+        v[r][0] = x.x; v[r][1] = x.y;
+      }
     }
     if (edge) {  // bytes of tokens outside the range may hold anything: 0 * NaN must not happen
 #pragma unroll
       for (int r = 0; r < 4; ++r) {
-        const int tok = tok0 + u * kPage + v_row(j, r);
-        if (tok < lo || tok >= hi) v[r][0] = v[r][1] = v[r][2] = v[r][3] = 0u;
+        const int tok = tok0 + u * kPage + bal_v_row<D>(j, r);
+        if (tok < lo || tok >= hi) {
+#pragma unroll
+          for (int w = 0; w < VW; ++w) v[r][w] = 0u;
+        }
       }
     }
 #pragma unroll
-    for (int w = 0; w < 4; ++w) {
-      const uint32_t x01 = prmt(v[0][w], v[1][w], 0x5140u), y01 = prmt(v[0][w], v[1][w], 0x7362u);
-      const uint32_t x23 = prmt(v[2][w], v[3][w], 0x5140u), y23 = prmt(v[2][w], v[3][w], 0x7362u);
+    for (int w = 0; w < VW; ++w) {
+      const uint32_t x01 = prmt(v[0][w], v[1][w], sel01), y01 = prmt(v[0][w], v[1][w], sel23);
+      const uint32_t x23 = prmt(v[2][w], v[3][w], sel01), y23 = prmt(v[2][w], v[3][w], sel23);
       const uint32_t e0 = cvt_e4m3x2_to_f16x2(x01), e1 = cvt_e4m3x2_to_f16x2(x01 >> 16);
       const uint32_t e2 = cvt_e4m3x2_to_f16x2(x23), e3 = cvt_e4m3x2_to_f16x2(x23 >> 16);
       const uint32_t f0 = cvt_e4m3x2_to_f16x2(y01), f1 = cvt_e4m3x2_to_f16x2(y01 >> 16);
@@ -251,40 +310,40 @@ __device__ __forceinline__ void bal_step(BalState<NH>& st, uint32_t stage, const
   }
 }
 
-template <bool QBF16>
-__device__ __forceinline__ void store_row16(const KernelParams& p, int b, int hq, int d0, const float (&v)[16],
-                                            float m_nat, float l, bool write_ml, uint32_t xstep) {
-  // 16 consecutive head-dim values of one (sequence, q head) row: final output, packed form, or
+template <bool QBF16, int D>
+__device__ __forceinline__ void store_row_part(const KernelParams& p, int b, int hq, int d0, const float (&v)[D / 8],
+                                               float m_nat, float l, bool write_ml, uint32_t xstep) {
+  // D / 8 consecutive head-dim values of one (sequence, q head) row: final output, packed form, or
   // tagged words into every rank's receive buffer
-  if (p.xch_world > 0) {
+  if (D == 128 && p.xch_world > 0) {
     for (int dest = 0; dest < p.xch_world; ++dest) {
       unsigned long long* dst = xch_row(p, dest, (int64_t)b * p.num_q_heads + hq, xstep);
 #pragma unroll
-      for (int t = 0; t < 16; t += 2) xch_store2(dst + d0 + t, v[t], v[t + 1], xstep);
-      if (write_ml) xch_store2(dst + 128, m_nat, l, xstep);
+      for (int t = 0; t < D / 8; t += 2) xch_store2(dst + d0 + t, v[t], v[t + 1], xstep);
+      if (write_ml) xch_store2(dst + D, m_nat, l, xstep);
     }
   } else if (p.packed_output != nullptr) {
-    float* dst = p.packed_output + ((int64_t)b * p.num_q_heads + hq) * 130 + d0;
+    float* dst = p.packed_output + ((int64_t)b * p.num_q_heads + hq) * (D + 2) + d0;
 #pragma unroll
-    for (int t = 0; t < 16; t += 2) *reinterpret_cast<float2*>(dst + t) = make_float2(v[t], v[t + 1]);
-    if (write_ml) { dst[128 - d0] = m_nat; dst[129 - d0] = l; }
+    for (int t = 0; t < D / 8; t += 2) *reinterpret_cast<float2*>(dst + t) = make_float2(v[t], v[t + 1]);
+    if (write_ml) { dst[D - d0] = m_nat; dst[D + 1 - d0] = l; }
   } else {
     const float inv = 1.f / l;
-    uint32_t w[8];
-#pragma unroll
-    for (int t = 0; t < 8; ++t) {
-      if constexpr (QBF16) {
-        __nv_bfloat162 x = __floats2bfloat162_rn(v[2 * t] * inv, v[2 * t + 1] * inv);
-        w[t] = *reinterpret_cast<uint32_t*>(&x);
-      } else {
-        w[t] = pack_f16x2(v[2 * t] * inv, v[2 * t + 1] * inv);
-      }
-    }
     uint16_t* dst = reinterpret_cast<uint16_t*>(p.output) + (int64_t)b * p.o_stride_b + (int64_t)hq * p.o_stride_h + d0;
-    *reinterpret_cast<uint2*>(dst) = make_uint2(w[0], w[1]);
-    *reinterpret_cast<uint2*>(dst + 4) = make_uint2(w[2], w[3]);
-    *reinterpret_cast<uint2*>(dst + 8) = make_uint2(w[4], w[5]);
-    *reinterpret_cast<uint2*>(dst + 12) = make_uint2(w[6], w[7]);
+#pragma unroll
+    for (int t = 0; t < D / 8; t += 4) {
+      uint32_t w[2];
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        if constexpr (QBF16) {
+          __nv_bfloat162 x = __floats2bfloat162_rn(v[t + 2 * e] * inv, v[t + 2 * e + 1] * inv);
+          w[e] = *reinterpret_cast<uint32_t*>(&x);
+        } else {
+          w[e] = pack_f16x2(v[t + 2 * e] * inv, v[t + 2 * e + 1] * inv);
+        }
+      }
+      *reinterpret_cast<uint2*>(dst + t) = make_uint2(w[0], w[1]);
+    }
   }
 }
 
@@ -341,15 +400,15 @@ __device__ __forceinline__ void kv16_load_q(uint32_t (&qb)[1][8][2], const Kerne
 // One step = two consecutive pages of one sequence, read from a stage [K0][K1][V0][V1] of
 // 4 KiB tiles (two swizzled halves each).  tok0 = token index of page 0's row 0.
 template <bool BF16>
-__device__ __forceinline__ void kv16_step(BalState<1>& st, uint32_t stage, const uint32_t (&qb)[1][8][2],
-                                          float scale_log2, int tok0, int lo, int hi, int lane) {
+__device__ __forceinline__ void kv16_step(BalState<1, 128>& st, uint32_t stage, const uint32_t (&qb)[1][8][2],
+                                          float scale_log2, float slack, int tok0, int lo, int hi, int lane) {
   constexpr uint32_t kTile = 2 * kPage * 128;
   const int i = lane >> 2, j = lane & 3;
   const int mid = lane >> 3, r8 = lane & 7;
   const bool edge = (tok0 < lo) | (tok0 + 2 * kPage > hi);
-  float s[2][4];
+  float s[1][2][4];
 #pragma unroll
-  for (int u = 0; u < 2; ++u) s[u][0] = s[u][1] = s[u][2] = s[u][3] = 0.f;
+  for (int u = 0; u < 2; ++u) s[0][u][0] = s[0][u][1] = s[0][u][2] = s[0][u][3] = 0.f;
   {
     // K: matrix `mid` of an x4 load = rows 8 (mid & 1) .., 16-byte chunk 2 ks + (mid >> 1)
     const int row = (mid & 1) * 8 + r8;
@@ -361,61 +420,47 @@ __device__ __forceinline__ void kv16_step(BalState<1>& st, uint32_t stage, const
       for (int u = 0; u < 2; ++u) {
         uint32_t a[4];
         ldsm_x4(stage + u * kTile + off, a);
-        mma_16816_kv16<BF16>(s[u], a, qb[0][ks][0], qb[0][ks][1]);
+        mma_16816_kv16<BF16>(s[0][u], a, qb[0][ks][0], qb[0][ks][1]);
       }
     }
   }
-  // scale + mask: s[u][c] is (token 16u + 8(c>>1) + i, head 2j + (c&1))
+  // mask: s[u][c] is (token 16u + 8(c>>1) + i, head 2j + (c&1))
+  uint32_t dead = 0u;  // bit 4u + c
+  if (edge) {
 #pragma unroll
-  for (int u = 0; u < 2; ++u)
+    for (int u = 0; u < 2; ++u)
 #pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      bool dead = false;
-      if (edge) {
+      for (int c = 0; c < 4; ++c) {
         const int tok = tok0 + u * kPage + 8 * (c >> 1) + i;
-        dead = (tok < lo) | (tok >= hi);
+        if ((tok < lo) | (tok >= hi)) {
+          dead |= 1u << (4 * u + c);
+          s[0][u][c] = -INFINITY;
+        }
       }
-      s[u][c] = dead ? -INFINITY : s[u][c] * scale_log2;
-    }
+  }
+  bal_raise_max<1, 8>(st.m, st.l, st.o, s, scale_log2, slack);
   // P^T B-fragments.  bf16 keeps 8 bits of a probability: there P goes in as two bf16 terms
   // (p = hi + lo, 16 bits together) and the PV product takes two MMAs; f16 keeps 11 bits.
   uint32_t pb[2][2], pl[2][2];
-  {
-    float mx[2], alpha[2];
 #pragma unroll
-    for (int e = 0; e < 2; ++e) {
-      float x = fmaxf(fmaxf(s[0][e], s[0][2 + e]), fmaxf(s[1][e], s[1][2 + e]));
-      x = fmaxf(x, __shfl_xor_sync(0xffffffffu, x, 4));
-      x = fmaxf(x, __shfl_xor_sync(0xffffffffu, x, 8));
-      x = fmaxf(x, __shfl_xor_sync(0xffffffffu, x, 16));
-      mx[e] = fmaxf(st.m[0][e], x);
-      alpha[e] = exp2f(st.m[0][e] - mx[e]);
-      st.m[0][e] = mx[e];
+  for (int u = 0; u < 2; ++u) {
+    float pr[4];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) pr[c] = exp2f(fmaf(s[0][u][c], scale_log2, -st.m[0][c & 1]));
+    if (edge) {
+#pragma unroll
+      for (int c = 0; c < 4; ++c)
+        if ((dead >> (4 * u + c)) & 1u) pr[c] = 0.f;
     }
-    float sum[2] = {0.f, 0.f};
-#pragma unroll
-    for (int u = 0; u < 2; ++u) {
-      const float p0 = exp2f(s[u][0] - mx[0]), p1 = exp2f(s[u][1] - mx[1]);
-      const float p2 = exp2f(s[u][2] - mx[0]), p3 = exp2f(s[u][3] - mx[1]);
-      sum[0] += p0 + p2;
-      sum[1] += p1 + p3;
-      // (token i, heads 2j, 2j+1) -> transpose -> (tokens 2j, 2j+1; head i)
-      pb[u][0] = movmatrix_trans(pack_kv16<BF16>(p0, p1));
-      pb[u][1] = movmatrix_trans(pack_kv16<BF16>(p2, p3));
-      if constexpr (BF16) {
-        const auto hi = [](float x) { return __bfloat162float(__float2bfloat16_rn(x)); };
-        pl[u][0] = movmatrix_trans(pack_kv16<true>(p0 - hi(p0), p1 - hi(p1)));
-        pl[u][1] = movmatrix_trans(pack_kv16<true>(p2 - hi(p2), p3 - hi(p3)));
-      }
-    }
-    st.l[0][0] = st.l[0][0] * alpha[0] + sum[0];
-    st.l[0][1] = st.l[0][1] * alpha[1] + sum[1];
-    if (__any_sync(0xffffffffu, (alpha[0] != 1.f) | (alpha[1] != 1.f))) {
-#pragma unroll
-      for (int mt = 0; mt < 8; ++mt) {
-        st.o[0][mt][0] *= alpha[0]; st.o[0][mt][1] *= alpha[1];
-        st.o[0][mt][2] *= alpha[0]; st.o[0][mt][3] *= alpha[1];
-      }
+    st.l[0][0] += pr[0] + pr[2];
+    st.l[0][1] += pr[1] + pr[3];
+    // (token i, heads 2j, 2j+1) -> transpose -> (tokens 2j, 2j+1; head i)
+    pb[u][0] = movmatrix_trans(pack_kv16<BF16>(pr[0], pr[1]));
+    pb[u][1] = movmatrix_trans(pack_kv16<BF16>(pr[2], pr[3]));
+    if constexpr (BF16) {
+      const auto hi = [](float x) { return __bfloat162float(__float2bfloat16_rn(x)); };
+      pl[u][0] = movmatrix_trans(pack_kv16<true>(pr[0] - hi(pr[0]), pr[1] - hi(pr[1])));
+      pl[u][1] = movmatrix_trans(pack_kv16<true>(pr[2] - hi(pr[2]), pr[3] - hi(pr[3])));
     }
   }
   // O^T += V^T P^T.  V^T fragments by transposing loads: matrix `mid` = tokens 8 (mid >> 1) ..,
@@ -805,12 +850,13 @@ __device__ __forceinline__ void write_empty_sequence(const KernelParams& p, int 
 // follows.  FUSED is a separate instantiation because the merge code costs the streaming loop
 // registers; on B200 it is the slower of the two (one warp per sequence and kv head merges
 // where the merge kernel has a warp per row).
-template <bool QBF16, int NSTAGE, int NWARPS, bool KV16 = false, bool FUSED = false>
+// D = 64 (e4m3 only): the same with 64-byte rows; see launch_decode for what runs it.
+template <bool QBF16, int NSTAGE, int NWARPS, bool KV16 = false, bool FUSED = false, int D = 128>
 __global__ void __launch_bounds__(NWARPS * 32, 1)
 paged_decode_fp8_chunk_kernel(const KernelParams p, const TmaParams tp, const ChunkParams cp,
                               const __grid_constant__ CUtensorMap tmap_k,
                               const __grid_constant__ CUtensorMap tmap_v) {
-  constexpr int D = 128;
+  static_assert(!(KV16 || FUSED) || D == 128, "not instantiated");
   constexpr int NT = NWARPS * 32;
   constexpr uint32_t kTile = (KV16 ? 2 : 1) * kPage * D;
   constexpr uint32_t kStage = 4 * kTile;
@@ -831,9 +877,9 @@ paged_decode_fp8_chunk_kernel(const KernelParams p, const TmaParams tp, const Ch
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, i = lane >> 2, j = lane & 3;
   const int B = cp.batch, hkv = p.num_kv_heads;
   const int page_first = p.kv_start / kPage;
-  const int W = (int)blockIdx.x * NWARPS + warp;
-  const int grp = W / hkv, kvh = W - grp * hkv;  // one warp per kv head and group
+  const int W = warp < cp.warps_per_cta ? (int)blockIdx.x * cp.warps_per_cta + warp : (int)gridDim.x * NWARPS;
   const int num_groups = cp.num_warps / hkv;
+  const int grp = W / hkv, kvh = W - grp * hkv;  // one warp per kv head and group
   const bool planned = cp.plan != nullptr;
 
   extern __shared__ uint8_t smem_raw[];
@@ -957,17 +1003,14 @@ paged_decode_fp8_chunk_kernel(const KernelParams p, const TmaParams tp, const Ch
   int ids_base = 0;
 
   // swizzled shared-memory offsets of this thread's fragments inside a tile
-  uint32_t k_off[2][2], v_off[4];
+  uint32_t k_off[2][D / 64], v_off[4];
 #pragma unroll
   for (int half = 0; half < 2; ++half)
 #pragma unroll
-    for (int l = 0; l < 2; ++l)
-      k_off[half][l] = (half * 8 + rho(i)) * D + (((j + 4 * l) ^ rho(i)) << 4);
+    for (int l = 0; l < D / 64; ++l) k_off[half][l] = bal_chunk<D>(half * 8 + rho(i), j + 4 * l);
 #pragma unroll
-  for (int r = 0; r < 4; ++r) {
-    const int row = v_row(j, r);
-    v_off[r] = row * D + ((i ^ (row & 7)) << 4);
-  }
+  for (int r = 0; r < 4; ++r)
+    v_off[r] = D == 128 ? bal_chunk<D>(bal_v_row<D>(j, r), i) : bal_chunk<D>(bal_v_row<D>(j, r), i >> 1) + 8 * (i & 1);
 
   // ---- consumer side: the pieces of the chunk in order
   struct Cursor { int b, np, start; };  // current sequence, its pairs, list index of its first pair
@@ -977,14 +1020,21 @@ paged_decode_fp8_chunk_kernel(const KernelParams p, const TmaParams tp, const Ch
   cur.start = prefix[cur.b];
   const float ks = KV16 ? 1.f : (p.k_scale_ph ? __ldg(p.k_scale_ph + kvh) : p.k_scale);
   const float vs = KV16 ? 1.f : (p.v_scale_ph ? __ldg(p.v_scale_ph + kvh) : p.v_scale);
-  const float scale_log2 = ks * p.sm_scale * kLog2e;
-  const auto load_q = [&](uint32_t (&dst)[1][8][2], int b) {
+  // The steps take maxima of raw scores, i.e. a scale that is not negative: a negative one's sign goes
+  // into the query.
+  const float scale_signed = ks * p.sm_scale * kLog2e;
+  const float scale_log2 = fabsf(scale_signed);
+  const uint32_t q_flip = scale_signed < 0.f ? 0x80008000u : 0u;
+  const float slack = p.max_slack;
+  const auto load_q = [&](uint32_t (&dst)[1][D / 16][2], int b) {
     if constexpr (KV16) kv16_load_q(dst, p, b, kvh, i, j);
-    else bal_load_q<QBF16, 1>(dst, p, b, kvh, i, j);
+    else bal_load_q<QBF16, 1, D>(dst, p, b, kvh, i, j);
+#pragma unroll
+    for (int f = 0; f < D / 16; ++f) { dst[0][f][0] ^= q_flip; dst[0][f][1] ^= q_flip; }
   };
-  uint32_t qb[1][8][2];
+  uint32_t qb[1][D / 16][2];
   load_q(qb, cur.b);
-  BalState<1> st;
+  BalState<1, D> st;
   bool ok = true;
   int t = 0;  // pairs consumed
   int g = P0;
@@ -994,7 +1044,7 @@ paged_decode_fp8_chunk_kernel(const KernelParams p, const TmaParams tp, const Ch
     const int piece_first = g;
     // the next piece's query is requested now and used when this piece is done
     Cursor nxt = cur;
-    uint32_t qn[1][8][2];
+    uint32_t qn[1][D / 16][2];
     if (e < P1) {
       do {  // sequences with nothing to attend have no pairs
         nxt.start += nxt.np;
@@ -1005,7 +1055,7 @@ paged_decode_fp8_chunk_kernel(const KernelParams p, const TmaParams tp, const Ch
     }
     const int seq_len = lens[cur.b];
     const bool whole = cur.start >= P0 && cur.start + cur.np <= P1;
-    bal_reset<1>(st);
+    bal_reset<1, D>(st);
 #pragma unroll 1
     for (; g < e; ++g, ++t) {
       const int s = t % NSTAGE;
@@ -1013,8 +1063,8 @@ paged_decode_fp8_chunk_kernel(const KernelParams p, const TmaParams tp, const Ch
       if (t == 0) mark_phase_at(tp, W, 3, lane == 0);  // first data landed
       if (t == n / 2) mark_phase_at(tp, W, 6, lane == 0);  // half of the chunk consumed
       const int tok0 = (page_first + 2 * (g - cur.start)) * kPage;
-      if constexpr (KV16) kv16_step<QBF16>(st, my_ring + s * kStage, qb, scale_log2, tok0, p.kv_start, seq_len, lane);
-      else bal_step<1>(st, my_ring + s * kStage, k_off, v_off, qb, scale_log2, tok0, p.kv_start, seq_len, i, j);
+      if constexpr (KV16) kv16_step<QBF16>(st, my_ring + s * kStage, qb, scale_log2, slack, tok0, p.kv_start, seq_len, lane);
+      else bal_step<1, D>(st, my_ring + s * kStage, k_off, v_off, qb, scale_log2, slack, tok0, p.kv_start, seq_len, i, j);
       // all reads of the stage fed MMAs above: hand it back to TMA for the chunk's pair t + NSTAGE
       __syncwarp();
       const int tn = t + NSTAGE;
@@ -1084,19 +1134,19 @@ paged_decode_fp8_chunk_kernel(const KernelParams p, const TmaParams tp, const Ch
           }
         }
       } else {
-        float v[16];
+        float v[D / 8];
 #pragma unroll
-        for (int mt = 0; mt < 8; ++mt) {
+        for (int mt = 0; mt < D / 16; ++mt) {
           v[2 * mt] = st.o[0][mt][c] * vs;
           v[2 * mt + 1] = st.o[0][mt][2 + c] * vs;
         }
         if (whole) {
-          store_row16<QBF16>(p, cur.b, hq, 16 * i, v, st.m[0][c] * kLn2, lsum[c], i == 0, xstep);
+          store_row_part<QBF16, D>(p, cur.b, hq, (D / 8) * i, v, st.m[0][c] * kLn2, lsum[c], i == 0, xstep);
         } else {
           const int64_t r = chunk_slot_row(grp, which, p.num_q_heads, hq);
-          float4* dst = reinterpret_cast<float4*>(reinterpret_cast<float*>(p.partial_output) + r * D + 16 * i);
+          float4* dst = reinterpret_cast<float4*>(reinterpret_cast<float*>(p.partial_output) + r * D + (D / 8) * i);
 #pragma unroll
-          for (int f = 0; f < 4; ++f) dst[f] = make_float4(v[4 * f], v[4 * f + 1], v[4 * f + 2], v[4 * f + 3]);
+          for (int f = 0; f < D / 32; ++f) dst[f] = make_float4(v[4 * f], v[4 * f + 1], v[4 * f + 2], v[4 * f + 3]);
           if (i == 0) {
             p.partial_max[r] = st.m[0][c] * kLn2;
             p.partial_sum[r] = lsum[c];
@@ -1150,7 +1200,7 @@ paged_decode_fp8_chunk_kernel(const KernelParams p, const TmaParams tp, const Ch
     }
     cur = nxt;
 #pragma unroll
-    for (int f = 0; f < 8; ++f) { qb[0][f][0] = qn[0][f][0]; qb[0][f][1] = qn[0][f][1]; }
+    for (int f = 0; f < D / 16; ++f) { qb[0][f][0] = qn[0][f][0]; qb[0][f][1] = qn[0][f][1]; }
   }
   mark_phase_at(tp, W, 4, lane == 0);  // chunk done
   mark_value_at(tp, W, 7, lane == 0, (unsigned long long)n);
@@ -1169,10 +1219,11 @@ paged_decode_fp8_chunk_kernel(const KernelParams p, const TmaParams tp, const Ch
 // the CTAs per SM the register budget is held to.  A row whose sequence lay inside one chunk
 // has been written already.  Same maths as _paged_split_kv_reduce
 // (integrations/vllm/l20_paged_split_kv.py:459-488).
-template <bool QBF16, int WPR, int KB, int MINB>
+template <bool QBF16, int WPR, int KB, int MINB, int D = 128>
 __global__ void __launch_bounds__(128, MINB)
 paged_decode_chunk_merge_kernel(const KernelParams p, const TmaParams tp, const ChunkParams cp) {
-  constexpr int D = 128, E = 4;
+  constexpr int E = D / 32;  // elements per lane
+  static_assert(E == 4 || E == 2, "head_dim 128 or 64");
   static_assert(WPR == 1 || WPR == 4, "one or four warps per row");
   pdl_launch_dependents();
   mark_phase_at(tp, cp.num_warps + blockIdx.x, 5, threadIdx.x == 0);  // merge CTA resident
@@ -1217,13 +1268,15 @@ paged_decode_chunk_merge_kernel(const KernelParams p, const TmaParams tp, const 
     if (keeper) pdl_wait();
     return;
   }
-  float acc[E] = {0.f, 0.f, 0.f, 0.f};
+  float acc[E];
+#pragma unroll
+  for (int e = 0; e < E; ++e) acc[e] = 0.f;
   float big = -INFINITY, den = 0.f;
   // pieces k0, k0 + WPR, ... (K of them) in one round trip, folded into (acc, big, den)
   auto round = [&](auto kc, int k0) {
     constexpr int K = decltype(kc)::value;
     float mv[K], lv[K];
-    float4 xv[K];
+    float xv[K][E];
 #pragma unroll
     for (int u = 0; u < K; ++u) {
       const int k = k0 + u * WPR;
@@ -1233,18 +1286,25 @@ paged_decode_chunk_merge_kernel(const KernelParams p, const TmaParams tp, const 
       mv[u] = on ? p.partial_max[r] : -INFINITY;
       lv[u] = on ? p.partial_sum[r] : 0.f;
       if (p.partial_dtype == 0) {
-        xv[u] = *reinterpret_cast<const float4*>(reinterpret_cast<const float*>(p.partial_output) + r * D + lane * E);
-      } else {
-        const uint2 raw = *reinterpret_cast<const uint2*>(reinterpret_cast<const uint16_t*>(p.partial_output) + r * D + lane * E);
-        if (p.partial_dtype == 1) {
-          const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&raw.x));
-          const float2 c = __half22float2(*reinterpret_cast<const __half2*>(&raw.y));
-          xv[u] = make_float4(a.x, a.y, c.x, c.y);
+        const float* src = reinterpret_cast<const float*>(p.partial_output) + r * D + lane * E;
+        if constexpr (E == 4) {
+          const float4 x = *reinterpret_cast<const float4*>(src);
+          xv[u][0] = x.x; xv[u][1] = x.y; xv[u][2] = x.z; xv[u][3] = x.w;
         } else {
-          const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.x));
-          const float2 c = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.y));
-          xv[u] = make_float4(a.x, a.y, c.x, c.y);
+          const float2 x = *reinterpret_cast<const float2*>(src);
+          xv[u][0] = x.x; xv[u][1] = x.y;
         }
+      } else if constexpr (E == 4) {  // (16-bit pieces: head_dim 128 only)
+        const uint2 raw = *reinterpret_cast<const uint2*>(reinterpret_cast<const uint16_t*>(p.partial_output) + r * D + lane * E);
+        float2 a, c;
+        if (p.partial_dtype == 1) {
+          a = __half22float2(*reinterpret_cast<const __half2*>(&raw.x));
+          c = __half22float2(*reinterpret_cast<const __half2*>(&raw.y));
+        } else {
+          a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.x));
+          c = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.y));
+        }
+        xv[u][0] = a.x; xv[u][1] = a.y; xv[u][2] = c.x; xv[u][3] = c.y;
       }
     }
     float m_new = big;
@@ -1258,7 +1318,8 @@ paged_decode_chunk_merge_kernel(const KernelParams p, const TmaParams tp, const 
     for (int u = 0; u < K; ++u) {
       const float c = (mv[u] == -INFINITY) ? 0.f : expf(mv[u] - m_new);
       den += lv[u] * c;
-      acc[0] += c * xv[u].x; acc[1] += c * xv[u].y; acc[2] += c * xv[u].z; acc[3] += c * xv[u].w;
+#pragma unroll
+      for (int e = 0; e < E; ++e) acc[e] += c * xv[u][e];
     }
     big = m_new;
   };
@@ -1274,27 +1335,32 @@ paged_decode_chunk_merge_kernel(const KernelParams p, const TmaParams tp, const 
     // combine the four warps' (acc, big, den) of this row; warp 0 finishes
     __shared__ __align__(16) float sh_acc[4][D];
     __shared__ float sh_m[4], sh_l[4];
-    *reinterpret_cast<float4*>(&sh_acc[warp][lane * E]) = make_float4(acc[0], acc[1], acc[2], acc[3]);
+#pragma unroll
+    for (int e = 0; e < E; e += 2) *reinterpret_cast<float2*>(&sh_acc[warp][lane * E + e]) = make_float2(acc[e], acc[e + 1]);
     if (lane == 0) { sh_m[warp] = big; sh_l[warp] = den; }
     __syncthreads();
     if (warp != 0) return;
     float m_all = fmaxf(fmaxf(sh_m[0], sh_m[1]), fmaxf(sh_m[2], sh_m[3]));
     den = 0.f;
-    acc[0] = acc[1] = acc[2] = acc[3] = 0.f;
+#pragma unroll
+    for (int e = 0; e < E; ++e) acc[e] = 0.f;
 #pragma unroll
     for (int w = 0; w < 4; ++w) {
       const float c = (sh_m[w] == -INFINITY) ? 0.f : expf(sh_m[w] - m_all);
-      const float4 x = *reinterpret_cast<const float4*>(&sh_acc[w][lane * E]);
       den += sh_l[w] * c;
-      acc[0] += c * x.x; acc[1] += c * x.y; acc[2] += c * x.z; acc[3] += c * x.w;
+#pragma unroll
+      for (int e = 0; e < E; e += 2) {
+        const float2 x = *reinterpret_cast<const float2*>(&sh_acc[w][lane * E + e]);
+        acc[e] += c * x.x; acc[e + 1] += c * x.y;
+      }
     }
     big = m_all;
   }
-  if (p.xch_world > 0) {
+  if (D == 128 && p.xch_world > 0) {
     for (int dest = 0; dest < p.xch_world; ++dest) {
       unsigned long long* dst = xch_row(p, dest, row, xstep);
-      xch_store2(dst + lane * E, acc[0], acc[1], xstep);
-      xch_store2(dst + lane * E + 2, acc[2], acc[3], xstep);
+#pragma unroll
+      for (int e = 0; e < E; e += 2) xch_store2(dst + lane * E + e, acc[e], acc[e + 1], xstep);
       if (lane == 0) xch_store2(dst + D, big, den, xstep);
     }
     mark_phase_at(tp, cp.num_warps + blockIdx.x, 7, threadIdx.x == 0);  // merged and sent
@@ -1302,25 +1368,26 @@ paged_decode_chunk_merge_kernel(const KernelParams p, const TmaParams tp, const 
   }
   if (p.packed_output != nullptr) {
     float* dst = p.packed_output + (int64_t)row * (D + 2);
-    *reinterpret_cast<float2*>(dst + lane * E) = make_float2(acc[0], acc[1]);
-    *reinterpret_cast<float2*>(dst + lane * E + 2) = make_float2(acc[2], acc[3]);
+#pragma unroll
+    for (int e = 0; e < E; e += 2) *reinterpret_cast<float2*>(dst + lane * E + e) = make_float2(acc[e], acc[e + 1]);
     if (lane == 0) { dst[D] = big; dst[D + 1] = den; }
     return;
   }
   mark_phase_at(tp, cp.num_warps + blockIdx.x, 7, threadIdx.x == 0);  // merged
   const float inv = ns > 0 ? 1.f / den : 0.f;
   uint16_t* dst = reinterpret_cast<uint16_t*>(p.output) + (int64_t)b * p.o_stride_b + (int64_t)hq * p.o_stride_h + lane * E;
-  uint32_t w0, w1;
-  if constexpr (QBF16) {
-    __nv_bfloat162 x = __floats2bfloat162_rn(acc[0] * inv, acc[1] * inv);
-    __nv_bfloat162 y = __floats2bfloat162_rn(acc[2] * inv, acc[3] * inv);
-    w0 = *reinterpret_cast<uint32_t*>(&x);
-    w1 = *reinterpret_cast<uint32_t*>(&y);
-  } else {
-    w0 = pack_f16x2(acc[0] * inv, acc[1] * inv);
-    w1 = pack_f16x2(acc[2] * inv, acc[3] * inv);
+  uint32_t w[E / 2];
+#pragma unroll
+  for (int e = 0; e < E; e += 2) {
+    if constexpr (QBF16) {
+      __nv_bfloat162 x = __floats2bfloat162_rn(acc[e] * inv, acc[e + 1] * inv);
+      w[e / 2] = *reinterpret_cast<uint32_t*>(&x);
+    } else {
+      w[e / 2] = pack_f16x2(acc[e] * inv, acc[e + 1] * inv);
+    }
   }
-  *reinterpret_cast<uint2*>(dst) = make_uint2(w0, w1);
+  if constexpr (E == 4) *reinterpret_cast<uint2*>(dst) = make_uint2(w[0], w[1]);
+  else *reinterpret_cast<uint32_t*>(dst) = w[0];
 }
 
 }  // namespace pfd

@@ -54,6 +54,7 @@ struct KernelParams {
   int32_t num_q_heads, num_kv_heads, group;
   int32_t split_size, kv_start;
   int32_t partial_dtype;
+  float max_slack;     // how far (log2 units) a score may lie above the running maximum before that is raised
   int32_t direct_out;  // 1: a sequence with a single split writes its final result itself
   int32_t bt_cols;     // width of a block-table row
   int32_t slot_offset; // workspace slots [0, slot_offset) are filled by another kernel (dense prefix pass)
@@ -262,23 +263,29 @@ __device__ __forceinline__ void qk_scores(float (&s)[NT][4], const uint32_t (&k)
   }
 }
 
-// Scale, mask, online softmax over NT/2 pages; rescales O and returns P as the f16 A-fragments
-// of the PV MMAs (pa[t] for page t).  Column tile nt covers tokens tok0 + 8*nt + rho(.).
+// Mask, scale, online softmax over NT/2 pages of raw scores; rescales O when it has to and returns P as
+// the f16 A-fragments of the PV MMAs (pa[t] for page t).  Column tile nt covers tokens
+// tok0 + 8*nt + rho(.).  The running maximum only has to keep the exponentials in range: it is raised
+// when a score lies more than `slack` (log2 units) above it, and a probability of up to 2^slack
+// against a stale one is as exact in f16 as one of up to 1.  So after a warp's first step the
+// shuffles, the rescaling factors and the rescaling hardly ever run, and with no slack in a few steps only.  scale_log2 >= 0
+// (a negative scale's sign is in the query, see load_q_frags).
 template <int D, int NT>
 __device__ __forceinline__ void softmax_step(WarpState<D>& st, float (&s)[NT][4],
-                                             uint32_t (&pa)[NT / 2][4], float scale_log2, bool edge,
+                                             uint32_t (&pa)[NT / 2][4], float scale_log2, float slack, bool edge,
                                              int tok0, int lo, int hi, int j) {
+  uint32_t dead = 0u;  // bit 2 nt + (c & 1)
+  if (edge) {
 #pragma unroll
-  for (int nt = 0; nt < NT; ++nt) {
+    for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      float x = s[nt][c] * scale_log2;
-      if (edge) {
-        const int tok = tok0 + nt * 8 + rho(2 * j + (c & 1));
-        if (tok < lo || tok >= hi) x = -INFINITY;
+      for (int e = 0; e < 2; ++e) {
+        const int tok = tok0 + nt * 8 + rho(2 * j + e);
+        if (tok < lo || tok >= hi) {
+          dead |= 1u << (2 * nt + e);
+          s[nt][e] = s[nt][2 + e] = -INFINITY;
+        }
       }
-      s[nt][c] = x;
-    }
   }
   float mx0 = fmaxf(s[0][0], s[0][1]), mx1 = fmaxf(s[0][2], s[0][3]);
 #pragma unroll
@@ -286,35 +293,41 @@ __device__ __forceinline__ void softmax_step(WarpState<D>& st, float (&s)[NT][4]
     mx0 = fmaxf(mx0, fmaxf(s[nt][0], s[nt][1]));
     mx1 = fmaxf(mx1, fmaxf(s[nt][2], s[nt][3]));
   }
-  mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, 1));
-  mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 1));
-  mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, 2));
-  mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 2));
-  const float mn0 = fmaxf(st.m[0], mx0);
-  const float mn1 = fmaxf(st.m[1], mx1);
-  const float alpha0 = exp2f(st.m[0] - mn0);
-  const float alpha1 = exp2f(st.m[1] - mn1);
-  st.m[0] = mn0;
-  st.m[1] = mn1;
-  float sum0 = 0.f, sum1 = 0.f;
-#pragma unroll
-  for (int nt = 0; nt < NT; ++nt) {
-    const float p0 = exp2f(s[nt][0] - mn0), p1 = exp2f(s[nt][1] - mn0);
-    const float p2 = exp2f(s[nt][2] - mn1), p3 = exp2f(s[nt][3] - mn1);
-    sum0 += p0 + p1;
-    sum1 += p2 + p3;
-    pa[nt >> 1][(nt & 1) * 2 + 0] = pack_f16x2(p0, p1);
-    pa[nt >> 1][(nt & 1) * 2 + 1] = pack_f16x2(p2, p3);
-  }
-  st.l[0] = st.l[0] * alpha0 + sum0;
-  st.l[1] = st.l[1] * alpha1 + sum1;
-  // the running max rarely moves after the first tiles: skip the 4*D/8 multiplies then
-  if (__any_sync(0xffffffffu, (alpha0 != 1.f) | (alpha1 != 1.f))) {
+  mx0 *= scale_log2;
+  mx1 *= scale_log2;
+  if (__any_sync(0xffffffffu, (mx0 > st.m[0] + slack) | (mx1 > st.m[1] + slack))) {
+    mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, 1));
+    mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 1));
+    mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, 2));
+    mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 2));
+    const float mn0 = fmaxf(st.m[0], mx0);
+    const float mn1 = fmaxf(st.m[1], mx1);
+    const float alpha0 = exp2f(st.m[0] - mn0);
+    const float alpha1 = exp2f(st.m[1] - mn1);
+    st.m[0] = mn0;
+    st.m[1] = mn1;
+    st.l[0] *= alpha0;
+    st.l[1] *= alpha1;
 #pragma unroll
     for (int m = 0; m < D / 8; ++m) {
       st.o[m][0] *= alpha0; st.o[m][1] *= alpha0;
       st.o[m][2] *= alpha1; st.o[m][3] *= alpha1;
     }
+  }
+#pragma unroll
+  for (int nt = 0; nt < NT; ++nt) {
+    float pr[4];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) pr[c] = exp2f(fmaf(s[nt][c], scale_log2, -st.m[c >> 1]));
+    if (edge) {
+#pragma unroll
+      for (int c = 0; c < 4; ++c)
+        if ((dead >> (2 * nt + (c & 1))) & 1u) pr[c] = 0.f;
+    }
+    st.l[0] += pr[0] + pr[1];
+    st.l[1] += pr[2] + pr[3];
+    pa[nt >> 1][(nt & 1) * 2 + 0] = pack_f16x2(pr[0], pr[1]);
+    pa[nt >> 1][(nt & 1) * 2 + 1] = pack_f16x2(pr[2], pr[3]);
   }
 }
 
@@ -351,21 +364,22 @@ __device__ __forceinline__ void pv_accumulate(WarpState<D>& st, uint32_t (&v)[4]
 
 template <int D>
 __device__ __forceinline__ void consume_tile(WarpState<D>& st, TileRegs<D>& t,
-                                             const uint32_t (&qa)[D / 16][4], float scale_log2,
+                                             const uint32_t (&qa)[D / 16][4], float scale_log2, float slack,
                                              int tok0, int lo, int hi, int j) {
   float s[2][4];
   uint32_t pa[1][4];
   const bool edge = (tok0 < lo) | (tok0 + kPage > hi);
   qk_scores<D, 2>(s, t.k, qa);
-  softmax_step<D, 2>(st, s, pa, scale_log2, edge, tok0, lo, hi, j);
+  softmax_step<D, 2>(st, s, pa, scale_log2, slack, edge, tok0, lo, hi, j);
   pv_accumulate<D>(st, t.v, pa[0], edge, tok0, lo, hi, j);
 }
 
 // Q rows i and i+8 of the kv head's group as f16 A-fragments, d permuted to match the K loads:
-// k-step ks = 4l + w covers d = 16*(j+4l) + 4w + {0,1 | 2,3}.
+// k-step ks = 4l + w covers d = 16*(j+4l) + 4w + {0,1 | 2,3}.  `flip` is XOR-ed into every pair (the
+// signs, where the softmax scale is negative).
 template <int D, bool QBF16>
 __device__ __forceinline__ void load_q_frags(uint32_t (&qa)[D / 16][4], const KernelParams& p, int b,
-                                             int kvh, int i, int j) {
+                                             int kvh, int i, int j, uint32_t flip) {
 #pragma unroll
   for (int half = 0; half < 2; ++half) {
     const int row = i + 8 * half;
@@ -385,8 +399,8 @@ __device__ __forceinline__ void load_q_frags(uint32_t (&qa)[D / 16][4], const Ke
           lo = pack_f16x2(__bfloat162float(a.x), __bfloat162float(a.y));
           hi = pack_f16x2(__bfloat162float(c.x), __bfloat162float(c.y));
         }
-        qa[l * 4 + w][half] = lo;       // a0 / a1 : k = 2j, 2j+1
-        qa[l * 4 + w][2 + half] = hi;   // a2 / a3 : k = 2j+8, 2j+9
+        qa[l * 4 + w][half] = lo ^ flip;       // a0 / a1 : k = 2j, 2j+1
+        qa[l * 4 + w][2 + half] = hi ^ flip;   // a2 / a3 : k = 2j+8, 2j+9
       }
     }
   }
@@ -550,10 +564,11 @@ paged_decode_fp8_partial_ldg_kernel(const KernelParams p) {
   __shared__ __align__(16) float sm_o[NWARPS * 16 * D];
 
   uint32_t qa[D / 16][4];
-  load_q_frags<D, QBF16>(qa, p, b, kvh, i, j);
   const float ks = p.k_scale_ph ? __ldg(p.k_scale_ph + kvh) : p.k_scale;
   const float vs = p.v_scale_ph ? __ldg(p.v_scale_ph + kvh) : p.v_scale;
-  const float scale_log2 = ks * p.sm_scale * kLog2e;
+  const float scale_signed = ks * p.sm_scale * kLog2e;
+  const float scale_log2 = fabsf(scale_signed);
+  load_q_frags<D, QBF16>(qa, p, b, kvh, i, j, scale_signed < 0.f ? 0x80008000u : 0u);
 
   WarpState<D> st;
 #pragma unroll
@@ -579,7 +594,7 @@ paged_decode_fp8_partial_ldg_kernel(const KernelParams p) {
       load_tile_global<D>(nxt, kbase + phys * p.k_stride_page, vbase + phys * p.v_stride_page,
                           p.k_stride_token, p.v_stride_token, i, j);
     }
-    consume_tile<D>(st, cur, qa, scale_log2, pg * kPage, lo, hi, j);
+    consume_tile<D>(st, cur, qa, scale_log2, p.max_slack, pg * kPage, lo, hi, j);
     cur = nxt;
   }
   cta_merge_and_store<D, QBF16, NWARPS>(st, p, b, kvh, split + p.slot_offset, nsplits_seq, vs, sm_m, sm_l, sm_o);
@@ -937,10 +952,11 @@ paged_decode_fp8_partial_tma_kernel(const KernelParams p, const TmaParams tp,
   dbg_mark(dbg_slot, 3, threadIdx.x == 0);  // first copies issued
 
   uint32_t qa[D / 16][4];
-  load_q_frags<D, QBF16>(qa, p, b, kvh, i, j);
   const float ks = p.k_scale_ph ? __ldg(p.k_scale_ph + kvh) : p.k_scale;
   const float vs = p.v_scale_ph ? __ldg(p.v_scale_ph + kvh) : p.v_scale;
-  const float scale_log2 = ks * p.sm_scale * kLog2e;
+  const float scale_signed = ks * p.sm_scale * kLog2e;
+  const float scale_log2 = fabsf(scale_signed);
+  load_q_frags<D, QBF16>(qa, p, b, kvh, i, j, scale_signed < 0.f ? 0x80008000u : 0u);
 
   WarpState<D> st;
 #pragma unroll
@@ -985,7 +1001,7 @@ paged_decode_fp8_partial_tma_kernel(const KernelParams p, const TmaParams tp,
         }
       qk_scores<D, 4>(sc, k, qa);
     }
-    softmax_step<D, 4>(st, sc, pa, scale_log2, edge, tok0, lo, hi, j);
+    softmax_step<D, 4>(st, sc, pa, scale_log2, p.max_slack, edge, tok0, lo, hi, j);
 #pragma unroll
     for (int u = 0; u < 2; ++u) {
       uint32_t v[4][4];

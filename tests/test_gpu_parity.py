@@ -524,3 +524,61 @@ def test_cuda_graph_capture_and_replay(built_libs):
         graph.replay()
     torch.cuda.synchronize()
     assert_within_gate(ws[3], exp, "graph replay")
+
+
+# ---------------------------------------------------------------- balanced kernel, head_dim 64
+@pytest.mark.parametrize("layout", ["nhd", "hnd"])
+@pytest.mark.parametrize("d,hq,hkv", [(64, 14, 2), (64, 8, 1), (64, 8, 8), (64, 6, 3), (64, 9, 1)])
+def test_balanced_kernel_with_head_dim_64(cabi, d, hq, hkv, layout):
+    """Batches large enough for the balanced kernel: every length around a page and a page pair, empty and long sequences,
+    unaligned kv_start, packed output, NaN bytes in the unused slots, a workspace with room for all warp groups and for
+    three quarters of them; and what the grid keeps: less room, nine heads per KV head, the fixed-split flag."""
+    gen = torch.Generator().manual_seed(d + hq)
+    batch, longest = 200, 700
+    lens = torch.cat([torch.arange(0, 70), torch.randint(1, longest + 1, (batch - 72,), generator=gen),
+                      torch.tensor([longest, longest - 1])]).to(torch.int32)
+    pages_of = (lens + 15) // 16
+    total = int(pages_of.sum()) + 1
+    table = torch.full((batch, -(-longest // 16)), total - 1, dtype=torch.int32)
+    free = torch.randperm(total - 1, generator=gen).to(torch.int32)
+    at = 0
+    for b, n in enumerate(pages_of.tolist()):
+        table[b, :n] = free[at:at + n]
+        at += n
+    kc, ks = oracle.quantize_fp8_e4m3_per_head(torch.randn(total, 16, hkv, d, generator=gen))
+    vc, vs = oracle.quantize_fp8_e4m3_per_head(torch.randn(total, 16, hkv, d, generator=gen))
+    q = torch.randn(batch, hq, d, generator=gen).to(torch.bfloat16)
+    for c in (kc, vc):  # what no sequence owns: NaN
+        for b, n in enumerate(lens.tolist()):
+            if n % 16:
+                c.view(torch.uint8)[table[b, n // 16], n % 16:] = 0x7F
+        c.view(torch.uint8)[total - 1] = 0x7F
+    g = [t.to(DEV) for t in (q, kc, vc, table, lens)]
+    if layout == "hnd":
+        g[1:3] = [t.permute(0, 2, 1, 3).contiguous().permute(0, 2, 1, 3) for t in g[1:3]]
+    all_rows = 2 * (148 * 16 // hkv) * hq
+    for kv_start in (0, 21):
+        live = lens > kv_start
+        exp = torch.zeros(batch, hq, d)
+        for b in live.nonzero()[:, 0].tolist():
+            one = slice(b, b + 1)
+            exp[b] = oracle.reference_fp32(q[one], kc, vc, table[one].long(), lens[one], ks, vs, kv_start=kv_start)[0]
+        for rows, flags, packed in ((all_rows + 2 * hq, 0, False), (3 * all_rows // 4 + 2 * hq, EARLY, False), (all_rows + 2 * hq, 0, True), (0, 0, False),
+                                    (all_rows, 8, False)):
+            ws = workspace(g[0], longest, 512, kv_start=kv_start, min_rows=rows)
+            out = torch.full_like(g[0], float("nan"))
+            pk = torch.full((batch, hq, d + 2), float("nan"), device=DEV) if packed else None
+            cabi.paged_decode_fp8_e4m3_split_out(
+                *g, k_scale=ks.to(DEV), v_scale=vs.to(DEV), max_seq_len=longest, split_size=512, output=None if packed else out,
+                packed_output=pk, workspace=ws, kv_start=kv_start, flags=flags)
+            torch.cuda.synchronize()
+            assert cabi.device_status() == 0
+            what = f"d={d} hq={hq} hkv={hkv} {layout} kv_start={kv_start} rows={rows} flags={flags} packed={packed}"
+            room = batch * ws[0].shape[2] // 2
+            grid = flags & 8 or hq // hkv > 8 or 4 * room < 3 * (148 * 16 // hkv)
+            assert cabi.last_path() == (PATH_LDG if grid else PATH_BALANCED), what
+            if packed:
+                o, m, l = pk[..., :d], pk[..., d], pk[..., d + 1]
+                assert torch.equal(l.cpu() > 0, live[:, None].expand(batch, hq)), what
+                out = torch.where(l[..., None] > 0, o / l[..., None], 0.0).to(q.dtype)
+            assert_within_gate(out, exp.to(q.dtype), what)
