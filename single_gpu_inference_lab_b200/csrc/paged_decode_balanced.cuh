@@ -41,10 +41,14 @@ struct ChunkParams {
 // sequence up (query fetch, state reset, output rows), then two units per page pair.  The cost
 // axis is cut into `groups` contiguous chunks whose lengths differ by at most one unit, and a
 // page pair belongs to the chunk that holds its first unit.  Tiny workloads use fewer groups so
-// that no chunk is shorter than kMinChunkCost units (a chunk inside a sequence is never empty).
+// that no chunk is shorter than kMinChunkCost units (a chunk inside a sequence is never empty): two page
+// pairs, since a warp's pairs are one chain of some 0.8 us each while more pieces cost the merge
+// less.  us per call, 16 + 2 heads, at a minimum of 8 / 6 / 4 / 2 units, lengths uniform up to the second
+// number: 1 x 512 10.3 / 9.4 / 8.2 / 7.3   8 x 1024 11.2 / 10.0 / 9.6 / 9.0   64 x 256 12.1 / 11.3 / 10.7 / 10.4
+// 1 x 8192 12.3 / 12.2 / 12.2 / 15.4   64 x 1024 13.6 / 12.7 / 11.9 / 12.0   256 x 512 17.2 / 17.3 / 17.2 / 17.3.
 // (Cutting at page granularity, a pair shared by two chunks that each attend one of its pages,
 // balances bytes better but was measured slower: the shared pairs cost both chunks a step.)
-constexpr int kMinChunkCost = 8;
+constexpr int kMinChunkCost = 4;
 struct Chunking {
   int base, rem, groups, piece_cost;
   __device__ __forceinline__ Chunking(int total_pairs, int batch, int max_groups, int cost) : piece_cost(cost) {

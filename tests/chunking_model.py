@@ -19,7 +19,7 @@ from dataclasses import dataclass
 PAGE = 16
 WARPS_PER_SM = 8
 PIECE_COST = 2
-MIN_CHUNK_COST = 8
+MIN_CHUNK_COST = 4
 
 
 def pairs_of(seq_len: int, kv_start: int = 0) -> int:
