@@ -60,6 +60,8 @@ def l20_rope_and_cache(
 
         def vec(s):
             if isinstance(s, torch.Tensor):
+                if s.dtype == torch.float32 and s.device == query.device and s.shape == (hkv,) and s.is_contiguous():
+                    return s  # the common case costs nothing
                 return s.to(device=query.device, dtype=torch.float32).reshape(-1).expand(hkv).contiguous()
             return _scale_vector(s, hkv, query.device)
 
