@@ -179,6 +179,62 @@ def test_graph_replay_with_metadata_rewritten_in_place(built_libs, kv16, planned
         assert_within_gate(ws[3], exp, f"replay {step} kv16={kv16}")
 
 
+@pytest.mark.parametrize("early", [False, True])
+@pytest.mark.parametrize("fused", [False, True])
+@pytest.mark.parametrize("kv16", [False, True])
+def test_plan_right_in_front_of_the_first_layer(built_libs, kv16, fused, early):
+    """A recorded step whose first call follows the plan kernel with nothing in between, lengths and table rewritten before
+    every replay, replays queued behind one another: each must read its own plan.  ``early``: the first call reads the plan
+    before its dependency wait too, so the plan kernel must not let it in before the plan is written."""
+    from single_gpu_inference_lab_b200 import l20_paged_split_kv as m
+
+    torch.manual_seed(6)
+    batch, hq, hkv, max_len, replays = 24, 16, 2, 900, 12
+    pages_per = -(-max_len // 16)
+    total = batch * pages_per
+    dtype = torch.bfloat16
+    k, v = torch.randn(total, 16, hkv, 128), torch.randn(total, 16, hkv, 128)
+    if kv16:
+        kc, vc, ks, vs = k.to(dtype), v.to(dtype), None, None
+    else:
+        (kc, ks), (vc, vs) = oracle.quantize_fp8_e4m3_per_head(k), oracle.quantize_fp8_e4m3_per_head(v)
+    q = torch.randn(batch, hq, 128).to(dtype)
+    lens = torch.randint(1, max_len + 1, (replays, batch)).to(torch.int32)
+    lens[3] = max_len
+    lens[4] = 1
+    tables = torch.stack([torch.randperm(total).to(torch.int32).reshape(batch, pages_per) for _ in range(replays)])
+    gq, gk, gv, glens, gtables = (t.to(DEV) for t in (q, kc, vc, lens, tables))
+    scales = {} if kv16 else dict(k_scale=ks.to(DEV), v_scale=vs.to(DEV))
+    attend = m.l20_paged_split_kv_attention if kv16 else m.l20_paged_split_kv_attention_fp8
+    table, lengths = gtables[0].clone(), glens[0].clone()
+    ws = m.allocate_l20_paged_split_kv_workspace(gq, max_len, split_size=512, num_kv_heads=hkv)
+    plan = m.plan_l20_paged_split_kv(gq, gk, gv, table, lengths, max_seq_len=max_len, split_size=512, workspace=ws)
+    outs = [torch.empty_like(gq) for _ in range(2)]
+
+    def step():
+        m.plan_l20_paged_split_kv(gq, gk, gv, table, lengths, max_seq_len=max_len, split_size=512, workspace=ws, plan=plan)
+        for layer, out in enumerate(outs):
+            attend(gq, gk, gv, table, lengths, split_size=512, workspace=ws, max_seq_len=max_len, plan=plan, output=out,
+                   metadata_stable=early or layer > 0, single_launch=fused, **scales)
+
+    step()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        step()
+    got = []
+    for r in range(replays):  # (no wait in between: the host stays ahead of the device)
+        table.copy_(gtables[r])
+        lengths.copy_(glens[r])
+        graph.replay()
+        got.append([out.clone() for out in outs])
+    torch.cuda.synchronize()
+    for r in range(replays):
+        exp = expected(q, kc, vc, tables[r], lens[r], ks, vs)
+        for layer, out in enumerate(got[r]):
+            assert_within_gate(out, exp, f"replay {r} layer {layer} kv16={kv16} fused={fused} early={early}")
+
+
 @pytest.mark.parametrize("flags,d", [(8, 128), (1, 128), (0, 64)])
 def test_random_cases_fixed_split_grid(cabi, flags, d):
     """The same for the fixed-split grid (TMA and plain loads) and head_dim 64, small split sizes."""
