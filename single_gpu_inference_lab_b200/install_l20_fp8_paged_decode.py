@@ -276,7 +276,9 @@ CALL_NEW = """                else:
                             split_size=512,
                             output=out_decode.view_as(decode_query),
                             workspace=l20_step.workspace,
-                            metadata_stable=True,  # built once per model step
+                            # built once per model step: metadata_stable=True, but not for
+                            # the layer whose call follows the plan kernel
+                            metadata_stable=l20_step.metadata_stable,
                             kv_stable=l20_static["early_kv"],
                             plan=l20_step.plan,
                         )
@@ -307,7 +309,7 @@ CALL_NEW = """                else:
                             workspace=l20_step.workspace,
                             max_seq_len=l20_fp8_max_seq,
                             output=out_decode.view_as(decode_query),
-                            metadata_stable=True,
+                            metadata_stable=l20_step.metadata_stable,
                             kv_stable=l20_static["early_kv"],
                             plan=l20_step.plan,
                         )

@@ -39,6 +39,7 @@ PREFIX_CHUNK = 256
 class DecodeStep:
     workspace: tuple
     plan: Optional[torch.Tensor] = None
+    metadata_stable: bool = True       # False for the layer whose call follows the plan kernel: it must not read the plan early
     groups: object = None              # PrefixGroups when this step takes the grouped path
     prefix_workspace: Optional[tuple] = None
     suffix_split: int = 512            # split size of the grouped path's split-KV pass
@@ -77,6 +78,7 @@ def l20_decode_step(meta, query, key_cache, value_cache, block_tables, seq_lens,
     """The step's shared state: computed by the first layer of a step, kept on ``meta.l20_step``."""
     step = getattr(meta, "l20_step", None)
     if step is not None:
+        step.metadata_stable = True  # a later layer: its own kernels have run since the plan was made
         return step
     from . import l20_paged_decode as ops
     from .l20_paged_split_kv import allocate_l20_paged_split_kv_workspace, plan_l20_paged_split_kv
@@ -98,6 +100,7 @@ def l20_decode_step(meta, query, key_cache, value_cache, block_tables, seq_lens,
                                                 plan=plan_buffer)
         except RuntimeError:
             step.plan = None  # this shape does not run the balanced kernel: the calls go without a plan
+    step.metadata_stable = step.plan is None
     capturing = torch.cuda.is_current_stream_capturing()
     if fp8 and sw["shared_prefix"] and head_dim == 128 and MIN_GROUP_BATCH <= batch <= 2048 and max_seq_len >= MIN_PREFIX_TOKENS \
             and (not capturing or sw["shared_prefix_force"]):

@@ -47,7 +47,7 @@ def test_plan_and_workspace_are_made_once_per_step_and_shared_by_the_layers(buil
             assert step is meta.l20_step and step.plan is not None and step.groups is None
             out = m.l20_paged_split_kv_attention_fp8(g.query, kc, vc, g.block_table, g.seq_lens, k_scale=g.k_scale, v_scale=g.v_scale,
                                                      max_seq_len=w.max_seq_len, split_size=512, workspace=step.workspace,
-                                                     metadata_stable=True, plan=step.plan, output=torch.empty_like(g.query))
+                                                     metadata_stable=step.metadata_stable, plan=step.plan, output=torch.empty_like(g.query))
             torch.cuda.synchronize()
             assert_within_gate(out, exp, "planned layer")
         steps.append(meta.l20_step)
@@ -95,3 +95,42 @@ def test_a_step_with_shared_prefix_groups_takes_the_grouped_operator_and_is_trac
     step = mod.l20_decode_step(meta, other.query, other.key_cache, other.value_cache, other.block_table, other.seq_lens,
                                other.max_seq_len)
     assert step.groups is None
+
+
+def test_a_recorded_step_in_the_hooks_order_reads_its_own_plan(built_libs, monkeypatch):
+    """Plan and layers recorded as the hook calls them, nothing between the plan and the first layer; lengths and table
+    rewritten before every replay."""
+    mod = _fresh(monkeypatch)
+    from single_gpu_inference_lab_b200 import l20_paged_split_kv as m
+
+    w = make_inputs("qwen2.5-coder-3b-b64", seed=35, batch=16, shrink=0.25)
+    g = w.to(DEV)
+    gen = torch.Generator().manual_seed(36)
+    pages, width = w.key_cache.shape[0], w.block_table.shape[1]
+    outs = [torch.empty_like(g.query) for _ in range(2)]
+
+    def step():
+        meta = SimpleNamespace(l20_step=None)
+        for layer, out in enumerate(outs):
+            state = mod.l20_decode_step(meta, g.query, g.key_cache, g.value_cache, g.block_table, g.seq_lens, w.max_seq_len)
+            assert state.plan is not None and state.metadata_stable == (layer > 0)
+            m.l20_paged_split_kv_attention_fp8(
+                g.query, g.key_cache, g.value_cache, g.block_table, g.seq_lens, k_scale=g.k_scale, v_scale=g.v_scale,
+                max_seq_len=w.max_seq_len, split_size=512, workspace=state.workspace, metadata_stable=state.metadata_stable,
+                plan=state.plan, output=out)
+
+    step()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        step()
+    for replay in range(6):
+        lens = torch.randint(1, w.max_seq_len + 1, w.seq_lens.shape, generator=gen).to(torch.int32)
+        table = torch.randint(0, pages, (w.seq_lens.shape[0], width), generator=gen).to(torch.int32)
+        g.seq_lens.copy_(lens)
+        g.block_table.copy_(table)
+        graph.replay()
+        torch.cuda.synchronize()
+        exp = oracle.reference(w.query, w.key_cache, w.value_cache, table.long(), lens, w.k_scale, w.v_scale)
+        for layer, out in enumerate(outs):
+            assert_within_gate(out, exp, f"replay {replay} layer {layer}")

@@ -164,3 +164,34 @@ def test_rope_hook_installs_compiles_and_uninstalls(tmp_path, built_libs, capsys
     ast.parse(backend.read_text())
     assert rope_installer.main(["--vllm-source-dir", str(root), "--uninstall"]) == 0
     assert (backend.read_text(), config.read_text()) == originals
+
+
+def test_only_the_layer_behind_the_plan_kernel_keeps_from_reading_the_plan_early(monkeypatch):
+    """``metadata_stable`` lets a call read the plan before the kernel in front of it has completed: not the call that
+    follows the plan kernel."""
+    from types import SimpleNamespace
+
+    import torch
+
+    from single_gpu_inference_lab_b200 import l20_decode_step as mod
+    from single_gpu_inference_lab_b200 import l20_paged_split_kv
+
+    assert installer.CALL_NEW.count("metadata_stable=l20_step.metadata_stable") == 2
+    assert "metadata_stable=True," not in installer.CALL_NEW.replace("metadata_stable=True, but not", "")
+    made = []
+    monkeypatch.setattr(mod, "_SWITCHES", {"shared_prefix": False, "shared_prefix_force": False, "trace": None, "no_plan": False})
+    monkeypatch.setattr(mod, "_BUFFERS", {})
+    monkeypatch.setattr(mod.torch.cuda, "is_current_stream_capturing", lambda: False)
+    monkeypatch.setattr(torch.ops.l20_stack, "plan_bytes", lambda batch, kv_heads: 64, raising=False)
+    monkeypatch.setattr(l20_paged_split_kv, "allocate_l20_paged_split_kv_workspace", lambda *a, **k: (torch.empty(1),) * 4)
+    monkeypatch.setattr(l20_paged_split_kv, "plan_l20_paged_split_kv",
+                        lambda *a, plan=None, **k: (made.append(plan), plan)[1])
+    q, cache = torch.empty(4, 16, 128), torch.empty(1, 16, 2, 128)
+    call = lambda meta, query: mod.l20_decode_step(meta, query, cache, cache, None, None, 1024).metadata_stable
+    for _step in range(2):
+        meta = SimpleNamespace(l20_step=None)
+        assert [call(meta, q) for _layer in range(3)] == [False, True, True]
+    assert len(made) == 2
+    assert [call(object(), q) for _layer in range(2)] == [False, False]  # metadata that keeps no step: a plan per layer
+    meta = SimpleNamespace(l20_step=None)  # nothing to plan (head_dim 64): no plan kernel in front of any layer
+    assert [call(meta, torch.empty(4, 14, 64)) for _layer in range(2)] == [True, True]
