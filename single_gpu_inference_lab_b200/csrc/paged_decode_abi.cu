@@ -477,8 +477,8 @@ int launch_decode(const pfd_decode_args& a, const pfd::KernelParams& kp, int num
   const dim3 grid(num_splits, a.num_kv_heads, a.batch);
   if (D == 128 && tma_eligible(a)) {
     g_last_path = PFD_PATH_FIXED_TMA;
-    const dim3 grid_with_loners(num_splits, a.num_kv_heads, a.batch + kp.loner_rows);
-    if (int rc = kp.loner_rows > 0 ? launch_partial_tma<QBF16, kWarps, kStages, true>(a, kp, grid_with_loners, stream)
+    const dim3 grid_with_loners(num_splits, a.num_kv_heads, a.batch + kp.loner.rows);
+    if (int rc = kp.loner.rows > 0 ? launch_partial_tma<QBF16, kWarps, kStages, true>(a, kp, grid_with_loners, stream)
                  : suffix_beside_prefix(a, kp.slot_offset, num_splits, kp.row_kv_start != nullptr)
                      ? launch_partial_tma<QBF16, 2, 1>(a, kp, grid, stream)
                      : launch_partial_tma<QBF16>(a, kp, grid, stream))
@@ -530,7 +530,6 @@ int64_t pfd_launch_count(void) { return g_launches.load(std::memory_order_relaxe
 }  // extern "C"
 
 namespace {
-constexpr int kLonerSplit = 256;  // tokens of a request in no group to an item, at least (two page pairs for each of four warps)
 static_assert(pfd::kGroupedMaxBatch == pfd::kGroupsMaxBatch, "batch of a grouped decode");
 // What the grouped shared-prefix entry adds to a split-KV pass: per-request attend starts read on
 // the device, their cap, the split size of requests in no group, and the grid's split count.
@@ -539,7 +538,7 @@ struct GroupedRows {
   int row_kv_cap = 0;
   int split_size_loner = 0;
   int num_splits = 0;
-  int loner_rows = 0, loner_splits = 0, loner_share = 0;  // see pfd::KernelParams
+  pfd::LonerGrid loner{};
   const int32_t* grouped_count = nullptr;
 };
 
@@ -578,10 +577,8 @@ pfd::KernelParams fill_params(const pfd_decode_args& a, int group, bool direct_o
     kp.row_kv_start = grouped->row_kv_start;
     kp.row_kv_cap = grouped->row_kv_cap;
     kp.split_size_loner = grouped->split_size_loner;
-    kp.loner_rows = grouped->loner_rows;
+    kp.loner = grouped->loner;
     kp.loner_grid_row = grouped->num_splits * a.num_kv_heads;
-    kp.loner_splits = grouped->loner_splits;
-    kp.loner_share = grouped->loner_share;
     kp.grouped_count = grouped->grouped_count;
     kp.batch = a.batch;
   }
@@ -1038,13 +1035,8 @@ int pfd_shared_prefix_decode_grouped_fp8_e4m3(const pfd_decode_args* args, const
   rows.split_size_loner = split_loner;
   if (tma_eligible(a) && !(a.flags & PFD_FLAG_ALL_IN_GROUPS)) {
     // Requests in no group get CTAs of their own, one wave of them, and all the slots of their rows
-    // (chunks + ns: the prefix chunks are none of theirs), kLonerSplit tokens or more to a slot.
-    const int slots = chunks + ns;
-    rows.split_size_loner = std::max(((a.max_seq_len + slots - 1) / slots + 15) / 16 * 16, kLonerSplit);
-    rows.loner_splits = std::max((a.max_seq_len + rows.split_size_loner - 1) / rows.split_size_loner, 1);
-    rows.loner_rows = (3 * t_device->sms + ns * a.num_kv_heads - 1) / (ns * a.num_kv_heads);
-    const int64_t ctas = (int64_t)rows.loner_rows * ns * a.num_kv_heads;
-    rows.loner_share = static_cast<int>(std::min<int64_t>(a.max_seq_len * (int64_t)a.num_kv_heads / ctas, 1 << 19));
+    // (chunks + ns: the prefix chunks are none of theirs).
+    rows.loner = pfd::loner_grid(a.max_seq_len, chunks + ns, ns, a.num_kv_heads, t_device->sms);
     rows.grouped_count = g + 4;
   }
   rows.num_splits = ns;

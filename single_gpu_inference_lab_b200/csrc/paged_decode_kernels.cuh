@@ -23,6 +23,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "loner_split.cuh"
+
 namespace pfd {
 
 constexpr int kPage = 16;
@@ -63,12 +65,11 @@ struct KernelParams {
   const int32_t* row_kv_start;
   int32_t row_kv_cap;  // upper bound applied to row_kv_start (a multiple of 16): the slots in front cover no more
   int32_t split_size_loner;  // grouped decode: split size of a request in no group (it attends from 0); 0 = split_size
-  // Grouped decode, requests in no group shared out over CTAs of their own (loner_rows > 0): that many
-  // grid rows in front of the batch's take their (request, kv head, split) items in turns, at most
-  // loner_splits to a request, of split_size_loner tokens or more (split_size_of); their partials fill
-  // the request's slots from 0 on, since it has no prefix chunks.
-  // (loner_grid_row: CTAs of one grid row; loner_share: tokens of one such request, as long as any, for each of those CTAs)
-  int32_t loner_rows, loner_grid_row, loner_splits, loner_share, batch;
+  // Grouped decode, requests in no group shared out over CTAs of their own (loner.rows > 0): that many
+  // grid rows in front of the batch's take their (request, kv head, split) items in turns (split_size_of);
+  // their partials fill the request's slots from 0 on, since it has no prefix chunks.
+  LonerGrid loner;
+  int32_t loner_grid_row, batch;  // CTAs of one grid row; requests of the call
   const int32_t* grouped_count;  // device word: requests of the batch that are in groups
   int32_t early_metadata;  // 1: seq_lens and block_table may be read before the preceding kernel has completed
   int32_t early_kv;        // 1: so may K/V pages, except each sequence's last (balanced kernel with a plan)
@@ -136,9 +137,8 @@ __device__ __forceinline__ int kv_start_of(const KernelParams& p, int b) {
 // items as those CTAs can take at once, of no less than the size that their slots allow.
 __device__ __forceinline__ int split_size_of(const KernelParams& p, int kv0) {
   if (p.row_kv_start == nullptr || kv0 != 0 || p.split_size_loner <= 0) return p.split_size;
-  if (p.loner_rows == 0) return p.split_size_loner;
-  const int loners = p.batch - __ldg(p.grouped_count);
-  return max(p.split_size_loner, (loners * p.loner_share + 63) & ~63);
+  if (p.loner.rows == 0) return p.split_size_loner;
+  return loner_split_size(p.loner, min(max(p.batch - __ldg(p.grouped_count), 0), p.batch));
 }
 
 __device__ __forceinline__ int32_t page_of(const int32_t* __restrict__ block_table,
@@ -782,7 +782,7 @@ __global__ void bounded_wait_selftest_kernel(int32_t* status, unsigned long long
 // softmax bookkeeping (shuffles, rescale).
 //
 // LONERS: a grouped shared-prefix decode whose requests in no group are shared out over CTAs of
-// their own (KernelParams::loner_rows).  A request in no group has some ten times the tokens of
+// their own (KernelParams::loner).  A request in no group has some ten times the tokens of
 // another's suffix; cut into as many splits as those, it is one chain of a dozen page pairs per
 // warp that the whole step waits for: with 64 requests, two groups behind 4096 and 5120 tokens and 8
 // requests of 4.3 K tokens in none, 2 kv heads, this pass took 29 us and a step of eight layers
@@ -813,7 +813,7 @@ paged_decode_fp8_partial_tma_kernel(const KernelParams p, const TmaParams tp,
   // A CTA of the rows in front takes the items of the requests in no group in turns: item
   // (request, kv head, split) number blockIdx, + CTAs of those rows, ...; the others have one item.
   int item = 0, n_items = 0;
-  const bool takes_turns = LONERS && (int)blockIdx.z < p.loner_rows;
+  const bool takes_turns = LONERS && (int)blockIdx.z < p.loner.rows;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t ring = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* ring_ptr = smem_raw + (ring - smem_u32(smem_raw));
@@ -843,10 +843,10 @@ paged_decode_fp8_partial_tma_kernel(const KernelParams p, const TmaParams tp,
         if (mine) sm_loners[before + __popc(votes & ((1u << lane) - 1u))] = (uint16_t)r;
         __syncthreads();
       }
-      n_items = n_loners * p.num_kv_heads * p.loner_splits;
+      n_items = n_loners * p.num_kv_heads * loner_split_count(p.loner, split_size_of(p, 0));
       item = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z);
     } else {
-      b -= p.loner_rows;
+      b -= p.loner.rows;
     }
   }
   // Behind the dense prefix pass (slot_offset > 0) this grid reads nothing of that pass, but it must
@@ -859,13 +859,14 @@ paged_decode_fp8_partial_tma_kernel(const KernelParams p, const TmaParams tp,
   if constexpr (LONERS) {
     if (takes_turns) {
       // splits of a request side by side; those behind its end are passed over
-      for (;; item += p.loner_rows * p.loner_grid_row) {
+      const int loner_size = split_size_of(p, 0), loner_splits = loner_split_count(p.loner, loner_size);
+      for (;; item += p.loner.rows * p.loner_grid_row) {
         if (item >= n_items) break;
-        split = item % p.loner_splits;
-        const int rest = item / p.loner_splits;
+        split = item % loner_splits;
+        const int rest = item / loner_splits;
         kvh = rest % p.num_kv_heads;
         b = sm_loners[rest / p.num_kv_heads];
-        if (split * split_size_of(p, 0) < p.seq_lens[b]) break;
+        if (split * loner_size < p.seq_lens[b]) break;
       }
       if (item >= n_items) {
         if (waits_at_exit) pdl_wait();
@@ -874,6 +875,10 @@ paged_decode_fp8_partial_tma_kernel(const KernelParams p, const TmaParams tp,
     }
   }
   const int kv0 = kv_start_of(p, b);
+  if (LONERS && !takes_turns && kv0 == 0) {  // a request in no group: not this CTA's
+    if (waits_at_exit) pdl_wait();
+    return;
+  }
   const int split_sz = split_size_of(p, kv0);
   const int lo = kv0 + split * split_sz;
 
@@ -891,11 +896,10 @@ paged_decode_fp8_partial_tma_kernel(const KernelParams p, const TmaParams tp,
   const int hi = min(lo + split_sz, seq_len);
   // grouped decode: the grid was sized from the caller's bound on the suffixes; a request that
   // needs more splits than the grid has would lose its tail silently, so it is reported instead
-  const bool not_mine = LONERS && !takes_turns && kv0 == 0;  // a request in no group
-  if (p.row_kv_start != nullptr && !not_mine && split == 0 && kvh == 0 && threadIdx.x == 0 &&
-      seq_len - kv0 > (takes_turns ? p.loner_splits : (int)gridDim.x) * (int64_t)split_sz)
+  if (p.row_kv_start != nullptr && split == 0 && kvh == 0 && threadIdx.x == 0 &&
+      seq_len - kv0 > (takes_turns ? loner_split_count(p.loner, split_sz) : (int)gridDim.x) * (int64_t)split_sz)
     atomicExch(tp.status, kErrSuffixBound);
-  if (lo >= hi || not_mine) {
+  if (lo >= hi) {
     if (waits_at_exit) pdl_wait();
     if (split == 0 && gridDim.x == 1 && p.direct_out) write_empty_rows<D>(p, b, kvh);
     return;
@@ -1048,7 +1052,7 @@ paged_decode_fp8_partial_tma_kernel(const KernelParams p, const TmaParams tp,
   dbg_mark(dbg_slot, 1, threadIdx.x == 0);
   if (!takes_turns) break;
   tbase += n_pairs;
-  item += p.loner_rows * p.loner_grid_row;
+  item += p.loner.rows * p.loner_grid_row;
   // the next item's copies and merge reuse what the merge above reads (no next item after a copy that never landed)
   if (__syncthreads_or(!ok)) break;
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -1090,7 +1094,7 @@ paged_decode_merge_kernel(const KernelParams p, int batch) {
   // slots in front of the splits: all slot_offset of them, or (grouped) those of this row's prefix
   const int pre = GROUPED ? (kv0 + 255) / 256 : p.slot_offset;
   // unused slots between the row's prefix chunks and its splits
-  const int skip = !GROUPED || (p.loner_rows > 0 && kv0 == 0) ? 0 : p.slot_offset - pre;
+  const int skip = !GROUPED || (p.loner.rows > 0 && kv0 == 0) ? 0 : p.slot_offset - pre;
   const int split_sz = GROUPED ? split_size_of(p, kv0) : p.split_size;
   const int ns = (live > 0 ? (live + split_sz - 1) / split_sz : 0) + pre;
   constexpr int E = D / 32;  // elements per lane
