@@ -374,8 +374,9 @@ int pfd_group_shared_prefixes(const int32_t* block_table, int64_t bt_stride_b, i
  * prefix.  max_suffix_len bounds what a request IN a group has behind its prefix (0 = unknown: the
  * whole context); the split-KV grid is sized for it, ceil(max_suffix_len / split_size) splits.  A
  * request in no group covers its whole context with as many splits as all its slots allow, of 256
- * tokens or more, taken by CTAs of their own (under PFD_FLAG_ALL_IN_GROUPS, or with a cache that TMA
- * cannot describe: with as many splits as the others' suffixes, longer ones).  A member whose
+ * tokens or more, taken by CTAs of their own (under PFD_FLAG_ALL_IN_GROUPS, with a cache that TMA
+ * cannot describe, or beside the prefix pass by pfd_set_suffix_form(1): with as many splits as the
+ * others' suffixes, longer ones).  A member whose
  * suffix exceeds the bound would be attended only up to it (device status 5 reports it): give a true bound (max_seq_len minus
  * the smallest prefix a group can have, i.e. the min_prefix_len of the grouping call).  The
  * workspace needs ceil(min(max_prefix_len, max_seq_len) / 256) +

@@ -477,7 +477,7 @@ int launch_decode(const pfd_decode_args& a, const pfd::KernelParams& kp, int num
   const dim3 grid(num_splits, a.num_kv_heads, a.batch);
   if (D == 128 && tma_eligible(a)) {
     g_last_path = PFD_PATH_FIXED_TMA;
-    const dim3 grid_with_loners(num_splits, a.num_kv_heads, a.batch + kp.loner.rows);
+    const dim3 grid_with_loners(num_splits, a.num_kv_heads, a.batch + kp.loner.rows);  // (rows > 0: not beside the prefix)
     if (int rc = kp.loner.rows > 0 ? launch_partial_tma<QBF16, kWarps, kStages, true>(a, kp, grid_with_loners, stream)
                  : suffix_beside_prefix(a, kp.slot_offset, num_splits, kp.row_kv_start != nullptr)
                      ? launch_partial_tma<QBF16, 2, 1>(a, kp, grid, stream)
@@ -1033,7 +1033,7 @@ int pfd_shared_prefix_decode_grouped_fp8_e4m3(const pfd_decode_args* args, const
   rows.row_kv_start = g + pfd::groups_row_prefix_off();
   rows.row_kv_cap = cap;
   rows.split_size_loner = split_loner;
-  if (tma_eligible(a) && !(a.flags & PFD_FLAG_ALL_IN_GROUPS)) {
+  if (tma_eligible(a) && !beside && !(a.flags & PFD_FLAG_ALL_IN_GROUPS)) {
     // Requests in no group get CTAs of their own, one wave of them, and all the slots of their rows
     // (chunks + ns: the prefix chunks are none of theirs).
     rows.loner = pfd::loner_grid(a.max_seq_len, chunks + ns, ns, a.num_kv_heads, t_device->sms);

@@ -492,3 +492,34 @@ def test_requests_in_no_group_have_ctas_of_their_own(cabi, batch, hq, hkv, group
         torch.cuda.synchronize()
         assert cabi.device_status() == 0
         assert_within_gate(out, exp, f"step {step}")
+
+
+@pytest.mark.parametrize("form", [0, 1, -1])
+def test_the_forced_suffix_form_is_the_one_that_runs(cabi, suffix_form, form):
+    """A grouped call without the all-in-groups word: beside the prefix pass (1) every request's partials lie behind the
+    prefix slots; requests in no group have CTAs of their own, whose partials begin in slot 0, in the other form only."""
+    suffix_form(form)
+    w = make_inputs("shared-prefix-b64", seed=23, batch=20, shrink=0.25)
+    gen = torch.Generator().manual_seed(23)
+    pages, prefix_pages, alone = w.key_cache.shape[0], w.prefix_len // 16, 4
+    w.block_table = w.block_table.clone()
+    w.block_table[-alone:, :prefix_pages] = torch.randint(0, pages, (alone, prefix_pages), generator=gen, dtype=torch.int32)
+    exp = oracle.reference(w.query, w.key_cache, w.value_cache, w.block_table.long(), w.seq_lens, w.k_scale, w.v_scale)
+    g = w.to(DEV)
+    groups, max_groups = cabi.group_shared_prefixes(g.block_table, seq_lens=g.seq_lens, min_batch=8, min_prefix_len=w.prefix_len,
+                                                    max_groups=2)
+    bound = w.max_seq_len - w.prefix_len
+    chunks = -(-w.prefix_len // 256)
+    b, hq, d = g.query.shape
+    shape = (b, hq, chunks + -(-bound // 128))
+    ws = tuple(torch.full(s, float("nan"), device=DEV) for s in ((*shape, d), shape, shape))
+    out = torch.full_like(g.query, float("nan"))
+    cabi.shared_prefix_decode_grouped_fp8_e4m3(
+        g.query, g.key_cache, g.value_cache, g.block_table, g.seq_lens, groups=groups, max_groups=max_groups,
+        max_prefix_len=w.prefix_len, max_suffix_len=bound, k_scale=g.k_scale, v_scale=g.v_scale, max_seq_len=w.max_seq_len,
+        split_size=128, output=out, workspace=ws)
+    torch.cuda.synchronize()
+    assert cabi.device_status() == 0 and groups[3:5].tolist() == [1, b - alone]
+    assert_within_gate(out, exp, f"form={form}")
+    in_front = ws[1][-alone:, :, :chunks].isnan()
+    assert in_front.all() if form == 1 else not in_front[:, :, 0].any()
