@@ -61,8 +61,8 @@ extern "C" {
                                 that end a sequence, and the queries, after it has completed                   */
 /*
  * Kernel selection.  For head_dim 128, at most 8 query heads per kv head, a TMA-describable
- * cache and a dense f32 workspace of at least pfd_balanced_workspace_rows() rows the balanced
- * persistent kernel + its merge kernel run (split_size then only sizes the workspace); with `plan`
+ * cache and a dense f32 workspace of at least pfd_balanced_workspace_rows() rows (its base 16-byte,
+ * packed_output 8-byte aligned) the balanced persistent kernel + its merge kernel run (split_size then only sizes the workspace); with `plan`
  * set both read their work split instead of deriving it.  So do (without a plan, which is ignored)
  * calls of head_dim 64 with at most 8 query heads per kv head, batch * (max_seq_len - kv_start) of
  * 2^17 tokens or more and slots for three quarters of the kernel's warp groups.  Anything else, or

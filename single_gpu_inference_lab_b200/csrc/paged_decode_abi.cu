@@ -327,12 +327,20 @@ constexpr int kChunkWarps16 = 6;
 // (us per step): 0 -> 53.9, 1 -> 44.2, 2 -> 43.0, 3 -> 43.3, 4 -> 44.0; the batch-64 one does not care.
 constexpr int kChunkPieceCost = 2;
 
+// Pieces are stored 16 bytes at a time and packed rows 8: the fixed-split grid, which may not need the workspace and
+// stores packed rows by element, takes calls whose buffers are aligned less.
+bool packed_aligned(const pfd_decode_args& a) {
+  return a.exchange != nullptr || (reinterpret_cast<uintptr_t>(a.packed_output) & 7u) == 0;
+}
+bool balanced_aligned(const pfd_decode_args& a) { return aligned16(a.partial_output) && packed_aligned(a); }
+
 bool balanced_eligible(const pfd_decode_args& a, int group, int slot_offset, int sms) {
   if (a.flags & (PFD_FLAG_FIXED_SPLITS | PFD_FLAG_NO_TMA | PFD_FLAG_NO_DIRECT_OUT)) return false;
   if (slot_offset != 0) return false;  // slots in front belong to the dense prefix pass
   if (a.head_dim != 128 || !tma_eligible(a) || group > 8 || a.batch > kChunkMaxBatch) return false;
   if (a.num_kv_heads > kChunkWarps * sms / 2) return false;  // one warp per kv head and group
   if (!a.partial_output || !a.partial_max || !a.partial_sum || a.partial_dtype != PFD_DTYPE_F32) return false;
+  if (!balanced_aligned(a)) return false;
   if (a.partial_stride_s != 1 || a.partial_stride_h != a.workspace_splits ||
       a.partial_stride_b != (int64_t)a.num_q_heads * a.workspace_splits)
     return false;
@@ -357,7 +365,7 @@ int balanced64_groups(const pfd_decode_args& a, int group, int slot_offset, int 
   if (a.flags & (PFD_FLAG_FIXED_SPLITS | PFD_FLAG_NO_TMA | PFD_FLAG_NO_DIRECT_OUT | PFD_FLAG_PARTIAL_ONLY)) return 0;
   if (slot_offset != 0 || a.page_indptr != nullptr || a.exchange != nullptr || !tma_describable(a)) return 0;
   if (group > 8 || a.batch > kChunkMaxBatch || a.num_kv_heads > kChunkWarps64 * sms / 2) return 0;
-  if (!a.partial_output || !a.partial_max || !a.partial_sum || a.partial_dtype != PFD_DTYPE_F32) return 0;
+  if (!a.partial_output || !a.partial_max || !a.partial_sum || a.partial_dtype != PFD_DTYPE_F32 || !balanced_aligned(a)) return 0;
   if (a.partial_stride_s != 1 || a.partial_stride_h != a.workspace_splits ||
       a.partial_stride_b != (int64_t)a.num_q_heads * a.workspace_splits)
     return 0;
@@ -395,7 +403,8 @@ int launch_balanced(const pfd_decode_args& a, const pfd::KernelParams& kp, int s
   tp.phase_times = g_phase_times;
   // A plan needs f32 pieces (its in-kernel merge reads them as such; the merge kernel takes either).
   const bool planned = D == 128 && a.plan != nullptr && a.partial_dtype == PFD_DTYPE_F32;
-  const bool fused = planned && (a.flags & PFD_FLAG_SINGLE_LAUNCH) && !(a.flags & PFD_FLAG_PARTIAL_ONLY);
+  // (16-bit caches, whose kernels have no other form, store packed rows by element but for the in-kernel merge)
+  const bool fused = planned && (a.flags & PFD_FLAG_SINGLE_LAUNCH) && !(a.flags & PFD_FLAG_PARTIAL_ONLY) && packed_aligned(a);
   auto kernel = pfd::paged_decode_fp8_chunk_kernel<QBF16, kStagesT, kWarpsT, KV16, false, D>;
   if constexpr (D == 128) {
     if (fused) kernel = pfd::paged_decode_fp8_chunk_kernel<QBF16, kStagesT, kWarpsT, KV16, true>;

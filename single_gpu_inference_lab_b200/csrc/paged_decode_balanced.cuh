@@ -1371,9 +1371,9 @@ paged_decode_chunk_merge_kernel(const KernelParams p, const TmaParams tp, const 
     return;
   }
   if (p.packed_output != nullptr) {
-    float* dst = p.packed_output + (int64_t)row * (D + 2);
+    float* dst = p.packed_output + (int64_t)row * (D + 2);  // (4-byte aligned, where the cache is a 16-bit one)
 #pragma unroll
-    for (int e = 0; e < E; e += 2) *reinterpret_cast<float2*>(dst + lane * E + e) = make_float2(acc[e], acc[e + 1]);
+    for (int e = 0; e < E; ++e) dst[lane * E + e] = acc[e];
     if (lane == 0) { dst[D] = big; dst[D + 1] = den; }
     return;
   }

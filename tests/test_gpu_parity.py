@@ -582,3 +582,45 @@ def test_balanced_kernel_with_head_dim_64(cabi, d, hq, hkv, layout):
                 assert torch.equal(l.cpu() > 0, live[:, None].expand(batch, hq)), what
                 out = torch.where(l[..., None] > 0, o / l[..., None], 0.0).to(q.dtype)
             assert_within_gate(out, exp.to(q.dtype), what)
+
+
+@pytest.mark.parametrize("what", ["d64 partials", "d128 partials", "d64 packed", "d128 packed", "kv16 packed", "kv16 packed fused"])
+def test_buffers_aligned_to_four_bytes_only(cabi, what):
+    """A workspace that a one-split call does not need, and packed rows, may lie at any float: the balanced kernel, which
+    stores 16 and 8 bytes at a time, leaves such calls to the grid (16-bit caches: stored by element)."""
+    gen = torch.Generator().manual_seed(3)
+    d, kv16, packed = 64 if "d64" in what else 128, "kv16" in what, "packed" in what
+    batch, longest, hq, hkv = 260, 512, 8, 8
+    lens = torch.randint(1, longest + 1, (batch,), generator=gen).to(torch.int32)
+    lens[:2] = torch.tensor([longest, longest - 1])
+    pages = 900
+    table = torch.randint(0, pages, (batch, longest // 16), generator=gen).to(torch.int32)
+    k, v = torch.randn(pages, 16, hkv, d, generator=gen), torch.randn(pages, 16, hkv, d, generator=gen)
+    q = torch.randn(batch, hq, d, generator=gen).to(torch.bfloat16)
+    if kv16:
+        kc, vc, scales = k.to(q.dtype), v.to(q.dtype), {}
+        exp = oracle.reference_kv16(q, kc, vc, table.long(), lens)
+    else:
+        (kc, ks), (vc, vs) = oracle.quantize_fp8_e4m3_per_head(k), oracle.quantize_fp8_e4m3_per_head(v)
+        scales = dict(k_scale=ks.to(DEV), v_scale=vs.to(DEV))
+        exp = oracle.reference(q, kc, vc, table.long(), lens, ks, vs)
+    g = [t.to(DEV) for t in (q, kc, vc, table, lens)]
+    split = 256 if packed else 512
+    at_float = lambda *shape: torch.full((math.prod(shape) + 1,), float("nan"), device=DEV)[1:].view(shape)
+    ws = list(workspace(g[0], longest, split, min_rows=cabi.balanced_workspace_rows(hq, hkv) * (2 if d == 64 else 1)))
+    if not packed:
+        ws[0] = at_float(*ws[0].shape)
+    out = torch.full_like(g[0], float("nan"))
+    pk = at_float(batch, hq, d + 2) if packed else None
+    assert (pk if packed else ws[0]).data_ptr() % 8 == 4
+    plan = cabi.plan_decode(*g, max_seq_len=longest, split_size=split, workspace=ws) if "fused" in what else None
+    call = cabi.paged_decode_kv16_split_out if kv16 else cabi.paged_decode_fp8_e4m3_split_out
+    call(*g, max_seq_len=longest, split_size=split, output=None if packed else out, packed_output=pk, workspace=ws, plan=plan,
+         flags=64 if plan is not None else 0, **scales)
+    torch.cuda.synchronize()
+    assert cabi.device_status() == 0
+    assert cabi.last_path() == (4 if kv16 else PATH_LDG if d == 64 else PATH_TMA)
+    if packed:
+        o, l = pk[..., :d], pk[..., d + 1:]
+        out = (o / l).to(q.dtype)
+    assert_within_gate(out, exp, what)
