@@ -604,13 +604,6 @@ pfd::KernelParams fill_params(const pfd_decode_args& a, int group, bool direct_o
     kp.packed_output = static_cast<float*>(x.recv[x.rank]);  // non-NULL selects the packed form; the kernels address through xch_recv
     kp.output = nullptr;
   }
-  // (o, m, l) rows that the caller gets to see, or that are stored in 16 bits, are relative to the true
-  // maximum.  So are fp16 calls': with the largest probabilities at and just below 1 their rounding to
-  // f16 is at its best, and unlike a bf16 output an fp16 one shows it (relative error against 64 bits, 32
-  // + 2 heads, 512 .. 4096 tokens: 2.6e-4 so, 2.8e-4 with a slack of 8; bf16 1.7e-3 either way).
-  kp.max_slack = kp.packed_output != nullptr || a.partial_dtype != PFD_DTYPE_F32 || a.query_dtype == PFD_DTYPE_F16 ||
-                         (a.flags & PFD_FLAG_PARTIAL_ONLY)
-                     ? 0.f : 8.f;
 #ifdef PFD_BOUNDS_CHECK
   kp.dbg_ws_rows = (int64_t)a.batch * a.num_q_heads * a.workspace_splits;
   kp.dbg_batch = a.batch;

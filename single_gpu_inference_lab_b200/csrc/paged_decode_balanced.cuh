@@ -156,15 +156,17 @@ __device__ __forceinline__ uint2 lds_8(uint32_t addr) {
 }
 
 // The running maximum of a step's raw scores s[head tile][page][c] (heads 2j + (c & 1)), scaled, brought
-// up to date -- only when some score lies more than `slack` (log2 units) above it: the maximum only has
-// to keep the exponentials in range, and a probability of up to 2^slack against a stale one is as
-// exact, in f16 or two bf16 terms, as one of up to 1.  So after a piece's first step the three
-// shuffles per head, the rescaling factors and the rescaling itself hardly ever run: they were the longest
-// part of a step's chain (a recorded step of eight layers, 16 + 2 heads, batch 64: 160.9 -> 150.7 us;
-// 4 x 131072 tokens: 173.4 -> 162.7).  scale_log2 >= 0 (see the kernel).
+// up to date.  The three shuffles per head, the rescaling factors and the rescaling are long links of a
+// step's chain and run only in steps in which some head's maximum rises, fewer the longer the piece (us so
+// / in every step: 4 x 131072 tokens 175.8 / 178.7, head_dim 64, 256 of 512 .. 4096 37.6 / 38.6, a recorded
+// step of eight layers, batch 64, a dozen page pairs to a piece 154.6 / 152.6).  The maximum is the true
+// one: left up to 8 (log2) behind, which keeps the exponentials in range and skips nearly all of it (151.2 us
+// for that step), it makes the largest probability another number than 1, which f16 holds exactly, and with
+// scores of a standard deviation of 1 (3) the rounded products' sum is, simulated, 1.1 .. 1.2 (2 .. 4) times as far off.
+// scale_log2 >= 0 (see the kernel).
 template <int NH, int MT>
 __device__ __forceinline__ void bal_raise_max(float (&m)[NH][2], float (&l)[NH][2], float (&o)[NH][MT][4],
-                                              const float (&s)[NH][2][4], float scale_log2, float slack) {
+                                              const float (&s)[NH][2][4], float scale_log2) {
   float x[NH][2];
   bool higher = false;
 #pragma unroll
@@ -172,7 +174,7 @@ __device__ __forceinline__ void bal_raise_max(float (&m)[NH][2], float (&l)[NH][
 #pragma unroll
     for (int e = 0; e < 2; ++e) {
       x[h][e] = fmaxf(fmaxf(s[h][0][e], s[h][0][2 + e]), fmaxf(s[h][1][e], s[h][1][2 + e])) * scale_log2;
-      higher |= x[h][e] > m[h][e] + slack;
+      higher |= x[h][e] > m[h][e];
     }
   if (!__any_sync(0xffffffffu, higher)) return;
 #pragma unroll
@@ -202,7 +204,7 @@ __device__ __forceinline__ void bal_raise_max(float (&m)[NH][2], float (&l)[NH][
 template <int NH, int D>
 __device__ __forceinline__ void bal_step(BalState<NH, D>& st, uint32_t stage, const uint32_t (&k_off)[2][D / 64],
                                          const uint32_t (&v_off)[4], const uint32_t (&qb)[NH][D / 16][2],
-                                         float scale_log2, float slack, int tok0, int lo, int hi, int i, int j) {
+                                         float scale_log2, int tok0, int lo, int hi, int i, int j) {
   constexpr uint32_t kTile = kPage * D;
   constexpr int KL = D / 64, VW = D / 32;
   const bool edge = (tok0 < lo) | (tok0 + 2 * kPage > hi);
@@ -250,7 +252,7 @@ __device__ __forceinline__ void bal_step(BalState<NH, D>& st, uint32_t stage, co
         }
       }
   }
-  bal_raise_max<NH, D / 16>(st.m, st.l, st.o, s, scale_log2, slack);
+  bal_raise_max<NH, D / 16>(st.m, st.l, st.o, s, scale_log2);
   uint32_t pb[NH][2][2];  // P^T B-fragments [head tile][page][b0|b1]
 #pragma unroll
   for (int h = 0; h < NH; ++h) {
@@ -405,7 +407,7 @@ __device__ __forceinline__ void kv16_load_q(uint32_t (&qb)[1][8][2], const Kerne
 // 4 KiB tiles (two swizzled halves each).  tok0 = token index of page 0's row 0.
 template <bool BF16>
 __device__ __forceinline__ void kv16_step(BalState<1, 128>& st, uint32_t stage, const uint32_t (&qb)[1][8][2],
-                                          float scale_log2, float slack, int tok0, int lo, int hi, int lane) {
+                                          float scale_log2, int tok0, int lo, int hi, int lane) {
   constexpr uint32_t kTile = 2 * kPage * 128;
   const int i = lane >> 2, j = lane & 3;
   const int mid = lane >> 3, r8 = lane & 7;
@@ -442,7 +444,7 @@ __device__ __forceinline__ void kv16_step(BalState<1, 128>& st, uint32_t stage, 
         }
       }
   }
-  bal_raise_max<1, 8>(st.m, st.l, st.o, s, scale_log2, slack);
+  bal_raise_max<1, 8>(st.m, st.l, st.o, s, scale_log2);
   // P^T B-fragments.  bf16 keeps 8 bits of a probability: there P goes in as two bf16 terms
   // (p = hi + lo, 16 bits together) and the PV product takes two MMAs; f16 keeps 11 bits.
   uint32_t pb[2][2], pl[2][2];
@@ -1029,7 +1031,6 @@ paged_decode_fp8_chunk_kernel(const KernelParams p, const TmaParams tp, const Ch
   const float scale_signed = ks * p.sm_scale * kLog2e;
   const float scale_log2 = fabsf(scale_signed);
   const uint32_t q_flip = scale_signed < 0.f ? 0x80008000u : 0u;
-  const float slack = p.max_slack;
   const auto load_q = [&](uint32_t (&dst)[1][D / 16][2], int b) {
     if constexpr (KV16) kv16_load_q(dst, p, b, kvh, i, j);
     else bal_load_q<QBF16, 1, D>(dst, p, b, kvh, i, j);
@@ -1067,8 +1068,8 @@ paged_decode_fp8_chunk_kernel(const KernelParams p, const TmaParams tp, const Ch
       if (t == 0) mark_phase_at(tp, W, 3, lane == 0);  // first data landed
       if (t == n / 2) mark_phase_at(tp, W, 6, lane == 0);  // half of the chunk consumed
       const int tok0 = (page_first + 2 * (g - cur.start)) * kPage;
-      if constexpr (KV16) kv16_step<QBF16>(st, my_ring + s * kStage, qb, scale_log2, slack, tok0, p.kv_start, seq_len, lane);
-      else bal_step<1, D>(st, my_ring + s * kStage, k_off, v_off, qb, scale_log2, slack, tok0, p.kv_start, seq_len, i, j);
+      if constexpr (KV16) kv16_step<QBF16>(st, my_ring + s * kStage, qb, scale_log2, tok0, p.kv_start, seq_len, lane);
+      else bal_step<1, D>(st, my_ring + s * kStage, k_off, v_off, qb, scale_log2, tok0, p.kv_start, seq_len, i, j);
       // all reads of the stage fed MMAs above: hand it back to TMA for the chunk's pair t + NSTAGE
       __syncwarp();
       const int tn = t + NSTAGE;

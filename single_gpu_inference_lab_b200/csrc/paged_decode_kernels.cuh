@@ -56,7 +56,6 @@ struct KernelParams {
   int32_t num_q_heads, num_kv_heads, group;
   int32_t split_size, kv_start;
   int32_t partial_dtype;
-  float max_slack;     // how far (log2 units) a score may lie above the running maximum before that is raised
   int32_t direct_out;  // 1: a sequence with a single split writes its final result itself
   int32_t bt_cols;     // width of a block-table row
   int32_t slot_offset; // workspace slots [0, slot_offset) are filled by another kernel (dense prefix pass)
@@ -265,14 +264,12 @@ __device__ __forceinline__ void qk_scores(float (&s)[NT][4], const uint32_t (&k)
 
 // Mask, scale, online softmax over NT/2 pages of raw scores; rescales O when it has to and returns P as
 // the f16 A-fragments of the PV MMAs (pa[t] for page t).  Column tile nt covers tokens
-// tok0 + 8*nt + rho(.).  The running maximum only has to keep the exponentials in range: it is raised
-// when a score lies more than `slack` (log2 units) above it, and a probability of up to 2^slack
-// against a stale one is as exact in f16 as one of up to 1.  So after a warp's first step the
-// shuffles, the rescaling factors and the rescaling hardly ever run, and with no slack in a few steps only.  scale_log2 >= 0
-// (a negative scale's sign is in the query, see load_q_frags).
+// tok0 + 8*nt + rho(.).  The shuffles, the rescaling factors and the rescaling run only in steps in which
+// some row's maximum rises (see bal_raise_max).  scale_log2 >= 0 (a negative scale's sign is in the
+// query, see load_q_frags).
 template <int D, int NT>
 __device__ __forceinline__ void softmax_step(WarpState<D>& st, float (&s)[NT][4],
-                                             uint32_t (&pa)[NT / 2][4], float scale_log2, float slack, bool edge,
+                                             uint32_t (&pa)[NT / 2][4], float scale_log2, bool edge,
                                              int tok0, int lo, int hi, int j) {
   uint32_t dead = 0u;  // bit 2 nt + (c & 1)
   if (edge) {
@@ -295,7 +292,7 @@ __device__ __forceinline__ void softmax_step(WarpState<D>& st, float (&s)[NT][4]
   }
   mx0 *= scale_log2;
   mx1 *= scale_log2;
-  if (__any_sync(0xffffffffu, (mx0 > st.m[0] + slack) | (mx1 > st.m[1] + slack))) {
+  if (__any_sync(0xffffffffu, (mx0 > st.m[0]) | (mx1 > st.m[1]))) {
     mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, 1));
     mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 1));
     mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, 2));
@@ -364,13 +361,13 @@ __device__ __forceinline__ void pv_accumulate(WarpState<D>& st, uint32_t (&v)[4]
 
 template <int D>
 __device__ __forceinline__ void consume_tile(WarpState<D>& st, TileRegs<D>& t,
-                                             const uint32_t (&qa)[D / 16][4], float scale_log2, float slack,
+                                             const uint32_t (&qa)[D / 16][4], float scale_log2,
                                              int tok0, int lo, int hi, int j) {
   float s[2][4];
   uint32_t pa[1][4];
   const bool edge = (tok0 < lo) | (tok0 + kPage > hi);
   qk_scores<D, 2>(s, t.k, qa);
-  softmax_step<D, 2>(st, s, pa, scale_log2, slack, edge, tok0, lo, hi, j);
+  softmax_step<D, 2>(st, s, pa, scale_log2, edge, tok0, lo, hi, j);
   pv_accumulate<D>(st, t.v, pa[0], edge, tok0, lo, hi, j);
 }
 
@@ -594,7 +591,7 @@ paged_decode_fp8_partial_ldg_kernel(const KernelParams p) {
       load_tile_global<D>(nxt, kbase + phys * p.k_stride_page, vbase + phys * p.v_stride_page,
                           p.k_stride_token, p.v_stride_token, i, j);
     }
-    consume_tile<D>(st, cur, qa, scale_log2, p.max_slack, pg * kPage, lo, hi, j);
+    consume_tile<D>(st, cur, qa, scale_log2, pg * kPage, lo, hi, j);
     cur = nxt;
   }
   cta_merge_and_store<D, QBF16, NWARPS>(st, p, b, kvh, split + p.slot_offset, nsplits_seq, vs, sm_m, sm_l, sm_o);
@@ -1005,7 +1002,7 @@ paged_decode_fp8_partial_tma_kernel(const KernelParams p, const TmaParams tp,
         }
       qk_scores<D, 4>(sc, k, qa);
     }
-    softmax_step<D, 4>(st, sc, pa, scale_log2, p.max_slack, edge, tok0, lo, hi, j);
+    softmax_step<D, 4>(st, sc, pa, scale_log2, edge, tok0, lo, hi, j);
 #pragma unroll
     for (int u = 0; u < 2; ++u) {
       uint32_t v[4][4];

@@ -624,3 +624,135 @@ def test_buffers_aligned_to_four_bytes_only(cabi, what):
         o, l = pk[..., :d], pk[..., d + 1:]
         out = (o / l).to(q.dtype)
     assert_within_gate(out, exp, what)
+
+
+# ---------------------------------------------------------------- the running maximum and the sign of the scale
+KERNELS = {  # head_dim, 16-bit cache, flags, path
+    "balanced": (128, False, 0, PATH_BALANCED), "balanced d64": (64, False, 0, PATH_BALANCED), "kv16": (128, True, 0, 4),
+    "grid tma": (128, False, 8, PATH_TMA), "grid loads": (128, False, 1, PATH_LDG), "grid d64": (64, False, 8, PATH_LDG),
+}
+
+
+def _exact(q, kc, vc, table, lens, ks=1.0, vs=1.0, sm_scale=None):
+    """Attention in 64 bits.  (The oracle rounds the dequantised cache to fp16, by up to 2^-11 of a value: of no account at
+    ordinary scores, but 0.13 of a score of 260 (log2), 9 % of a weight where the gate allows 1 %.)"""
+    batch, hq, d = q.shape
+    hkv = kc.shape[2]
+    scale = d ** -0.5 if sm_scale is None else sm_scale
+    per_head = lambda s: (s.double() if isinstance(s, torch.Tensor) else torch.full((hkv,), s, dtype=torch.float64))[:, None, None]
+    out = torch.empty(batch, hq, d, dtype=torch.float64)
+    for b, n in enumerate(lens.tolist()):
+        rows = lambda c, s: c[table[b].long()].double().reshape(-1, hkv, d)[:n].transpose(0, 1) * per_head(s)
+        w = torch.softmax(q[b].double().view(hkv, hq // hkv, d) @ rows(kc, ks).transpose(1, 2) * scale, -1)
+        out[b] = (w @ rows(vc, vs)).reshape(hq, d)
+    return out.to(q.dtype)
+
+
+def _one_direction(kernel, dtype, log2_scores, sm_scale=None, k_sign=1.0, seed=0):
+    """A batch in which every key is a multiple of one vector: score (log2) of token t for query head h of sequence b is
+    ``log2_scores(t) * (1, -1, 0.5, 0)[h % 4]`` or, the keys being quantised, nearly that.  (operands, expected)"""
+    d, kv16, _, _ = KERNELS[kernel]
+    gen = torch.Generator().manual_seed(seed)
+    batch, longest, hq, hkv = 256 if d == 64 else 12, 520, 8, 2  # (head_dim 64: enough work for the balanced kernel)
+    lens = torch.randint(1, longest + 1, (batch,), generator=gen).to(torch.int32)
+    lens[:5] = torch.tensor([longest, longest - 1, 33, 17, 1])
+    width, pages = -(-longest // 16), 200
+    u = torch.nn.functional.normalize(torch.randn(d, generator=gen), dim=0) * d ** 0.5
+    t = torch.arange(width * 16, dtype=torch.float64)
+    scale = d ** -0.5 if sm_scale is None else sm_scale
+    # pages of the table in token order, so that page p holds tokens 16 p .. 16 p + 15 of every sequence
+    rows = log2_scores(t) / (1.4426950408889634 * scale * k_sign * float(u.double() @ u.double()))
+    k = (rows[:, None].float() * u).view(width, 16, 1, d).expand(width, 16, hkv, d).contiguous()
+    v = torch.randn(width, 16, hkv, d, generator=gen)
+    table = torch.arange(width).expand(batch, width).contiguous().to(torch.int32)
+    q = (u * torch.tensor([1.0, -1.0, 0.5, 0.0]).repeat(hq // 4)[:, None]).expand(batch, hq, d).to(dtype).contiguous()
+    if kv16:
+        kc, vc, scales = k.to(dtype), v.to(dtype), {}
+        assert sm_scale is None and k_sign == 1.0
+    else:
+        (kc, ks), (vc, vs) = oracle.quantize_fp8_e4m3_per_head(k), oracle.quantize_fp8_e4m3_per_head(v)
+        ks = ks * k_sign
+        scales = dict(k_scale=ks, v_scale=vs)
+    return (q, kc, vc, table, lens), scales, longest, _exact(q, kc, vc, table, lens, *scales.values(), sm_scale=sm_scale)
+
+
+def _attend(cabi, kernel, operands, scales, longest, **kw):
+    d, kv16, flags, path = KERNELS[kernel]
+    g = [t.to(DEV) for t in operands]
+    ws = workspace(g[0], longest, 512, min_rows=2 * cabi.balanced_workspace_rows(g[0].shape[1], g[1].shape[2]))
+    out = torch.full_like(g[0], float("nan"))
+    call = cabi.paged_decode_kv16_split_out if kv16 else cabi.paged_decode_fp8_e4m3_split_out
+    call(*g, max_seq_len=longest, split_size=512, output=out, workspace=ws, flags=flags,
+         **{n: s.to(DEV) for n, s in scales.items()}, **kw)
+    torch.cuda.synchronize()
+    assert cabi.device_status() == 0 and cabi.last_path() == path
+    return out
+
+
+def _normal_scores(kernel, dtype, sharp, seed):
+    """Normal queries and keys, scores of a standard deviation of ``sharp`` (natural units)."""
+    d, kv16, _, _ = KERNELS[kernel]
+    gen = torch.Generator().manual_seed(seed)
+    batch, longest, hq, hkv = 256 if d == 64 else 48, 1024 if d == 128 else 520, 8, 2
+    lens = torch.randint(longest // 2, longest + 1, (batch,), generator=gen).to(torch.int32)
+    pages = 400
+    table = torch.randint(0, pages, (batch, -(-longest // 16)), generator=gen).to(torch.int32)
+    q = (sharp * torch.randn(batch, hq, d, generator=gen)).to(dtype)
+    k, v = torch.randn(pages, 16, hkv, d, generator=gen), torch.randn(pages, 16, hkv, d, generator=gen)
+    if kv16:
+        kc, vc, scales = k.to(dtype), v.to(dtype), {}
+    else:
+        (kc, ks), (vc, vs) = oracle.quantize_fp8_e4m3_per_head(k), oracle.quantize_fp8_e4m3_per_head(v)
+        scales = dict(k_scale=ks, v_scale=vs)
+    return (q, kc, vc, table, lens), scales, longest, _exact(q, kc, vc, table, lens, *scales.values())
+
+
+@pytest.mark.parametrize("kernel", [k for k in KERNELS if k != "kv16"])  # (whose bf16 probabilities have 16 bits)
+def test_probabilities_are_relative_to_the_true_maximum(cabi, kernel):
+    """The largest probability is then 1, exact in f16, and a bf16 output shows it: of outputs whose error before the last
+    rounding is r (relative, rms), about 0.8 r / (2^-8 / 1.44) are not the rounded 64-bit result.  At scores of a standard
+    deviation of 3, r is 0.6e-4 .. 0.9e-4 with the true maximum (measured here: 2.7 % .. 3.5 % of the outputs) and 1.5e-4 ..
+    2e-4 with one up to 8 (log2) behind (5.2 % .. 6.7 %)."""
+    operands, scales, longest, exp = _normal_scores(kernel, torch.bfloat16, 3.0, seed=0)
+    out = _attend(cabi, kernel, operands, scales, longest).cpu()
+    assert float((out != exp).float().mean()) < 0.043
+    assert_within_gate(out, exp, kernel)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("kernel", list(KERNELS))
+def test_scores_that_rise_along_the_sequence(cabi, kernel, dtype):
+    """The maximum moves in every step, by a little or by a lot, late, or never: falling and constant scores, a step of a
+    page, a jump far above everything before it.  (Half the heads see the scores with the other sign.)"""
+    rises = {
+        "slowly": lambda t: 0.0625 * t, "by 7.9 a page pair": lambda t: 7.9 * (t // 32), "by 8.1 a page": lambda t: 8.1 * (t // 16),
+        "falling": lambda t: -0.5 * t, "constant": lambda t: torch.zeros_like(t), "a late jump": lambda t: 40.0 * (t >= 500),
+    }
+    for what, scores in rises.items():
+        operands, scales, longest, exp = _one_direction(kernel, dtype, scores, seed=len(what))
+        assert_within_gate(_attend(cabi, kernel, operands, scales, longest), exp, f"{kernel} {dtype} {what}")
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("kernel", [k for k in KERNELS if k != "kv16"])
+def test_scales_below_and_at_zero(cabi, kernel, dtype):
+    """A negative softmax scale or K scale (its sign goes into the query), both, and a K scale of zero (all tokens alike)."""
+    rising = lambda t: 0.05 * t
+    for sm_scale, k_sign in ((-0.07, 1.0), (None, -1.0), (-0.07, -1.0), (0.11, 1.0)):
+        operands, scales, longest, exp = _one_direction(kernel, dtype, rising, sm_scale, k_sign)
+        out = _attend(cabi, kernel, operands, scales, longest, **({} if sm_scale is None else {"sm_scale": sm_scale}))
+        assert_within_gate(out, exp, f"{kernel} {dtype} sm_scale={sm_scale} k_sign={k_sign}")
+    operands, scales, longest, _ = _one_direction(kernel, dtype, rising)
+    scales["k_scale"] = torch.zeros_like(scales["k_scale"])
+    exp = _exact(*operands, *scales.values())
+    assert_within_gate(_attend(cabi, kernel, operands, scales, longest), exp, f"{kernel} {dtype} k_scale=0")
+
+
+@pytest.mark.parametrize("kernel", list(KERNELS))
+def test_an_infinite_query_value_spoils_its_own_head_only(cabi, kernel):
+    operands, scales, longest, exp = _one_direction(kernel, torch.bfloat16, lambda t: 0.05 * t)
+    operands[0][1, 3, 7] = float("inf")
+    out = _attend(cabi, kernel, operands, scales, longest)
+    assert out[1, 3].isnan().all()
+    out[1, 3] = exp[1, 3].to(DEV)
+    assert_within_gate(out, exp, kernel)
