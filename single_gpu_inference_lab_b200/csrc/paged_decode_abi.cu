@@ -250,7 +250,7 @@ int launch_partial_tma(const pfd_decode_args& a, const pfd::KernelParams& kp, di
   tp.wait_limit_ns = g_wait_limit_ns.load(std::memory_order_relaxed);
   auto kernel = pfd::paged_decode_fp8_partial_tma_kernel<QBF16, kWarpsT, kStagesT, LONERS>;
   constexpr int smem = 1024 + kWarpsT * kStagesT * 8192 + kWarpsT * kStagesT * 8 + 2 * kWarpsT * 16 * 4 +
-                       (LONERS ? kWarpsT * 4 + pfd::kGroupedMaxBatch * 2 : 0);
+                       (LONERS ? kWarpsT * 4 + 2 * 4 + pfd::kGroupedMaxBatch * 2 : 0);
   static std::atomic<bool> configured[kMaxDevices];  // (one array per instantiation)
   if (int rc = configure_smem(configured, kernel, smem, kWarpsT != kWarps)) return rc;
   {

@@ -820,11 +820,17 @@ paged_decode_fp8_partial_tma_kernel(const KernelParams p, const TmaParams tp,
   float* sm_l = sm_m + NWARPS * 16;
   float* sm_o = reinterpret_cast<float*>(ring_ptr);
   static_assert(NSTAGE * kStageBytes >= 16 * D * 4, "merge buffer must fit in the ring");
-  // LONERS only: counts of the scan below, then the requests in no group, ascending
+  // LONERS only: counts of the scan below, size and number of the splits of the requests in no group, then
+  // those requests, ascending
   int* sm_count = reinterpret_cast<int*>(sm_l + NWARPS * 16);
-  uint16_t* sm_loners = reinterpret_cast<uint16_t*>(sm_count + NWARPS);
+  int* sm_split = sm_count + NWARPS;
+  uint16_t* sm_loners = reinterpret_cast<uint16_t*>(sm_split + 2);
   if constexpr (LONERS) {
     if (takes_turns) {
+      // (worked out before the scan, whose barriers publish it: behind it this was one more round trip and an
+      // integer division in front of each CTA's first item, 3.3 of 260.5 us for a step of eight layers)
+      const int loner_size = split_size_of(p, 0), loner_splits = loner_split_count(p.loner, loner_size);
+      if (threadIdx.x == 0) { sm_split[0] = loner_size; sm_split[1] = loner_splits; }
       int n_loners = 0;
       for (int b0 = 0; b0 < p.batch; b0 += NWARPS * 32) {
         const int r = b0 + (int)threadIdx.x;
@@ -840,7 +846,7 @@ paged_decode_fp8_partial_tma_kernel(const KernelParams p, const TmaParams tp,
         if (mine) sm_loners[before + __popc(votes & ((1u << lane) - 1u))] = (uint16_t)r;
         __syncthreads();
       }
-      n_items = n_loners * p.num_kv_heads * loner_split_count(p.loner, split_size_of(p, 0));
+      n_items = n_loners * p.num_kv_heads * loner_splits;
       item = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z);
     } else {
       b -= p.loner.rows;
@@ -856,7 +862,7 @@ paged_decode_fp8_partial_tma_kernel(const KernelParams p, const TmaParams tp,
   if constexpr (LONERS) {
     if (takes_turns) {
       // splits of a request side by side; those behind its end are passed over
-      const int loner_size = split_size_of(p, 0), loner_splits = loner_split_count(p.loner, loner_size);
+      const int loner_size = sm_split[0], loner_splits = sm_split[1];
       for (;; item += p.loner.rows * p.loner_grid_row) {
         if (item >= n_items) break;
         split = item % loner_splits;
@@ -876,7 +882,7 @@ paged_decode_fp8_partial_tma_kernel(const KernelParams p, const TmaParams tp,
     if (waits_at_exit) pdl_wait();
     return;
   }
-  const int split_sz = split_size_of(p, kv0);
+  const int split_sz = LONERS && takes_turns ? sm_split[0] : split_size_of(p, kv0);
   const int lo = kv0 + split * split_sz;
 
   // Page ids of this warp's first 16 page pairs, one page per lane, fetched before the
@@ -894,7 +900,7 @@ paged_decode_fp8_partial_tma_kernel(const KernelParams p, const TmaParams tp,
   // grouped decode: the grid was sized from the caller's bound on the suffixes; a request that
   // needs more splits than the grid has would lose its tail silently, so it is reported instead
   if (p.row_kv_start != nullptr && split == 0 && kvh == 0 && threadIdx.x == 0 &&
-      seq_len - kv0 > (takes_turns ? loner_split_count(p.loner, split_sz) : (int)gridDim.x) * (int64_t)split_sz)
+      seq_len - kv0 > (LONERS && takes_turns ? sm_split[1] : (int)gridDim.x) * (int64_t)split_sz)
     atomicExch(tp.status, kErrSuffixBound);
   if (lo >= hi) {
     if (waits_at_exit) pdl_wait();
