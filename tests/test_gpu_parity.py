@@ -527,9 +527,9 @@ def test_cuda_graph_capture_and_replay(built_libs):
 
 
 # ---------------------------------------------------------------- balanced kernel, head_dim 64
-@pytest.mark.parametrize("layout", ["nhd", "hnd"])
+@pytest.mark.parametrize("layout,dtype", [("nhd", torch.bfloat16), ("hnd", torch.bfloat16), ("nhd", torch.float16)])
 @pytest.mark.parametrize("d,hq,hkv", [(64, 14, 2), (64, 8, 1), (64, 8, 8), (64, 6, 3), (64, 9, 1)])
-def test_balanced_kernel_with_head_dim_64(cabi, d, hq, hkv, layout):
+def test_balanced_kernel_with_head_dim_64(cabi, d, hq, hkv, layout, dtype):
     """Batches large enough for the balanced kernel: every length around a page and a page pair, empty and long sequences,
     unaligned kv_start, packed output, NaN bytes in the unused slots, a workspace with room for all warp groups and for
     three quarters of them; and what the grid keeps: less room, nine heads per KV head, the fixed-split flag."""
@@ -547,7 +547,7 @@ def test_balanced_kernel_with_head_dim_64(cabi, d, hq, hkv, layout):
         at += n
     kc, ks = oracle.quantize_fp8_e4m3_per_head(torch.randn(total, 16, hkv, d, generator=gen))
     vc, vs = oracle.quantize_fp8_e4m3_per_head(torch.randn(total, 16, hkv, d, generator=gen))
-    q = torch.randn(batch, hq, d, generator=gen).to(torch.bfloat16)
+    q = torch.randn(batch, hq, d, generator=gen).to(dtype)
     for c in (kc, vc):  # what no sequence owns: NaN
         for b, n in enumerate(lens.tolist()):
             if n % 16:
@@ -556,7 +556,8 @@ def test_balanced_kernel_with_head_dim_64(cabi, d, hq, hkv, layout):
     g = [t.to(DEV) for t in (q, kc, vc, table, lens)]
     if layout == "hnd":
         g[1:3] = [t.permute(0, 2, 1, 3).contiguous().permute(0, 2, 1, 3) for t in g[1:3]]
-    all_rows = 2 * (148 * 16 // hkv) * hq
+    all_groups = torch.cuda.get_device_properties(DEV).multi_processor_count * 16 // hkv
+    all_rows = 2 * all_groups * hq
     for kv_start in (0, 21):
         live = lens > kv_start
         exp = torch.zeros(batch, hq, d)
@@ -573,15 +574,49 @@ def test_balanced_kernel_with_head_dim_64(cabi, d, hq, hkv, layout):
                 packed_output=pk, workspace=ws, kv_start=kv_start, flags=flags)
             torch.cuda.synchronize()
             assert cabi.device_status() == 0
-            what = f"d={d} hq={hq} hkv={hkv} {layout} kv_start={kv_start} rows={rows} flags={flags} packed={packed}"
+            what = f"d={d} hq={hq} hkv={hkv} {layout} {dtype} kv_start={kv_start} rows={rows} flags={flags} packed={packed}"
             room = batch * ws[0].shape[2] // 2
-            grid = flags & 8 or hq // hkv > 8 or 4 * room < 3 * (148 * 16 // hkv)
+            grid = flags & 8 or hq // hkv > 8 or 4 * room < 3 * all_groups
             assert cabi.last_path() == (PATH_LDG if grid else PATH_BALANCED), what
             if packed:
                 o, m, l = pk[..., :d], pk[..., d], pk[..., d + 1]
                 assert torch.equal(l.cpu() > 0, live[:, None].expand(batch, hq)), what
                 out = torch.where(l[..., None] > 0, o / l[..., None], 0.0).to(q.dtype)
             assert_within_gate(out, exp.to(q.dtype), what)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("rows_per_sm,longest", [(6, 2100), (10, 4100)])
+def test_head_dim_64_rows_merged_by_four_warps(cabi, rows_per_sm, longest, dtype):
+    """The merge kernel gives a row four warps at up to eight rows per SM, and up to sixteen where sequences can be longer
+    than 4096 tokens: sequences of many pieces, of one, and of none, packed and final."""
+    sms = torch.cuda.get_device_properties(DEV).multi_processor_count
+    d, hq, hkv = 64, 14, 2
+    batch = max(rows_per_sm * sms // hq, -(-(1 << 17) // longest))
+    gen = torch.Generator().manual_seed(longest)
+    lens = torch.randint(1, 200, (batch,), generator=gen).to(torch.int32)
+    lens[:4] = torch.tensor([longest, 0, longest - 1, 33])
+    pages = 400
+    table = torch.randint(0, pages, (batch, -(-longest // 16)), generator=gen).to(torch.int32)
+    kc, ks = oracle.quantize_fp8_e4m3_per_head(torch.randn(pages, 16, hkv, d, generator=gen))
+    vc, vs = oracle.quantize_fp8_e4m3_per_head(torch.randn(pages, 16, hkv, d, generator=gen))
+    q = torch.randn(batch, hq, d, generator=gen).to(dtype)
+    live = lens > 0
+    exp = torch.zeros_like(q)
+    exp[live] = oracle.reference(q[live], kc, vc, table[live].long(), lens[live], ks, vs)
+    g = [t.to(DEV) for t in (q, kc, vc, table, lens)]
+    ws = workspace(g[0], longest, 512, min_rows=2 * (sms * 16 // hkv) * hq + 2 * hq)
+    for packed in (False, True):
+        out = torch.full_like(g[0], float("nan"))
+        pk = torch.full((batch, hq, d + 2), float("nan"), device=DEV) if packed else None
+        cabi.paged_decode_fp8_e4m3_split_out(*g, k_scale=ks.to(DEV), v_scale=vs.to(DEV), max_seq_len=longest, split_size=512,
+                                             output=None if packed else out, packed_output=pk, workspace=ws)
+        torch.cuda.synchronize()
+        assert cabi.device_status() == 0 and cabi.last_path() == PATH_BALANCED
+        if packed:
+            o, l = pk[..., :d], pk[..., d + 1:]
+            out = torch.where(l > 0, o / l, 0.0).to(q.dtype)
+        assert_within_gate(out, exp, f"batch={batch} longest={longest} {dtype} packed={packed}")
 
 
 @pytest.mark.parametrize("what", ["d64 partials", "d128 partials", "d64 packed", "d128 packed", "kv16 packed", "kv16 packed fused"])

@@ -259,3 +259,35 @@ def test_chunk_kernel_edges_bit_for_bit(built_libs, is_neox, cache):
         for name, got, exp in zip(("query", "key", "key cache", "value cache"), (gq, gk, gkc, gvc), want):
             assert torch.equal(as_bytes(got), as_bytes(exp)), f"{name}: case {seed} neox={is_neox} cache={cache}"
         assert torch.equal(as_bytes(gv), as_bytes(v))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_every_finite_value_quantised_as_by_a_division(built_libs, dtype):
+    """All finite 16-bit values as V, at 75 scales (powers of two, where quotients tie, their neighbours, and others): the bytes
+    of x / scale rounded, saturated, without a division per value."""
+    from single_gpu_inference_lab_b200 import l20_rope_kv
+
+    bits = torch.arange(-(1 << 15), 1 << 15, dtype=torch.int32).to(torch.int16)
+    x = bits.view(dtype)
+    x = torch.where(x.float().abs() <= torch.finfo(dtype).max, x, torch.zeros_like(x))  # (NaN compares false)
+    d, hkv = 128, 4
+    tokens = x.numel() // (d * hkv)
+    v = x.view(tokens, hkv, d)
+    zeros = torch.zeros_like(v)
+    pos, slots = torch.zeros(tokens, dtype=torch.long), torch.arange(tokens)
+    cs = torch.zeros(1, d)
+    gen = torch.Generator().manual_seed(17)
+    powers = [2.0 ** e for e in range(-12, 13)]
+    near = [p * (1 + s * 2.0 ** -23) for p in powers[::5] for s in (-1, 1)]
+    others = torch.exp(torch.rand(75 - len(powers) - len(near), generator=gen) * 16 - 11).tolist()
+    g = [t.to(DEV) for t in (zeros, zeros, v, pos, cs, slots)]
+    kc = torch.zeros(tokens // 16, 16, hkv, d, dtype=torch.float8_e4m3fn, device=DEV)
+    vc = torch.zeros_like(kc)
+    one = torch.ones(hkv, device=DEV)
+    for scale in powers + near + others:
+        s = torch.full((hkv,), scale, dtype=torch.float32)
+        l20_rope_kv.l20_rope_and_cache(g[0], g[1], g[2], g[3], g[4], True, kc, vc, g[5], k_scale=one, v_scale=s.to(DEV))
+        got = vc.view(torch.uint8).cpu().view(tokens, hkv, d)
+        want = oracle.quantize(v, s).view(torch.uint8)
+        assert torch.equal(got, want), f"scale {scale!r}: {int((got != want).sum())} bytes differ"
