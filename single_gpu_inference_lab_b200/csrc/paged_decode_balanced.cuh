@@ -102,6 +102,9 @@ __device__ __forceinline__ void bal_reset(BalState<NH, D>& st) {
 }
 
 // Q of head (8h + i) as B-fragments: k-step ks = 4l + w covers d = 16(j+4l) + 4w + {0,1 | 2,3}.
+// (Ordinary loads, here and for the plan: the kernel in front may write what this one reads while this one is
+// resident and waits for it.  The read-only path is for what does not change as long as a kernel lasts, and
+// the compiler may move such loads over the wait.)
 template <bool QBF16, int NH, int D>
 __device__ __forceinline__ void bal_load_q(uint32_t (&qb)[NH][D / 16][2], const KernelParams& p, int b,
                                            int kvh, int i, int j) {
@@ -116,7 +119,7 @@ __device__ __forceinline__ void bal_load_q(uint32_t (&qb)[NH][D / 16][2], const 
 #pragma unroll
       for (int w = 0; w < 4; ++w) {
         uint2 raw = make_uint2(0u, 0u);
-        if (live) raw = __ldg(reinterpret_cast<const uint2*>(q + 16 * (j + 4 * l) + 4 * w));
+        if (live) raw = *reinterpret_cast<const uint2*>(q + 16 * (j + 4 * l) + 4 * w);
         if constexpr (QBF16) {
           const __nv_bfloat162 a = *reinterpret_cast<const __nv_bfloat162*>(&raw.x);
           const __nv_bfloat162 c = *reinterpret_cast<const __nv_bfloat162*>(&raw.y);
@@ -398,8 +401,8 @@ __device__ __forceinline__ void kv16_load_q(uint32_t (&qb)[1][8][2], const Kerne
       (int64_t)(kvh * p.group + (live ? i : 0)) * p.q_stride_h);
 #pragma unroll
   for (int ks = 0; ks < 8; ++ks) {
-    qb[0][ks][0] = live ? __ldg(q + 8 * ks + j) : 0u;
-    qb[0][ks][1] = live ? __ldg(q + 8 * ks + 4 + j) : 0u;
+    qb[0][ks][0] = live ? q[8 * ks + j] : 0u;
+    qb[0][ks][1] = live ? q[8 * ks + 4 + j] : 0u;
   }
 }
 
@@ -917,19 +920,19 @@ paged_decode_fp8_chunk_kernel(const KernelParams p, const TmaParams tp, const Ch
     // one round trip: header, this group's range and the page ids of its first 16 pairs.  Every
     // lane reads the same header words (broadcast loads), so nothing below depends on the lane.
     const int32_t* gw = cp.plan + plan_groups_off(B) + (int64_t)min(grp, num_groups - 1) * kPlanGroupWords;
-    const int4 h0 = __ldg(reinterpret_cast<const int4*>(cp.plan));      // magic, batch, kv_start, kv heads
-    const int4 h1 = __ldg(reinterpret_cast<const int4*>(cp.plan) + 1);  // groups, piece cost, total, indptr
-    const int4 g0 = __ldg(reinterpret_cast<const int4*>(gw));  // P0, P1, pairs that end a sequence
+    const int4 h0 = reinterpret_cast<const int4*>(cp.plan)[0];  // magic, batch, kv_start, kv heads
+    const int4 h1 = reinterpret_cast<const int4*>(cp.plan)[1];  // groups, piece cost, total, indptr
+    const int4 g0 = *reinterpret_cast<const int4*>(gw);  // P0, P1, pairs that end a sequence
     cr.P0 = g0.x;
     cr.P1 = g0.y;
     seq_ends = (uint32_t)g0.z;
-    ids_cur = __ldg(gw + 4 + lane);
+    ids_cur = gw[4 + lane];
     plan_ok = h0.x == kPlanMagic && h0.y == B && h0.z == p.kv_start && h0.w == hkv && h1.x == num_groups &&
               h1.y == cp.piece_cost && h1.w == (p.page_indptr != nullptr ? 1 : 0);
     total = h1.z;
     if (grp >= num_groups || !plan_ok) { cr.P0 = cr.P1 = total; ids_cur = -1; }
     // prefix sum and lengths into shared memory; used only after the barrier further down
-    for (int x = threadIdx.x; x < 2 * B + 1; x += NT) prefix[x] = __ldg(cp.plan + kPlanHeaderWords + x);
+    for (int x = threadIdx.x; x < 2 * B + 1; x += NT) prefix[x] = cp.plan[kPlanHeaderWords + x];
   } else {
     scan_pairs<NT>(p.seq_lens, B, p.kv_start, sm_scan, prefix, lens);  // ends with the last CTA-wide barrier
     total = prefix[B];
@@ -1249,9 +1252,9 @@ paged_decode_chunk_merge_kernel(const KernelParams p, const TmaParams tp, const 
   int below = 0, all = 0, np = 0;
   if (cp.plan != nullptr) {
     const int32_t* pre = cp.plan + kPlanHeaderWords;
-    below = __ldg(pre + b);
-    np = __ldg(pre + b + 1) - below;
-    all = __ldg(pre + cp.batch);
+    below = pre[b];
+    np = pre[b + 1] - below;
+    all = pre[cp.batch];
   } else {
     for (int x = lane; x < cp.batch; x += 32) {
       const int n = pairs_of(__ldg(p.seq_lens + x), p.kv_start);

@@ -214,6 +214,65 @@ def test_append_then_decode_equals_the_oracles(built_libs):
         assert_within_gate(out, exp, f"append + planned decode with early K/V, repetition {rep}")
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("kv_stable", [False, True])
+def test_recorded_producer_and_decode_read_what_the_step_wrote(built_libs, kv_stable):
+    """Plan, append and decode recorded, then replayed behind one another with new lengths, rows and slots: the decode kernel,
+    resident while the append kernel runs, reads this replay's plan, rotated queries and new tokens."""
+    from single_gpu_inference_lab_b200 import l20_paged_split_kv, l20_rope_kv
+    from single_gpu_inference_lab_b200.workloads import make_inputs
+
+    w = make_inputs("qwen2.5-coder-3b-b64", seed=13, batch=16, shrink=0.25)
+    batch, hq, d = w.query.shape
+    hkv, replays = w.key_cache.shape[2], 6
+    gen = torch.Generator().manual_seed(14)
+    angle = torch.arange(w.max_seq_len)[:, None] * (1e4 ** (-torch.arange(0, d, 2) / d))[None, :]
+    cos_sin = torch.cat([torch.cos(angle), torch.sin(angle)], dim=1).float()
+    lens = torch.stack([(w.seq_lens - i).clamp_min(1) for i in range(replays)])
+    rows = torch.randn(replays, batch, hq + 2 * hkv, d, generator=gen).to(torch.bfloat16)
+    positions = lens.long() - 1
+    slots = w.block_table[torch.arange(batch), positions // 16].long() * 16 + positions % 16
+    g = w.to(DEV)
+    g_lens, g_rows, g_positions, g_slots, g_cs = (t.to(DEV) for t in (lens, rows, positions, slots, cos_sin))
+    now_lens, now_rows, now_positions, now_slots = (t[0].clone() for t in (g_lens, g_rows, g_positions, g_slots))
+    ws = l20_paged_split_kv.allocate_l20_paged_split_kv_workspace(g.query, w.max_seq_len, split_size=512)
+    shape = dict(max_seq_len=w.max_seq_len, split_size=512, workspace=ws)
+    caches = g.key_cache, g.value_cache, g.block_table
+    plan = l20_paged_split_kv.plan_l20_paged_split_kv(g.query, *caches, now_lens, **shape)
+    out, work = torch.empty_like(g.query), torch.empty_like(now_rows)
+
+    def step():
+        l20_paged_split_kv.plan_l20_paged_split_kv(g.query, *caches, now_lens, plan=plan, **shape)
+        work.copy_(now_rows)
+        q, k, v = work[:, :hq], work[:, hq:hq + hkv], work[:, hq + hkv:]
+        l20_rope_kv.l20_rope_and_cache(q, k, v, now_positions, g_cs, True, g.key_cache, g.value_cache, now_slots,
+                                       k_scale=g.k_scale, v_scale=g.v_scale)
+        l20_paged_split_kv.l20_paged_split_kv_attention_fp8(q, *caches, now_lens, k_scale=g.k_scale, v_scale=g.v_scale, plan=plan,
+                                                            output=out, metadata_stable=True, kv_stable=kv_stable, **shape)
+
+    kc, vc = w.key_cache, w.value_cache
+    kc0, vc0 = g.key_cache.clone(), g.value_cache.clone()
+    step()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        step()
+    g.key_cache.copy_(kc0)
+    g.value_cache.copy_(vc0)
+    got = []
+    for r in range(replays):
+        for now, new in ((now_lens, g_lens), (now_rows, g_rows), (now_positions, g_positions), (now_slots, g_slots)):
+            now.copy_(new[r])
+        graph.replay()
+        got.append(out.clone())
+    torch.cuda.synchronize()
+    for r in range(replays):
+        q, k, v = rows[r][:, :hq], rows[r][:, hq:hq + hkv], rows[r][:, hq + hkv:]
+        q, _, kc, vc = oracle.rope_and_cache(q, k, v, positions[r], cos_sin, True, kc, vc, slots[r], w.k_scale, w.v_scale)
+        exp = decode_oracle.reference(q, kc, vc, w.block_table.long(), lens[r], w.k_scale, w.v_scale)
+        assert_within_gate(got[r], exp, f"replay {r} kv_stable={kv_stable}")
+
+
 def test_wrapper_argument_errors_without_a_gpu():
     from single_gpu_inference_lab_b200 import l20_rope_kv
 
