@@ -351,8 +351,9 @@ bool balanced_eligible(const pfd_decode_args& a, int group, int slot_offset, int
 // The balanced kernel for head_dim 64 (up to eight query heads per KV head): pages are half as many bytes
 // and a page pair nearly as many instructions as with 128, so sixteen warps share an SM's 192 KiB
 // ring, three 4 KiB stages each (14 + 2 heads, batch 256, 512 .. 4096 tokens, us per call: 8 warps 42.7, 12
-// 37.4, 16 37.2; the fixed-split grid with plain loads 53.3).  It needs slots for three quarters of
-// its warp groups: us balanced / grid, 14 + 2 heads, lengths all alike, uniform, log-uniform to the maximum
+// 37.4, 16 37.2; the fixed-split grid with plain loads 53.3; all with a running maximum up to 8 (log2) behind the true
+// one, with which the 37.2 are 37.7).  It needs slots for three quarters of its warp groups: us balanced / grid
+// (measured likewise), 14 + 2 heads, lengths all alike, uniform, log-uniform to the maximum
 //   room 0.86: 128 x 8192: 53.2 / 77.1, 34.7 / 48.2, 17.0 / 17.9   256 x 4096: 56.2 / 77.1, 37.5 / 51.2, 17.7 / 19.4
 //   room 0.43: 128 x 4096: 40.8 / 43.7, 26.9 / 28.4, 14.3 / 14.0    64 x 8192: 39.8 / 43.6, 25.0 / 23.8, 13.9 / 13.0
 //   room 0.22:  64 x 4096: 34.6 / 20.4, 23.8 / 16.8, 11.6 /  9.9
@@ -452,6 +453,7 @@ int launch_balanced(const pfd_decode_args& a, const pfd::KernelParams& kp, int s
     // (one warp per row on the batch-64 configuration: 21.0 against 19.9 us).  Head_dim 64, whose rows are
     // half as long, up to sixteen rows per SM where sequences can be long, i.e. have many pieces: batch
     // 128 x 8192, log-uniform: 20.8 -> 17.0 us per call; batch 256 x 1024, 8 KV heads, would lose (48.5 -> 50.8).
+    // (These two points only.)
     const bool wide = rows <= 8 * sms || (D == 64 && rows <= 16 * sms && a.max_seq_len > 4096);
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(wide ? rows : (rows + 3) / 4);
@@ -693,7 +695,8 @@ int log2_or_none(int x) { return x > 0 && (x & (x - 1)) == 0 ? __builtin_ctz(sta
 // us at 256 / 128 / 64 / 32 threads per token, 28 + 4 heads of 128, FP8 cache, 148 SMs:
 //   512 tokens 4.1 / 4.2 / 5.4 / 7.7    1024: 6.2 / 5.5 / 6.2 / 7.9    2048: 10.2 / 8.8 / 8.6 / 8.9
 //   4096: 17.5 / 14.8 / 14.0 / 13.9     8192: 40.1 / 32.4 / 29.1 / 27.2 (28.4 as it stands)
-// A token's threads have to cover the rotation tasks of one head (16 elements each).
+// (That geometry only: the rule goes by the tokens, not by heads x head_dim.)  A token's threads have to
+// cover the rotation tasks of one head (16 elements each).
 constexpr int kRopeMaxRotary = 16 * 32;
 template <bool BF16, bool NEOX>
 cudaError_t launch_rope_vec(const pfd::RopeParams& p, int sms, cudaStream_t stream) {

@@ -859,7 +859,7 @@ __device__ __forceinline__ void write_empty_sequence(const KernelParams& p, int 
 // follows.  FUSED is a separate instantiation because the merge code costs the streaming loop
 // registers; on B200 it is the slower of the two (one warp per sequence and kv head merges
 // where the merge kernel has a warp per row).
-// D = 64 (e4m3 only): the same with 64-byte rows; see launch_decode for what runs it.
+// D = 64 (e4m3 only): the same with 64-byte rows; see balanced64_groups for what runs it.
 template <bool QBF16, int NSTAGE, int NWARPS, bool KV16 = false, bool FUSED = false, int D = 128>
 __global__ void __launch_bounds__(NWARPS * 32, 1)
 paged_decode_fp8_chunk_kernel(const KernelParams p, const TmaParams tp, const ChunkParams cp,

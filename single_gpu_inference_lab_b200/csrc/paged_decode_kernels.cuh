@@ -783,7 +783,8 @@ __global__ void bounded_wait_selftest_kernel(int32_t* status, unsigned long long
 // another's suffix; cut into as many splits as those, it is one chain of a dozen page pairs per
 // warp that the whole step waits for: with 64 requests, two groups behind 4096 and 5120 tokens and 8
 // requests of 4.3 K tokens in none, 2 kv heads, this pass took 29 us and a step of eight layers
-// 357 us that way, and 260 us with 256 tokens to an item (128: 260, 512: 266).
+// 358 us that way, and 258 us with 256 tokens to an item.  (128 cost the same and 512 2 % more, on this batch;
+// others were not measured.)
 template <bool QBF16, int NWARPS, int NSTAGE, bool LONERS = false>
 __global__ void __launch_bounds__(NWARPS * 32, NWARPS <= 12 ? 12 / NWARPS : 1)  // twelve warps per SM: at most 168 registers
 paged_decode_fp8_partial_tma_kernel(const KernelParams p, const TmaParams tp,
