@@ -73,7 +73,10 @@ extern "C" {
  * Stream order.  Every kernel of a call is launched with programmatic stream serialisation: it may
  * become resident while the kernel in front of it in the stream drains, but it reads and writes
  * nothing before that kernel has completed -- except, under PFD_FLAG_EARLY_METADATA, seq_lens,
- * block_table and the plan.  The last kernel of a call completes only after every kernel of the
+ * block_table and the plan, and except the merge kernel of a call without a plan, which may read seq_lens as
+ * soon as the kernel in front of the call has let its dependents in: a kernel of the caller's that writes
+ * seq_lens and triggers early (griddepcontrol.launch_dependents) has to write them first; one that does
+ * not trigger, i.e. any ordinary kernel, is complete by then.  The last kernel of a call completes only after every kernel of the
  * call has (whatever rows it had to merge itself), so whoever enqueues work behind a call, with or
  * without programmatic launch attributes, finds the call's output complete.  Nothing is allocated,
  * nothing synchronises with the host; the entry points that take a workspace are captured in CUDA
