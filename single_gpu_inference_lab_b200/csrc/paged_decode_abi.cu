@@ -13,7 +13,7 @@
 #include <vector>
 
 #include "paged_decode_balanced.cuh"
-#include "shared_prefix_dense.cuh"
+#include "shared_prefix_fused.cuh"
 #include "paged_decode_kernels.cuh"
 #include "rope_kv_append.cuh"
 #include "shared_prefix_groups.cuh"
@@ -470,8 +470,71 @@ int launch_balanced(const pfd_decode_args& a, const pfd::KernelParams& kp, int s
   return check_launch("balanced merge kernel");
 }
 
+// What the fused shared-prefix kernel is told beside the split-KV arguments.
+struct FusedPrefix {
+  int prefix_len;         // tokens that all requests share, or (groups) the cap on the groups' prefixes
+  const int32_t* groups;  // groups buffer on the device, or nullptr
+  int max_groups;
+};
+
+template <bool QBF16>
+int launch_fused(const pfd_decode_args& a, const pfd::KernelParams& kp, const FusedPrefix& f, cudaStream_t stream) {
+  CUtensorMap mk, mv;
+  if (int rc = get_tensor_map(a.key_cache, a.k_stride_page, a.k_stride_token, a.k_stride_head, a.num_pages,
+                              a.num_kv_heads, 256, &mk))
+    return rc;
+  if (int rc = get_tensor_map(a.value_cache, a.v_stride_page, a.v_stride_token, a.v_stride_head, a.num_pages,
+                              a.num_kv_heads, 256, &mv))
+    return rc;
+  pfd::TmaParams tp{};
+  tp.head_is_dim1 = head_is_dim1(a.k_stride_token, a.k_stride_head) ? 1 : 0;
+  if (int rc = status_pointer(&tp.status)) return rc;
+  tp.wait_limit_ns = g_wait_limit_ns.load(std::memory_order_relaxed);
+  pfd::PrefixParams pp{};
+  pp.prefix_len = f.prefix_len;
+  pp.batch = a.batch;
+  pp.groups = f.groups;
+  pp.groups_batch = a.batch;
+  pp.max_groups = f.max_groups;
+  pp.status = tp.status;
+  pp.wait_limit_ns = tp.wait_limit_ns;
+  pp.phase_times = g_phase_times;
+  auto kernel = pfd::shared_prefix_fused_kernel<QBF16>;
+  static std::atomic<bool> configured[kMaxDevices], checked[kMaxDevices];
+  if (int rc = configure_smem(configured, kernel, pfd::kFusedSmem)) return rc;
+  if (!checked[t_device->dev].load(std::memory_order_acquire)) {
+    // the warps' register shares add up to what the block is launched with, or the second half would wait for ever
+    cudaFuncAttributes attr;
+    const cudaError_t e = cudaFuncGetAttributes(&attr, kernel);
+    if (e != cudaSuccess) return fail(PFD_ERR_CUDA, "cudaFuncGetAttributes failed: %s", cudaGetErrorString(e));
+    if ((attr.numRegs + 7) / 8 * 8 != pfd::kFusedRegs)
+      return fail(PFD_ERR_CUDA, "fused shared-prefix kernel built with %d registers a thread, not %d", attr.numRegs, pfd::kFusedRegs);
+    checked[t_device->dev].store(true, std::memory_order_release);
+  }
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(t_device->sms);
+  cfg.blockDim = dim3(pfd::kFusedThreads);
+  cfg.dynamicSmemBytes = pfd::kFusedSmem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, kp, tp, pp, mk, mv);
+  if (e != cudaSuccess) return fail(PFD_ERR_CUDA, "fused shared-prefix kernel launch failed: %s", cudaGetErrorString(e));
+  return check_launch("fused shared-prefix kernel");
+}
+
+// Calls that the fused kernel takes.
+bool fused_eligible(const pfd_decode_args& a, int prefix_chunks) {
+  if (prefix_chunks <= 0 || a.head_dim != 128 || !tma_eligible(a)) return false;
+  if (g_suffix_form.load(std::memory_order_relaxed) >= 0) return false;  // a form of the two-kernel passes is asked for
+  return a.num_q_heads / a.num_kv_heads <= 8 && a.batch <= pfd::kGroupedMaxBatch;
+}
+
 template <int D, bool QBF16>
-int launch_decode(const pfd_decode_args& a, const pfd::KernelParams& kp, int num_splits) {
+int launch_decode(const pfd_decode_args& a, const pfd::KernelParams& kp, int num_splits, const FusedPrefix* fused) {
   cudaStream_t stream = static_cast<cudaStream_t>(a.stream);
   if constexpr (D == 128) {
     const int sms = t_device->sms;
@@ -486,7 +549,10 @@ int launch_decode(const pfd_decode_args& a, const pfd::KernelParams& kp, int num
                 "page_indptr addressing needs the balanced kernel (head_dim 128, at most 8 query heads per KV "
                 "head, dense f32 workspace of pfd_balanced_workspace_rows() rows)");
   const dim3 grid(num_splits, a.num_kv_heads, a.batch);
-  if (D == 128 && tma_eligible(a)) {
+  if (D == 128 && fused != nullptr) {
+    g_last_path = PFD_PATH_FIXED_TMA;
+    if (int rc = launch_fused<QBF16>(a, kp, *fused, stream)) return rc;
+  } else if (D == 128 && tma_eligible(a)) {
     g_last_path = PFD_PATH_FIXED_TMA;
     const dim3 grid_with_loners(num_splits, a.num_kv_heads, a.batch + kp.loner.rows);  // (rows > 0: not beside the prefix)
     if (int rc = kp.loner.rows > 0 ? launch_partial_tma<QBF16, kWarps, kStages, true>(a, kp, grid_with_loners, stream)
@@ -591,8 +657,8 @@ pfd::KernelParams fill_params(const pfd_decode_args& a, int group, bool direct_o
     kp.loner = grouped->loner;
     kp.loner_grid_row = grouped->num_splits * a.num_kv_heads;
     kp.grouped_count = grouped->grouped_count;
-    kp.batch = a.batch;
   }
+  kp.batch = a.batch;
   kp.early_metadata = (a.flags & PFD_FLAG_EARLY_METADATA) ? 1 : 0;
   kp.early_kv = (kp.early_metadata && (a.flags & PFD_FLAG_EARLY_KV)) ? 1 : 0;
   kp.kv_evict_first = 1;
@@ -615,7 +681,8 @@ pfd::KernelParams fill_params(const pfd_decode_args& a, int group, bool direct_o
 
 // slot_offset > 0: workspace slots [0, slot_offset) are filled by the dense prefix pass; the
 // split-KV kernels then write behind them and the merge kernel covers both.
-int decode_impl(const pfd_decode_args* args, int slot_offset, const GroupedRows* grouped = nullptr) {
+int decode_impl(const pfd_decode_args* args, int slot_offset, const GroupedRows* grouped = nullptr,
+                const FusedPrefix* fused = nullptr) {
   if (args == nullptr) return fail(PFD_ERR_INVALID, "args is NULL");
   if (args->struct_size != sizeof(pfd_decode_args))
     return fail(PFD_ERR_INVALID, "pfd_decode_args size mismatch: caller %u, library %zu",
@@ -680,12 +747,13 @@ int decode_impl(const pfd_decode_args* args, int slot_offset, const GroupedRows*
   }
 
   if (int rc = enter_call()) return rc;  // (argument errors above are reported without a device)
-  const pfd::KernelParams kp = fill_params(a, group, direct_ok, slot_offset, grouped);
+  pfd::KernelParams kp = fill_params(a, group, direct_ok, slot_offset, grouped);
+  if (fused != nullptr) kp.fused_splits = num_splits;
 
   const bool bf16 = a.query_dtype == PFD_DTYPE_BF16;
   if (a.head_dim == 128)
-    return bf16 ? launch_decode<128, true>(a, kp, num_splits) : launch_decode<128, false>(a, kp, num_splits);
-  return bf16 ? launch_decode<64, true>(a, kp, num_splits) : launch_decode<64, false>(a, kp, num_splits);
+    return bf16 ? launch_decode<128, true>(a, kp, num_splits, fused) : launch_decode<128, false>(a, kp, num_splits, fused);
+  return bf16 ? launch_decode<64, true>(a, kp, num_splits, nullptr) : launch_decode<64, false>(a, kp, num_splits, nullptr);
 }
 
 int log2_or_none(int x) { return x > 0 && (x & (x - 1)) == 0 ? __builtin_ctz(static_cast<unsigned>(x)) : -1; }
@@ -756,7 +824,7 @@ int launch_prefix(const pfd_decode_args& a, int prefix_len, int chunks, bool suf
   // the slim instantiation (80 registers, whole-SM carve-out) leaves room for the suffix pass's
   // two-warp CTAs on the same SM; it is 1 us slower by itself, so the other one runs otherwise
   auto kernel = suffix_beside ? pfd::shared_prefix_dense_kernel<QBF16, true> : pfd::shared_prefix_dense_kernel<QBF16, false>;
-  constexpr int smem = 1024 + 160 * 1024 + 32 + 2 * 4 * 128 * 4;
+  constexpr int smem = 1024 + pfd::DenseLayout::kBytes + 32;
   static std::atomic<bool> configured[2][kMaxDevices];
   if (int rc = configure_smem(configured[suffix_beside ? 1 : 0], kernel, smem, suffix_beside)) return rc;
   const int rows = a.batch * kp.group;
@@ -770,7 +838,7 @@ int launch_prefix(const pfd_decode_args& a, int prefix_len, int chunks, bool suf
   const int spare = std::max(0, std::min(max_groups, t_device->sms / std::max(chunks * a.num_kv_heads, 1) - tiles));
   const dim3 grid = groups == nullptr ? dim3(chunks, tiles, a.num_kv_heads)
                                       : dim3(chunks * a.num_kv_heads, tiles + spare, 1);
-  kernel<<<grid, 512, smem, static_cast<cudaStream_t>(a.stream)>>>(kp, pp);
+  kernel<<<grid, pfd::kDenseThreads, smem, static_cast<cudaStream_t>(a.stream)>>>(kp, pp);
   return check_launch("shared-prefix dense kernel");
 }
 }  // namespace
@@ -968,6 +1036,10 @@ int pfd_shared_prefix_decode_fp8_e4m3(const pfd_decode_args* args, int32_t prefi
                   chunks + ns);
   }
   if (int rc = enter_call()) return rc;
+  if (fused_eligible(a, chunks)) {
+    const FusedPrefix fused{prefix_len, nullptr, 0};
+    return decode_impl(&a, chunks, nullptr, &fused);
+  }
   const int span = a.max_seq_len - prefix_len;
   const bool beside = suffix_beside_prefix(a, chunks, span > 0 ? (span + a.split_size - 1) / a.split_size : 1, false);
   if (int rc = bf16 ? launch_prefix<true>(a, prefix_len, chunks, beside) : launch_prefix<false>(a, prefix_len, chunks, beside))
@@ -1029,6 +1101,14 @@ int pfd_shared_prefix_decode_grouped_fp8_e4m3(const pfd_decode_args* args, const
   a.plan = nullptr;
   if (int rc = enter_call()) return rc;
   const int32_t* g = static_cast<const int32_t*>(groups);
+  if (fused_eligible(a, chunks)) {
+    GroupedRows rows;
+    rows.row_kv_start = g + pfd::groups_row_prefix_off();
+    rows.row_kv_cap = cap;
+    rows.num_splits = ns;
+    const FusedPrefix fused{cap, g, max_groups};
+    return decode_impl(&a, chunks, &rows, &fused);
+  }
   const bool beside = suffix_beside_prefix(a, chunks, ns, true);
   if (chunks > 0)
     if (int rc = bf16 ? launch_prefix<true>(a, cap, chunks, beside, g, max_groups)

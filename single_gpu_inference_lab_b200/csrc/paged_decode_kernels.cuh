@@ -24,6 +24,7 @@
 #include <stdint.h>
 
 #include "loner_split.cuh"
+#include "suffix_cut.cuh"
 
 namespace pfd {
 
@@ -70,6 +71,9 @@ struct KernelParams {
   LonerGrid loner;
   int32_t loner_grid_row, batch;  // CTAs of one grid row; requests of the call
   const int32_t* grouped_count;  // device word: requests of the batch that are in groups
+  // Fused shared-prefix kernel (> 0): slots behind the prefix chunks' for the pieces of a request's own tokens
+  // (own_tokens); split_size x this is the caller's bound on them.
+  int32_t fused_splits;
   int32_t early_metadata;  // 1: seq_lens and block_table may be read before the preceding kernel has completed
   int32_t early_kv;        // 1: so may K/V pages, except each sequence's last (balanced kernel with a plan)
   int32_t kv_evict_first;  // 1: K/V tiles are loaded with the L2 evict-first hint
@@ -138,6 +142,27 @@ __device__ __forceinline__ int split_size_of(const KernelParams& p, int kv0) {
   if (p.row_kv_start == nullptr || kv0 != 0 || p.split_size_loner <= 0) return p.split_size;
   if (p.loner.rows == 0) return p.split_size_loner;
   return loner_split_size(p.loner, min(max(p.batch - __ldg(p.grouped_count), 0), p.batch));
+}
+
+// Fused shared-prefix kernel: own tokens of request b -- behind its prefix, or its whole context if it is in no group --
+// and the slots of their pieces: behind the prefix chunks' slots, or all of the row's.
+struct OwnTokens {
+  int kv0, live, slot0, slots;
+};
+__device__ __forceinline__ OwnTokens own_tokens(const KernelParams& p, int b) {
+  OwnTokens x;
+  // (ordinary loads: the kernel in front may write what this one reads while it is resident and waits)
+  x.kv0 = p.row_kv_start != nullptr ? min(p.row_kv_start[b] & ~15, p.row_kv_cap) : p.kv_start;
+  const bool alone = p.row_kv_start != nullptr && x.kv0 == 0;
+  x.slot0 = alone ? 0 : p.slot_offset;
+  x.slots = alone ? p.slot_offset + p.fused_splits : p.fused_splits;
+  // (no further than the caller's bounds, which the block table covers)
+  const int64_t most = alone ? (int64_t)p.bt_cols * kPage : (int64_t)p.fused_splits * p.split_size;
+  x.live = (int)min((int64_t)max(p.seq_lens[b] - x.kv0, 0), most);
+  return x;
+}
+__device__ __forceinline__ SuffixCut own_cut(const OwnTokens& x) {
+  return suffix_cut(((x.live + kPage - 1) / kPage + 1) / 2, x.slots);
 }
 
 __device__ __forceinline__ int32_t page_of(const int32_t* __restrict__ block_table,
@@ -1092,15 +1117,22 @@ paged_decode_merge_kernel(const KernelParams p, int batch) {
     return;
   }
   const int b = row / p.num_q_heads, hq = row % p.num_q_heads;
-  const int seq_len = p.seq_lens[b];
-  const int kv0 = GROUPED ? kv_start_of(p, b) : p.kv_start;
-  const int live = seq_len - kv0;
+  int kv0, own;  // first own token, pieces of the own tokens
+  if (D == 128 && p.fused_splits > 0) {
+    const OwnTokens x = own_tokens(p, b);
+    kv0 = x.kv0;
+    own = own_cut(x).pieces;
+  } else {
+    kv0 = GROUPED ? kv_start_of(p, b) : p.kv_start;
+    const int live = p.seq_lens[b] - kv0;
+    const int split_sz = GROUPED ? split_size_of(p, kv0) : p.split_size;
+    own = live > 0 ? (live + split_sz - 1) / split_sz : 0;
+  }
   // slots in front of the splits: all slot_offset of them, or (grouped) those of this row's prefix
   const int pre = GROUPED ? (kv0 + 255) / 256 : p.slot_offset;
   // unused slots between the row's prefix chunks and its splits
-  const int skip = !GROUPED || (p.loner.rows > 0 && kv0 == 0) ? 0 : p.slot_offset - pre;
-  const int split_sz = GROUPED ? split_size_of(p, kv0) : p.split_size;
-  const int ns = (live > 0 ? (live + split_sz - 1) / split_sz : 0) + pre;
+  const int skip = !GROUPED || ((p.loner.rows > 0 || p.fused_splits > 0) && kv0 == 0) ? 0 : p.slot_offset - pre;
+  const int ns = own + pre;
   constexpr int E = D / 32;  // elements per lane
   float acc[E];
 #pragma unroll

@@ -21,6 +21,8 @@
 // rows x 128 tokens), src/l20_stack/ops/triton_decode_attention.py:704-813.
 #pragma once
 
+#include <type_traits>
+
 #include "paged_decode_kernels.cuh"
 #include "shared_prefix_groups.cuh"
 
@@ -174,11 +176,261 @@ __device__ __forceinline__ void prefix_mark(const PrefixParams& pp, int k) {
 #endif
 }
 
+// One tile: 128 (request, head) rows of one kv head against one chunk of the prefix.
+struct PrefixTile {
+  int kvh, chunk, mtile;
+  int prefix_len;           // tokens shared by the rows' requests (a multiple of 16)
+  int n_req, page_row;      // those requests; whose block-table row names the prefix pages
+  const int32_t* req_list;  // request index of the i-th of them; nullptr: i itself
+};
+
+// Shared memory of the dense pass, in bytes from a 1 KiB boundary.
+struct DenseLayout {
+  static constexpr uint32_t kQ = kPrefixRows * 128 * 2;    // 32 KiB: 2 k-blocks of [128][64]; later the rows' maxima and sums
+  static constexpr uint32_t kK = kPrefixChunk * 128 * 2;   // 64 KiB: 2 k-blocks of [256][64]; later P: 4 x [128][64]; later O rows
+  static constexpr uint32_t kV = 128 * kPrefixChunk * 2;   // 64 KiB: 2 d-blocks of [256 tokens][64]
+  static constexpr uint32_t kBytes = kQ + kK + kV;
+};
+constexpr int kDenseThreads = 512;
+__device__ __forceinline__ void dense_sync() { asm volatile("bar.sync 1, %0;" ::"n"(kDenseThreads) : "memory"); }
+
+// The first kDenseThreads threads of a CTA take one tile.  Warp w works on TMEM lanes (= rows)
+// 32 * (w % 4) .. +31, the only ones it may address, and on column group w / 4 of whatever is being read:
+// with 16 warps the staging, the softmax and the stores around the two MMAs are spread over all four
+// schedulers four warps deep.
+// The pass is a chain of latencies (block table, operands, MMA, softmax, MMA, stores), so what does not
+// depend on one another is issued together: the query rows before the page id is waited for, V converted
+// and staged while the tensor cores compute S.
+// Ordinary loads throughout: as a programmatic dependent the CTA is resident while the kernel in front writes what it
+// reads behind its wait.
+// bars: two mbarriers, waited on with `parity`; false if a wait for the tensor cores gave up.
+template <bool QBF16>
+__device__ __forceinline__ bool dense_tile(const KernelParams& p, const PrefixParams& pp, const PrefixTile& tile,
+                                           uint8_t* gen, uint32_t base, uint32_t bars,
+                                           const volatile uint32_t* tslot_ptr, uint32_t parity) {
+  constexpr int D = 128;
+  const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
+  const int qd = warp & 3, cg = warp >> 2;  // TMEM lane quarter, column group
+  const int row = 32 * qd + lane;           // this thread's (request, head) row of the tile
+  const uint32_t sq = base, sk = base + DenseLayout::kQ, sv = sk + DenseLayout::kK;
+  float* red = reinterpret_cast<float*>(gen);  // [2][4][128] row partials, where the query tile was
+  const int kvh = tile.kvh, chunk = tile.chunk, n_req = tile.n_req;
+  const int tok_lo = chunk * kPrefixChunk;
+  const int tok_hi = min(tok_lo + kPrefixChunk, tile.prefix_len);
+
+  // ---- K and V chunk: warp w stages page w of the chunk (16 tokens); per load instruction its
+  // lanes cover four whole 128-byte token rows (lane = 8 * token + 16-byte group), so every
+  // sector that is fetched is used at once -- with the whole-SM shared-memory carve-out the L1
+  // is too small to keep half-used lines until the thread's next load comes back for them
+  const int e16 = lane & 7;
+  const bool live = tok_lo + kPage * warp < tok_hi;  // (the prefix ends on a page boundary)
+  int64_t phys = 0;
+  if (live) phys = p.block_table[(int64_t)tile.page_row * p.bt_stride_b + tok_lo / kPage + warp];
+  // ---- Q tile: warp w takes rows 8w .. 8w+7, two whole 256-byte rows per load instruction
+  // (lane = 16 * row + 16-byte chunk), fully used sectors as for K and V
+  uint4 qin[4];
+#pragma unroll
+  for (int it = 0; it < 4; ++it) {
+    const int rg = tile.mtile * kPrefixRows + 8 * warp + 2 * it + (lane >> 4);
+    const int req = rg / p.group;
+    qin[it] = make_uint4(0u, 0u, 0u, 0u);
+    if (req < n_req) {
+      const int rb = tile.req_list != nullptr ? tile.req_list[req] : req;
+      const uint16_t* q = reinterpret_cast<const uint16_t*>(p.query) + (int64_t)rb * p.q_stride_b +
+                          (int64_t)(kvh * p.group + rg % p.group) * p.q_stride_h;
+      qin[it] = reinterpret_cast<const uint4*>(q)[lane & 15];
+    }
+  }
+  uint4 kin[4], vin[4];
+  {
+    const uint8_t* kpage = p.key_cache + phys * p.k_stride_page + (int64_t)kvh * p.k_stride_head;
+    const uint8_t* vpage = p.value_cache + phys * p.v_stride_page + (int64_t)kvh * p.v_stride_head;
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      const int tp = 4 * c + (lane >> 3);  // token of the page
+      kin[c] = make_uint4(0u, 0u, 0u, 0u);
+      if (live) kin[c] = reinterpret_cast<const uint4*>(kpage + (int64_t)tp * p.k_stride_token)[e16];
+    }
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      const int tp = 4 * c + (lane >> 3);
+      vin[c] = make_uint4(0u, 0u, 0u, 0u);
+      if (live) vin[c] = reinterpret_cast<const uint4*>(vpage + (int64_t)tp * p.v_stride_token)[e16];
+    }
+  }
+#pragma unroll
+  for (int it = 0; it < 4; ++it) {
+    const int r = 8 * warp + 2 * it + (lane >> 4), c = lane & 15;
+    uint4 x = qin[it];
+    if constexpr (QBF16) {
+      uint32_t* w = reinterpret_cast<uint32_t*>(&x);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const __nv_bfloat162 v = *reinterpret_cast<const __nv_bfloat162*>(&w[e]);
+        w[e] = pack_f16x2(__bfloat162float(v.x), __bfloat162float(v.y));
+      }
+    }
+    sts_16(sq + (c >> 3) * (kPrefixRows * 128) + sw128_chunk(r, c & 7), x);
+  }
+  // row = token, k = d; elements 16 e16 .. +15 are chunks 2 e16, 2 e16 + 1 of block e16 / 4.  V goes into the same
+  // token-major rows (two blocks of 64 head-dim elements): the second MMA reads them as an MN-major operand
+  const auto stage = [&](uint32_t to, const uint4 (&in)[4]) {
+    const uint32_t block = to + (e16 >> 2) * (kPrefixChunk * 128);
+#pragma unroll
+    for (int cc = 0; cc < 4; ++cc) {
+      const int tr = kPage * warp + 4 * cc + (lane >> 3);  // token row of the chunk
+      uint4 lo, hi;
+      cvt16_e4m3_f16(in[cc], lo, hi);
+      sts_16(block + sw128_chunk(tr, (2 * e16) & 7), lo);
+      sts_16(block + sw128_chunk(tr, (2 * e16 + 1) & 7), hi);
+    }
+  };
+  stage(sk, kin);
+  // generic-proxy writes -> visible to the tensor core's (async proxy) reads
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  tc_fence_before_sync();
+  dense_sync();
+  tc_fence_after_sync();
+  const uint32_t tmem = *tslot_ptr;
+  prefix_mark(pp, 1);  // query and K staged
+
+  // ---- S = Q K^T : M 128, N 256, K 128 = 2 k-blocks x 4 slices of 16
+  if (t == 0) {
+    const uint32_t idesc = umma_idesc_f16(128, 256);
+#pragma unroll
+    for (int kb = 0; kb < 2; ++kb)
+#pragma unroll
+      for (int s = 0; s < 4; ++s)
+        umma_f16(tmem, umma_desc_k_sw128(sq + kb * (kPrefixRows * 128) + 32 * s),
+                 umma_desc_k_sw128(sk + kb * (kPrefixChunk * 128) + 32 * s), idesc, (kb | s) ? 1u : 0u);
+    umma_commit(bars);
+  }
+  stage(sv, vin);  // (published by the barrier in front of the second product)
+  // this thread's own row (TMEM lane) of the tile, for the stores of its maximum and sum; and, in lanes 0..7, the
+  // workspace rows that this warp stores
+  const float ks = p.k_scale_ph ? p.k_scale_ph[kvh] : p.k_scale;
+  const float vs = p.v_scale_ph ? p.v_scale_ph[kvh] : p.v_scale;
+  const auto workspace_row = [&](int r) -> int64_t {  // of row r of the tile, -1: no such row
+    const int rg = tile.mtile * kPrefixRows + r;
+    const int req = rg / p.group;
+    if (req >= n_req) return -1;
+    const int rb = tile.req_list != nullptr ? tile.req_list[req] : req;
+    return (int64_t)rb * p.partial_stride_b + (int64_t)(kvh * p.group + rg - req * p.group) * p.partial_stride_h +
+           (int64_t)chunk * p.partial_stride_s;
+  };
+  const int64_t store_row = workspace_row(8 * warp + (lane & 7));
+  const float scale_log2 = ks * p.sm_scale * kLog2e;
+  bool ok = mbar_wait_bounded(bars, parity, pp.wait_limit_ns);
+  tc_fence_after_sync();
+  prefix_mark(pp, 2);  // S ready
+
+  // ---- softmax: thread (row, cg) holds the row's scores of tokens [64 cg, 64 cg + 64)
+  const uint32_t lane_addr = tmem + ((uint32_t)(qd * 32) << 16);  // this warp's 32 TMEM lanes
+  const int n_live = tok_hi - tok_lo;
+  float sc[64];
+  {
+    uint32_t r0[32], r1[32];
+    tmem_ld32_nowait(lane_addr + 64 * cg, r0);
+    tmem_ld32_nowait(lane_addr + 64 * cg + 32, r1);
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+    for (int e = 0; e < 32; ++e) { sc[e] = __uint_as_float(r0[e]); sc[32 + e] = __uint_as_float(r1[e]); }
+  }
+  if (64 * cg + 64 > n_live) {  // the last chunk of a prefix
+#pragma unroll
+    for (int e = 0; e < 64; ++e)
+      if (64 * cg + e >= n_live) sc[e] = -INFINITY;
+  }
+  float mx = -INFINITY, mx2 = -INFINITY;
+#pragma unroll
+  for (int e = 0; e < 64; e += 2) { mx = fmaxf(mx, sc[e]); mx2 = fmaxf(mx2, sc[e + 1]); }
+  red[cg * 128 + row] = fmaxf(mx, mx2);
+  dense_sync();
+  mx = fmaxf(fmaxf(red[row], red[128 + row]), fmaxf(red[256 + row], red[384 + row])) * scale_log2;  // scale > 0
+  float lsum[2] = {0.f, 0.f};
+  const auto exponentials = [&](auto ragged) {
+#pragma unroll
+    for (int e8 = 0; e8 < 8; ++e8) {
+      uint4 out;
+      uint32_t* w = reinterpret_cast<uint32_t*>(&out);
+#pragma unroll
+      for (int e = 0; e < 8; e += 2) {
+        float pr[2];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          pr[h] = exp2f(fmaf(sc[8 * e8 + e + h], scale_log2, -mx));
+          if constexpr (decltype(ragged)::value)
+            if (64 * cg + 8 * e8 + e + h >= n_live) pr[h] = 0.f;
+          lsum[h] += pr[h];
+        }
+        w[e >> 1] = pack_f16x2(pr[0], pr[1]);
+      }
+      // P: row = row, k = token 64 cg + 8 e8 ..: chunk e8 of k-block cg
+      sts_16(sk + cg * (kPrefixRows * 128) + sw128_chunk(row, e8), out);
+    }
+  };
+  if (64 * cg + 64 > n_live) exponentials(std::true_type{});
+  else exponentials(std::false_type{});
+  red[512 + cg * 128 + row] = lsum[0] + lsum[1];
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  tc_fence_before_sync();
+  dense_sync();
+  tc_fence_after_sync();
+  prefix_mark(pp, 3);  // P written
+
+  // ---- O = P V : M 128, N 128, K 256 = 16 slices of 16 tokens.  A = P (K-major: 4 k-blocks of
+  // 64 tokens), B = V (MN-major: 16 tokens = two 1 KiB atoms, d blocks 32 KiB apart)
+  if (t == 0) {
+    const uint32_t idesc = umma_idesc_f16(128, 128, true);
+#pragma unroll
+    for (int s = 0; s < 16; ++s)
+      umma_f16(tmem + 256, umma_desc_k_sw128(sk + (s >> 2) * (kPrefixRows * 128) + 32 * (s & 3)),
+               umma_desc_mn_sw128(sv + 2048 * s, kPrefixChunk * 128), idesc, s ? 1u : 0u);
+    umma_commit(bars + 8);
+  }
+  if (cg == 0) {
+    const int64_t r = workspace_row(row);
+    if (r >= 0) {
+      p.partial_max[r] = mx * kLn2;
+      p.partial_sum[r] = (red[512 + row] + red[640 + row]) + (red[768 + row] + red[896 + row]);
+    }
+  }
+  ok = mbar_wait_bounded(bars + 8, parity, pp.wait_limit_ns) && ok;
+  tc_fence_after_sync();
+  prefix_mark(pp, 4);  // O ready
+
+  // ---- the rows into slot `chunk` of the workspace.  Thread (row, cg) parks columns [32 cg, +32) of its row
+  // in shared memory (16-byte chunks XOR-swizzled by the row); then every warp writes whole rows, 32 lanes
+  // x 16 bytes = one contiguous 512-byte row per store.
+  {
+    float v[32];
+    tmem_ld32(lane_addr + 256 + 32 * cg, v);
+#pragma unroll
+    for (int c = 0; c < 8; ++c)
+      sts_16(sk + row * 512 + (((8 * cg + c) ^ (row & 31)) << 4),
+             make_uint4(__float_as_uint(v[4 * c] * vs), __float_as_uint(v[4 * c + 1] * vs),
+                        __float_as_uint(v[4 * c + 2] * vs), __float_as_uint(v[4 * c + 3] * vs)));
+    dense_sync();
+#pragma unroll
+    for (int r = 0; r < 8; ++r) {
+      const int orow = warp * 8 + r;
+      const int64_t to = __shfl_sync(0xffffffffu, (long long)store_row, r);
+      if (to >= 0) {
+        const uint4 x = lds_16(sk + orow * 512 + ((lane ^ (orow & 31)) << 4));
+        reinterpret_cast<uint4*>(reinterpret_cast<float*>(p.partial_output) + to * D)[lane] = x;
+      }
+    }
+  }
+  prefix_mark(pp, 5);  // stored
+  // the next tile's staging overwrites what the stores above read, and its MMAs the accumulators
+  tc_fence_before_sync();
+  dense_sync();
+  tc_fence_after_sync();
+  return ok;
+}
+
 // grid = (prefix chunks, 128-row tiles, kv heads), block = 512 threads, 1 CTA per SM
-// (grouped form: see PrefixParams).
-// Warp w works on TMEM lanes (= rows) 32 * (w % 4) .. +31, the only ones it may address, and on
-// column group w / 4 of whatever is being read: with 16 warps the staging, the softmax and the
-// stores around the two MMAs are spread over all four schedulers four warps deep.
+// (grouped form: see PrefixParams).  For calls that the kernel of shared_prefix_fused.cuh does not take.
 // SLIM caps the kernel at 80 registers per thread (128 otherwise; the cap costs about 1 us of the
 // pass).  Registers are handed out per SM sub-partition (16 K each): four warps of this CTA at 80
 // registers leave 6144 there, one warp of up to 192 registers -- the two-warp instantiation of
@@ -189,33 +441,24 @@ __device__ __forceinline__ void prefix_mark(const PrefixParams& pp, int k) {
 template <bool QBF16, bool SLIM>
 __global__ void __maxnreg__(SLIM ? 80 : 128)
 shared_prefix_dense_kernel(const KernelParams p, const PrefixParams pp) {
-  constexpr int D = 128;
-  constexpr uint32_t kQBytes = kPrefixRows * D * 2;         // 32 KiB: 2 k-blocks of [128][64]
-  constexpr uint32_t kKBytes = kPrefixChunk * D * 2;        // 64 KiB: 2 k-blocks of [256][64]; later P: 4 x [128][64]; later O rows
-  constexpr uint32_t kVBytes = D * kPrefixChunk * 2;        // 64 KiB: 2 d-blocks of [256 tokens][64]
   int chunk = blockIdx.x, mtile = blockIdx.y;
   int kvh = blockIdx.z;
-  const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
-  const int qd = warp & 3, cg = warp >> 2;  // TMEM lane quarter, column group
-  const int row = 32 * qd + lane;           // this thread's (request, head) row of the tile
+  const int t = threadIdx.x, warp = t >> 5;
   pdl_launch_dependents();
   prefix_mark(pp, 0);
 
   extern __shared__ uint8_t smem_raw[];
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
-  const uint32_t sq = base, sk = base + kQBytes, sv = sk + kKBytes;
-  const uint32_t bars = sv + kVBytes;       // two mbarriers
-  const uint32_t tslot = bars + 16;         // TMEM base address written by tcgen05.alloc
+  const uint32_t bars = base + DenseLayout::kBytes;  // two mbarriers
+  const uint32_t tslot = bars + 16;                  // TMEM base address written by tcgen05.alloc
   uint8_t* gen = smem_raw + (base - smem_u32(smem_raw));
-  volatile uint32_t* tslot_ptr = reinterpret_cast<volatile uint32_t*>(gen + kQBytes + kKBytes + kVBytes + 16);
-  float* red = reinterpret_cast<float*>(gen + kQBytes + kKBytes + kVBytes + 32);  // [2][4][128] row partials
+  const volatile uint32_t* tslot_ptr = reinterpret_cast<volatile uint32_t*>(gen + DenseLayout::kBytes + 16);
 
   // Grouped form: the grid has as many tile slots as the rows of the batch fill; the groups'
   // ragged last tiles can make a few more, which the CTAs of the first slots take in a second
   // turn (tiles done so far = `turns`, the parity the two mbarriers are waited on).  The other
   // form has one tile per CTA.
   int turns = 0;
-  uint32_t tmem = 0;
   bool ok = true;
   for (int slot0 = blockIdx.y;; slot0 += gridDim.y) {
     // Which requests, which prefix: the whole batch and pp.prefix_len, or one group of the table.
@@ -275,201 +518,13 @@ shared_prefix_dense_kernel(const KernelParams p, const PrefixParams pp) {
       }
       if (warp == 0) tmem_alloc(tslot, 512);
     }
-    const uint32_t parity = turns & 1;
-    const int tok_lo = chunk * kPrefixChunk;
-    const int tok_hi = min(tok_lo + kPrefixChunk, prefix_len);
-
-    // ---- K and V chunk: warp w stages page w of the chunk (16 tokens); per load instruction its
-    // lanes cover four whole 128-byte token rows (lane = 8 * token + 16-byte group), so every
-    // sector that is fetched is used at once -- with the whole-SM shared-memory carve-out the L1
-    // is too small to keep half-used lines until the thread's next load comes back for them
-    const int e16 = lane & 7;
-    uint4 kin[4], vin[4];
-    {
-      const bool live = tok_lo + kPage * warp < tok_hi;  // (the prefix ends on a page boundary)
-      int64_t phys = 0;
-      if (live) phys = page_of(p.block_table, p.bt_stride_b, page_row, tok_lo / kPage + warp);
-      const uint8_t* kpage = p.key_cache + phys * p.k_stride_page + (int64_t)kvh * p.k_stride_head;
-      const uint8_t* vpage = p.value_cache + phys * p.v_stride_page + (int64_t)kvh * p.v_stride_head;
-#pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        const int tp = 4 * c + (lane >> 3);  // token of the page
-        kin[c] = vin[c] = make_uint4(0u, 0u, 0u, 0u);
-        if (live) {
-          kin[c] = __ldg(reinterpret_cast<const uint4*>(kpage + (int64_t)tp * p.k_stride_token) + e16);
-          vin[c] = __ldg(reinterpret_cast<const uint4*>(vpage + (int64_t)tp * p.v_stride_token) + e16);
-        }
-      }
-    }
-    // ---- Q tile.  This thread's own row (TMEM lane) of the tile, for the softmax and the stores:
-    const int row_g = mtile * kPrefixRows + row;
-    const int head = row_g % p.group;
-    const bool row_live = row_g / p.group < n_req;
-    const int b = !row_live ? 0 : (req_list != nullptr ? __ldg(req_list + row_g / p.group) : row_g / p.group);
-    // Staging: warp w takes rows 8w .. 8w+7, two whole 256-byte rows per load instruction
-    // (lane = 16 * row + 16-byte chunk), fully used sectors as for K and V.
-#pragma unroll
-    for (int it = 0; it < 4; ++it) {
-      const int r = 8 * warp + 2 * it + (lane >> 4), c = lane & 15;
-      const int rg = mtile * kPrefixRows + r;
-      const int req = rg / p.group;
-      uint4 x = make_uint4(0u, 0u, 0u, 0u);
-      if (req < n_req) {
-        const int rb = req_list != nullptr ? __ldg(req_list + req) : req;
-        const uint16_t* q = reinterpret_cast<const uint16_t*>(p.query) + (int64_t)rb * p.q_stride_b +
-                            (int64_t)(kvh * p.group + rg % p.group) * p.q_stride_h;
-        x = __ldg(reinterpret_cast<const uint4*>(q) + c);
-      }
-      if constexpr (QBF16) {
-        uint32_t* w = reinterpret_cast<uint32_t*>(&x);
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const __nv_bfloat162 v = *reinterpret_cast<const __nv_bfloat162*>(&w[e]);
-          w[e] = pack_f16x2(__bfloat162float(v.x), __bfloat162float(v.y));
-        }
-      }
-      sts_16(sq + (c >> 3) * (kPrefixRows * 128) + sw128_chunk(r, c & 7), x);
-    }
-#pragma unroll
-    for (int cc = 0; cc < 4; ++cc) {  // 16 bytes = 16 head-dim elements at a time
-      const int tr = kPage * warp + 4 * cc + (lane >> 3);  // token row of the chunk
-      const int c = e16;
-      uint4 lo, hi;
-      cvt16_e4m3_f16(kin[cc], lo, hi);
-      // K: row = token, k = d; elements 16c .. 16c+15 are chunks 2c, 2c+1 of k-block (c / 4)
-      const uint32_t kb = sk + (c >> 2) * (kPrefixChunk * 128);
-      sts_16(kb + sw128_chunk(tr, (2 * c) & 7), lo);
-      sts_16(kb + sw128_chunk(tr, (2 * c + 1) & 7), hi);
-      // V: the same token-major rows (two blocks of 64 head-dim elements); the second MMA reads
-      // them as an MN-major operand, so no transposition is needed
-      cvt16_e4m3_f16(vin[cc], lo, hi);
-      const uint32_t vb = sv + (c >> 2) * (kPrefixChunk * 128);
-      sts_16(vb + sw128_chunk(tr, (2 * c) & 7), lo);
-      sts_16(vb + sw128_chunk(tr, (2 * c + 1) & 7), hi);
-    }
-    // generic-proxy writes -> visible to the tensor core's (async proxy) reads
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    tc_fence_before_sync();
-    __syncthreads();
-    tc_fence_after_sync();
-    tmem = *tslot_ptr;
-    prefix_mark(pp, 1);  // operands staged
-
-    // ---- S = Q K^T : M 128, N 256, K 128 = 2 k-blocks x 4 slices of 16
-    if (t == 0) {
-      const uint32_t idesc = umma_idesc_f16(128, 256);
-#pragma unroll
-      for (int kb = 0; kb < 2; ++kb)
-#pragma unroll
-        for (int s = 0; s < 4; ++s)
-          umma_f16(tmem, umma_desc_k_sw128(sq + kb * (kPrefixRows * 128) + 32 * s),
-                   umma_desc_k_sw128(sk + kb * (kPrefixChunk * 128) + 32 * s), idesc, (kb | s) ? 1u : 0u);
-      umma_commit(bars);
-    }
-    ok = mbar_wait_bounded(bars, parity, pp.wait_limit_ns) && ok;
-    tc_fence_after_sync();
-    prefix_mark(pp, 2);  // S ready
-
-    // ---- softmax: thread (row, cg) holds the row's scores of tokens [64 cg, 64 cg + 64)
-    const float ks = p.k_scale_ph ? __ldg(p.k_scale_ph + kvh) : p.k_scale;
-    const float vs = p.v_scale_ph ? __ldg(p.v_scale_ph + kvh) : p.v_scale;
-    const float scale_log2 = ks * p.sm_scale * kLog2e;
-    const uint32_t lane_addr = tmem + ((uint32_t)(qd * 32) << 16);  // this warp's 32 TMEM lanes
-    const int n_live = tok_hi - tok_lo;
-    float sc[64];
-    {
-      uint32_t r0[32], r1[32];
-      tmem_ld32_nowait(lane_addr + 64 * cg, r0);
-      tmem_ld32_nowait(lane_addr + 64 * cg + 32, r1);
-      asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-      for (int e = 0; e < 32; ++e) { sc[e] = __uint_as_float(r0[e]); sc[32 + e] = __uint_as_float(r1[e]); }
-    }
-    float mx = -INFINITY;
-#pragma unroll
-    for (int e = 0; e < 64; ++e)
-      if (64 * cg + e < n_live) mx = fmaxf(mx, sc[e]);
-    red[cg * 128 + row] = mx;
-    __syncthreads();
-    mx = fmaxf(fmaxf(red[row], red[128 + row]), fmaxf(red[256 + row], red[384 + row])) * scale_log2;  // scale > 0
-    float lsum = 0.f;
-#pragma unroll
-    for (int e8 = 0; e8 < 8; ++e8) {
-      uint4 out;
-      uint32_t* w = reinterpret_cast<uint32_t*>(&out);
-#pragma unroll
-      for (int e = 0; e < 8; e += 2) {
-        const int i0 = 8 * e8 + e;
-        const float p0 = (64 * cg + i0 < n_live) ? exp2f(sc[i0] * scale_log2 - mx) : 0.f;
-        const float p1 = (64 * cg + i0 + 1 < n_live) ? exp2f(sc[i0 + 1] * scale_log2 - mx) : 0.f;
-        lsum += p0 + p1;
-        w[e >> 1] = pack_f16x2(p0, p1);
-      }
-      // P: row = row, k = token 64 cg + 8 e8 ..: chunk e8 of k-block cg
-      sts_16(sk + cg * (kPrefixRows * 128) + sw128_chunk(row, e8), out);
-    }
-    red[512 + cg * 128 + row] = lsum;
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    tc_fence_before_sync();
-    __syncthreads();
-    tc_fence_after_sync();
-    lsum = red[512 + row] + red[640 + row] + red[768 + row] + red[896 + row];
-
-    prefix_mark(pp, 3);  // P written
-    // ---- O = P V : M 128, N 128, K 256 = 16 slices of 16 tokens.  A = P (K-major: 4 k-blocks of
-    // 64 tokens), B = V (MN-major: 16 tokens = two 1 KiB atoms, d blocks 32 KiB apart)
-    if (t == 0) {
-      const uint32_t idesc = umma_idesc_f16(128, 128, true);
-#pragma unroll
-      for (int s = 0; s < 16; ++s)
-        umma_f16(tmem + 256, umma_desc_k_sw128(sk + (s >> 2) * (kPrefixRows * 128) + 32 * (s & 3)),
-                 umma_desc_mn_sw128(sv + 2048 * s, kPrefixChunk * 128), idesc, s ? 1u : 0u);
-      umma_commit(bars + 8);
-    }
-    ok = mbar_wait_bounded(bars + 8, parity, pp.wait_limit_ns) && ok;
-    tc_fence_after_sync();
-    prefix_mark(pp, 4);  // O ready
-
-    // ---- (o, m, l) of the rows into slot `chunk` of the workspace.  Thread (row, cg) parks
-    // columns [32 cg, +32) of its row in shared memory (16-byte chunks XOR-swizzled by the row);
-    // then every warp writes whole rows, 32 lanes x 16 bytes = one contiguous 512-byte row per store.
-    {
-      float v[32];
-      tmem_ld32(lane_addr + 256 + 32 * cg, v);
-#pragma unroll
-      for (int c = 0; c < 8; ++c)
-        sts_16(sk + row * 512 + (((8 * cg + c) ^ (row & 31)) << 4),
-               make_uint4(__float_as_uint(v[4 * c] * vs), __float_as_uint(v[4 * c + 1] * vs),
-                          __float_as_uint(v[4 * c + 2] * vs), __float_as_uint(v[4 * c + 3] * vs)));
-      if (row_live && cg == 0) {
-        const int64_t pidx = (int64_t)b * p.partial_stride_b + (int64_t)(kvh * p.group + head) * p.partial_stride_h +
-                             (int64_t)chunk * p.partial_stride_s;
-        p.partial_max[pidx] = mx * kLn2;
-        p.partial_sum[pidx] = lsum;
-      }
-      __syncthreads();
-      for (int r = 0; r < 8; ++r) {
-        const int orow = warp * 8 + r;
-        const int rg = mtile * kPrefixRows + orow;
-        const int rh = rg % p.group;
-        if (rg / p.group >= n_req) break;
-        const int rb = req_list != nullptr ? __ldg(req_list + rg / p.group) : rg / p.group;
-        const uint4 x = lds_16(sk + orow * 512 + ((lane ^ (orow & 31)) << 4));
-        const int64_t pidx = (int64_t)rb * p.partial_stride_b + (int64_t)(kvh * p.group + rh) * p.partial_stride_h +
-                             (int64_t)chunk * p.partial_stride_s;
-        reinterpret_cast<uint4*>(reinterpret_cast<float*>(p.partial_output) + pidx * D)[lane] = x;
-      }
-    }
-    prefix_mark(pp, 5);  // stored
+    const PrefixTile tile{kvh, chunk, mtile, prefix_len, n_req, page_row, req_list};
+    ok = dense_tile<QBF16>(p, pp, tile, gen, base, bars, tslot_ptr, turns & 1) && ok;
     ++turns;
-    // the next tile's staging overwrites what the stores above read, and its MMAs the accumulators
-    tc_fence_before_sync();
-    __syncthreads();
-    tc_fence_after_sync();
   }
   if (turns == 0) return;
   if (!ok && t == 0) atomicExch(pp.status, kErrUmmaTimeout);
-  if (warp == 0) tmem_dealloc(tmem, 512);
+  if (warp == 0) tmem_dealloc(*tslot_ptr, 512);
 }
 
 }  // namespace pfd
