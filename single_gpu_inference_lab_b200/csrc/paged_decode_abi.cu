@@ -526,11 +526,28 @@ int launch_fused(const pfd_decode_args& a, const pfd::KernelParams& kp, const Fu
   return check_launch("fused shared-prefix kernel");
 }
 
-// Calls that the fused kernel takes.
-bool fused_eligible(const pfd_decode_args& a, int prefix_chunks) {
+// Calls that the fused kernel takes.  Its four warps per SM for the requests' own tokens have the dense tiles' time
+// for them: some 9.5 us a round of tiles, against 2.5 us and 1.2 us a page pair of the longest piece, or of the
+// average warp's share.  Where the own tokens take clearly longer, the split-KV kernel's twelve warps per SM
+// behind the dense pass win, and its splits are shared by four warps each.  The host knows bounds only: requests
+// have half of theirs on average, and in groups behind unequal prefixes all of them fewer.  us, fused / two
+// kernels, three layers, 16 + 2 heads, batch x prefix + own tokens up to:
+//   64 x 4096 + 1024: 57.4 / 61.5   128 x 4096 + 1024: 104 / 127   128 x 8192 + 512: 145 / 178   16 x 8192 + 1024: 49.5 / 50.4
+//   40 x 4096 + 1000 (grouped): 68.2 / 71.6   90 x 5120 .. 7680 + 512, 30 in none: 172 / 219
+//   64 x 256 + 2048: 75.0 / 52.4   64 x 2048 + 2560: 105 / 76.7   16 x 256 + 8192: 70.4 / 51.7   128 x 1024 + 4096: 191 / 123
+//   64 x 512 + 4000, 30 in none: 155 / 101   24 x 1024 + 16000, 8 in none: 152 / 129
+bool fused_eligible(const pfd_decode_args& a, int prefix_chunks, int num_splits, int own_bound, bool grouped) {
   if (prefix_chunks <= 0 || a.head_dim != 128 || !tma_eligible(a)) return false;
   if (g_suffix_form.load(std::memory_order_relaxed) >= 0) return false;  // a form of the two-kernel passes is asked for
-  return a.num_q_heads / a.num_kv_heads <= 8 && a.batch <= pfd::kGroupedMaxBatch;
+  const int group = a.num_q_heads / a.num_kv_heads;
+  if (group > 8 || a.batch > pfd::kGroupedMaxBatch) return false;
+  const int64_t sms = t_device->sms;
+  const int64_t tiles = ((int64_t)a.batch * group + pfd::kPrefixRows - 1) / pfd::kPrefixRows * prefix_chunks * a.num_kv_heads;
+  const int64_t rounds = (tiles + sms - 1) / sms;
+  const int64_t pairs = ((int64_t)own_bound + 31) / 32;
+  const double longest = static_cast<double>((pairs + num_splits - 1) / num_splits) * (grouped ? 0.5 : 1.0);
+  const double share = 0.5 * static_cast<double>(a.batch * pairs * a.num_kv_heads) / static_cast<double>(pfd::kFusedSuffixWarps * sms);
+  return 2.5 + 1.2 * std::max(longest, share) <= 12.4 * static_cast<double>(rounds);
 }
 
 template <int D, bool QBF16>
@@ -1036,12 +1053,13 @@ int pfd_shared_prefix_decode_fp8_e4m3(const pfd_decode_args* args, int32_t prefi
                   chunks + ns);
   }
   if (int rc = enter_call()) return rc;
-  if (fused_eligible(a, chunks)) {
+  const int span = a.max_seq_len - prefix_len;
+  const int num_splits = span > 0 ? (span + a.split_size - 1) / a.split_size : 1;
+  if (fused_eligible(a, chunks, num_splits, span, false)) {
     const FusedPrefix fused{prefix_len, nullptr, 0};
     return decode_impl(&a, chunks, nullptr, &fused);
   }
-  const int span = a.max_seq_len - prefix_len;
-  const bool beside = suffix_beside_prefix(a, chunks, span > 0 ? (span + a.split_size - 1) / a.split_size : 1, false);
+  const bool beside = suffix_beside_prefix(a, chunks, num_splits, false);
   if (int rc = bf16 ? launch_prefix<true>(a, prefix_len, chunks, beside) : launch_prefix<false>(a, prefix_len, chunks, beside))
     return rc;
   return decode_impl(&a, chunks);
@@ -1101,7 +1119,7 @@ int pfd_shared_prefix_decode_grouped_fp8_e4m3(const pfd_decode_args* args, const
   a.plan = nullptr;
   if (int rc = enter_call()) return rc;
   const int32_t* g = static_cast<const int32_t*>(groups);
-  if (fused_eligible(a, chunks)) {
+  if (fused_eligible(a, chunks, ns, suffix, true)) {
     GroupedRows rows;
     rows.row_kv_start = g + pfd::groups_row_prefix_off();
     rows.row_kv_cap = cap;

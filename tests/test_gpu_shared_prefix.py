@@ -525,23 +525,23 @@ def test_the_forced_suffix_form_is_the_one_that_runs(cabi, suffix_form, form):
     assert in_front.all() if form == 1 else not in_front[:, :, 0].any()
 
 
-@pytest.mark.parametrize("batch,hq,hkv,members,own,split,hnd", [
-    (70, 16, 2, 33, (0, 1, 31, 32, 33, 63, 64, 65, 66, 96, 97, 127, 128), 128, False),  # ends of pages, pairs and pieces
-    (70, 8, 1, 64, (0, 1, 600, 1055, 1056, 1057, 1100), 1104, False),  # one piece of more than sixteen pairs (two fetches of page ids)
-    (300, 32, 8, 290, (40, 300, 301), 64, True),  # more pieces than warps, and more tiles than CTAs; head-major pages
-    (24, 28, 4, 10, (5, 90), 64, False),  # seven heads to a kv head: rows of the last tile missing
-    (100, 16, 2, 9, (17, 33), 48, False),  # eleven groups: more than are looked up at once
+@pytest.mark.parametrize("batch,hq,hkv,members,base,own,split,hnd", [
+    (70, 16, 2, 33, 272, (0, 1, 31, 32, 33, 63, 64, 65, 66, 96, 97, 127, 128), 128, False),  # ends of pages, pairs and pieces
+    (66, 32, 4, 64, 5120, (0, 1, 600, 1055, 1056, 1057, 1100), 1104, False),  # one piece of more than sixteen pairs (two fetches of page ids)
+    (300, 32, 8, 290, 272, (40, 200, 201), 64, True),  # more pieces than warps, and more tiles than CTAs; head-major pages
+    (24, 28, 4, 10, 272, (5, 90), 64, False),  # seven heads to a kv head: rows of the last tile missing
+    (100, 16, 2, 9, 272, (17, 33), 48, False),  # eleven groups: more than are looked up at once
 ])
-def test_fused_kernel_at_the_ends_of_pieces_tiles_and_groups(cabi, batch, hq, hkv, members, own, split, hnd):
-    """Groups of `members` requests behind prefixes of 272 (one chunk and a page) + 16 g tokens, the rest in none; own
-    tokens as listed in turn."""
+def test_fused_kernel_at_the_ends_of_pieces_tiles_and_groups(cabi, batch, hq, hkv, members, base, own, split, hnd):
+    """Groups of `members` requests behind prefixes of `base` (272: one chunk and a page) + 16 g tokens, the rest in
+    none; own tokens as listed in turn."""
     from single_gpu_inference_lab_b200.workloads import quantize_per_head
 
     gen = torch.Generator().manual_seed(batch)
     pages, d, n_groups = 2500, 128, batch // members
     kc, ks = quantize_per_head(torch.randn(pages, 16, hkv, d, generator=gen))
     vc, vs = quantize_per_head(torch.randn(pages, 16, hkv, d, generator=gen))
-    prefix = [272 + 16 * g for g in range(n_groups)]
+    prefix = [base + 16 * g for g in range(n_groups)]
     lens = torch.tensor([(prefix[r // members] if r < n_groups * members else 0) + own[r % len(own)] for r in range(batch)], dtype=torch.int32)
     table = torch.randint(0, pages, (batch, -(-int(lens.max()) // 16)), generator=gen, dtype=torch.int32)
     for g in range(n_groups):
@@ -562,9 +562,10 @@ def test_fused_kernel_at_the_ends_of_pieces_tiles_and_groups(cabi, batch, hq, hk
     ws = tuple(torch.full(s, float("nan"), device=DEV) for s in ((batch, hq, slots, d), (batch, hq, slots), (batch, hq, slots)))
     for step in range(2):
         out = torch.full_like(gq, float("nan"))
+        before = cabi.launch_count()
         cabi.shared_prefix_decode_grouped_fp8_e4m3(
             gq, gkc, gvc, gt, gl, groups=groups, max_groups=max_groups, max_prefix_len=max(prefix), max_suffix_len=max(own),
             k_scale=gks, v_scale=gvs, max_seq_len=int(lens.max()), split_size=split, output=out, workspace=ws)
         torch.cuda.synchronize()
-        assert cabi.device_status() == 0
+        assert cabi.device_status() == 0 and cabi.launch_count() - before == 2  # (the fused kernel and the merge)
         assert_within_gate(out, exp, f"step {step}")
