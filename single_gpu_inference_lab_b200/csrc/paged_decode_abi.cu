@@ -324,8 +324,11 @@ constexpr int kChunkMaxBatch = 2048;
 constexpr int kChunkStages16 = 2;
 constexpr int kChunkWarps16 = 6;
 // Half page pairs charged for starting a sequence.  Measured on the batch-256 configuration
-// (us per step): 0 -> 53.9, 1 -> 44.2, 2 -> 43.0, 3 -> 43.3, 4 -> 44.0; the batch-64 one does not care.
-constexpr int kChunkPieceCost = 2;
+// (us per step): 0 -> 53.9, 1 -> 44.2, 2 -> 43.0, 3 -> 43.3, 4 -> 44.0; the batch-64 one does not care.  A pair costs
+// less since its copies are issued with fewer instructions; us a call at 2 / 3 / 4: 256 ragged sequences without a
+// plan 51.0 / 50.7 / 50.8, 16-bit caches, batch 64 34.1 / 33.6 / 33.4, head_dim 64, batch 256 36.9 / 36.6 / 36.6, a
+// recorded step of eight layers, batch 64 150.9 / 151.2 / 152.9.
+constexpr int kChunkPieceCost = 3;
 
 // Pieces are stored 16 bytes at a time and packed rows 8: the fixed-split grid, which may not need the workspace and
 // stores packed rows by element, takes calls whose buffers are aligned less.
@@ -443,10 +446,11 @@ int launch_balanced(const pfd_decode_args& a, const pfd::KernelParams& kp, int s
   {
     // Few rows mean few, long sequences whose pieces are many: four warps then share a row,
     // which also puts more loads in flight per SM (64 registers, 8 CTAs per SM).  Many rows: one
-    // warp per row, up to 16 pieces requested in one round trip (128 registers, 4 CTAs per SM):
+    // warp per row, up to 11 pieces requested in one round trip (96 registers, 5 CTAs per SM):
     // most rows of a large batch have nothing to merge and leave at once, and the few long
     // sequences that were cut into a dozen pieces set the tail -- 44.9 -> 43.0 us per step on the
-    // batch-256 configuration against 8 pieces per round at 8 CTAs per SM.
+    // batch-256 configuration with 16 pieces (4 CTAs per SM) against 8 pieces per round at 8 CTAs per SM.  A call of 256
+    // ragged sequences without a plan, at pieces (CTAs): 8 (8) 52.1 us, 10 (6) 51.3, 12 (5, spills) 50.2, 16 (4) 50.7, 11 (5) 49.5.
     // (CTAs of a single warp and row, all resident beside the chunk kernel, were measured
     // slower: 21.8 against 19.9 us per step on the batch-64 configuration.)
     const int rows = a.batch * a.num_q_heads;
@@ -464,7 +468,7 @@ int launch_balanced(const pfd_decode_args& a, const pfd::KernelParams& kp, int s
     cfg.numAttrs = 1;
     const cudaError_t e =
         wide ? cudaLaunchKernelEx(&cfg, pfd::paged_decode_chunk_merge_kernel<QBF16, 4, 4, 8, D>, kp, tp, cp)
-             : cudaLaunchKernelEx(&cfg, pfd::paged_decode_chunk_merge_kernel<QBF16, 1, 16, 4, D>, kp, tp, cp);
+             : cudaLaunchKernelEx(&cfg, pfd::paged_decode_chunk_merge_kernel<QBF16, 1, 11, 5, D>, kp, tp, cp);
     if (e != cudaSuccess) return fail(PFD_ERR_CUDA, "balanced merge kernel launch failed: %s", cudaGetErrorString(e));
   }
   return check_launch("balanced merge kernel");
@@ -678,7 +682,6 @@ pfd::KernelParams fill_params(const pfd_decode_args& a, int group, bool direct_o
   kp.batch = a.batch;
   kp.early_metadata = (a.flags & PFD_FLAG_EARLY_METADATA) ? 1 : 0;
   kp.early_kv = (kp.early_metadata && (a.flags & PFD_FLAG_EARLY_KV)) ? 1 : 0;
-  kp.kv_evict_first = 1;
   if (a.exchange != nullptr) {
     const pfd_exchange& x = *a.exchange;
     kp.xch_world = x.world;

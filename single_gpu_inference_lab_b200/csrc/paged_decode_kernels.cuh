@@ -76,7 +76,6 @@ struct KernelParams {
   int32_t fused_splits;
   int32_t early_metadata;  // 1: seq_lens and block_table may be read before the preceding kernel has completed
   int32_t early_kv;        // 1: so may K/V pages, except each sequence's last (balanced kernel with a plan)
-  int32_t kv_evict_first;  // 1: K/V tiles are loaded with the L2 evict-first hint
   // KV-range exchange (xch_world > 0): the packed (o, m, l) rows of this rank go, instead of to
   // packed_output, into slot xch_rank of every rank's receive buffer [2][world][rows][kXchRow]
   // (8-byte words) with plain stores over NVLink.  Every word carries its value in the low and
@@ -668,16 +667,7 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint32_t bar, uint32_t parity,
   return false;
 }
 // 4-D tiled TMA load of one (page, kv head) tile: CTA-local destination, every CTA issues its own copies.
-__device__ __forceinline__ void tma_load_tile(uint32_t dst, const void* tmap, uint32_t bar, int c1,
-                                              int c2, int c3) {
-  asm volatile(
-      "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes "
-      "[%0], [%1, {%3, %4, %5, %6}], [%2];"
-      ::"r"(dst), "l"(reinterpret_cast<uint64_t>(tmap)), "r"(bar), "r"(0), "r"(c1), "r"(c2), "r"(c3)
-      : "memory");
-}
-
-// The same load with an L2 eviction-priority hint.  K/V bytes are read once per step: marked
+// With an L2 eviction-priority hint: K/V bytes are read once per step: marked
 // evict-first they do not push the step's small reused data (query rows, block table, the
 // partial results the merge kernel reads back) out of L2.
 __device__ __forceinline__ uint64_t l2_policy_evict_first() {
@@ -694,15 +684,7 @@ __device__ __forceinline__ void tma_load_tile(uint32_t dst, const void* tmap, ui
       : "memory");
 }
 
-// The same two loads with an explicit innermost coordinate (in elements of the tensor map).
-__device__ __forceinline__ void tma_load_tile_x(uint32_t dst, const void* tmap, uint32_t bar, int x, int c1,
-                                                int c2, int c3) {
-  asm volatile(
-      "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes "
-      "[%0], [%1, {%3, %4, %5, %6}], [%2];"
-      ::"r"(dst), "l"(reinterpret_cast<uint64_t>(tmap)), "r"(bar), "r"(x), "r"(c1), "r"(c2), "r"(c3)
-      : "memory");
-}
+// The same load with an explicit innermost coordinate (in elements of the tensor map).
 __device__ __forceinline__ void tma_load_tile_x(uint32_t dst, const void* tmap, uint32_t bar, int x, int c1,
                                                 int c2, int c3, uint64_t policy) {
   asm volatile(
@@ -959,21 +941,12 @@ paged_decode_fp8_partial_tma_kernel(const KernelParams p, const TmaParams tp,
     mbar_expect_tx(bar, two ? kStageBytes : kStageBytes / 2);
     const int c1 = tp.head_is_dim1 ? kvh : 0;
     const int c2 = tp.head_is_dim1 ? 0 : kvh;
-    if (p.kv_evict_first) {
-      const uint64_t pol = l2_policy_evict_first();
-      tma_load_tile(dst, &tmap_k, bar, c1, c2, phys0, pol);
-      tma_load_tile(dst + 2 * kTileBytes, &tmap_v, bar, c1, c2, phys0, pol);
-      if (two) {
-        tma_load_tile(dst + kTileBytes, &tmap_k, bar, c1, c2, phys1, pol);
-        tma_load_tile(dst + 3 * kTileBytes, &tmap_v, bar, c1, c2, phys1, pol);
-      }
-    } else {
-      tma_load_tile(dst, &tmap_k, bar, c1, c2, phys0);
-      tma_load_tile(dst + 2 * kTileBytes, &tmap_v, bar, c1, c2, phys0);
-      if (two) {
-        tma_load_tile(dst + kTileBytes, &tmap_k, bar, c1, c2, phys1);
-        tma_load_tile(dst + 3 * kTileBytes, &tmap_v, bar, c1, c2, phys1);
-      }
+    const uint64_t pol = l2_policy_evict_first();
+    tma_load_tile(dst, &tmap_k, bar, c1, c2, phys0, pol);
+    tma_load_tile(dst + 2 * kTileBytes, &tmap_v, bar, c1, c2, phys0, pol);
+    if (two) {
+      tma_load_tile(dst + kTileBytes, &tmap_k, bar, c1, c2, phys1, pol);
+      tma_load_tile(dst + 3 * kTileBytes, &tmap_v, bar, c1, c2, phys1, pol);
     }
   };
 #pragma unroll

@@ -115,7 +115,8 @@ __device__ __forceinline__ void suffix_pieces(const KernelParams& p, const TmaPa
   int before = 0, total = 0, incl = 0;
   OwnTokens own{};
   SuffixCut cut{};
-  int issued_before = 0;  // page pairs that went through this warp's ring
+  int s = 0, parity = 0;  // the ring's next stage, and its barrier's phase
+  const uint64_t policy = l2_policy_evict_first();
   bool ok = true;
 #pragma unroll 1
   for (int turn = 0; ok; ++turn) {
@@ -160,26 +161,24 @@ __device__ __forceinline__ void suffix_pieces(const KernelParams& p, const TmaPa
     };
     int32_t ids = fetch(0), ids_next = n > 16 ? fetch(16) : -1;
     int ids_base = 0;
-    const auto fire = [&](int t) {  // all lanes call; lane 0 issues
+    const auto fire = [&](int t, int s) {  // pair t into stage s; all lanes call, lane 0 issues
       const int32_t phys0 = __shfl_sync(0xffffffffu, ids, (2 * (t - ids_base)) & 31);
       const int32_t phys1 = __shfl_sync(0xffffffffu, ids, (2 * (t - ids_base) + 1) & 31);
       if (lane == 0) {
-        const int s = (issued_before + t) % kFusedStages;
         const uint32_t bar = my_bars + 8 * s, dst = my_ring + s * kFusedStage;
         mbar_expect_tx(bar, phys1 >= 0 ? kFusedStage : kFusedStage / 2);
         const int c1 = tp.head_is_dim1 ? kvh : 0, c2 = tp.head_is_dim1 ? 0 : kvh;
-        const uint64_t pol = l2_policy_evict_first();
-        tma_load_tile(dst, &tmap_k, bar, c1, c2, phys0, pol);
-        tma_load_tile(dst + 2 * kPage * D, &tmap_v, bar, c1, c2, phys0, pol);
+        tma_load_tile(dst, &tmap_k, bar, c1, c2, phys0, policy);
+        tma_load_tile(dst + 2 * kPage * D, &tmap_v, bar, c1, c2, phys0, policy);
         if (phys1 >= 0) {
-          tma_load_tile(dst + kPage * D, &tmap_k, bar, c1, c2, phys1, pol);
-          tma_load_tile(dst + 3 * kPage * D, &tmap_v, bar, c1, c2, phys1, pol);
+          tma_load_tile(dst + kPage * D, &tmap_k, bar, c1, c2, phys1, policy);
+          tma_load_tile(dst + 3 * kPage * D, &tmap_v, bar, c1, c2, phys1, policy);
         }
       }
     };
 #pragma unroll
     for (int t = 0; t < kFusedStages; ++t)
-      if (t < n) fire(t);
+      if (t < n) fire(t, (s + t) % kFusedStages);
 
     const float ks = p.k_scale_ph ? p.k_scale_ph[kvh] : p.k_scale;
     const float vs = p.v_scale_ph ? p.v_scale_ph[kvh] : p.v_scale;
@@ -194,8 +193,7 @@ __device__ __forceinline__ void suffix_pieces(const KernelParams& p, const TmaPa
     int t = 0;
 #pragma unroll 1
     for (; t < n; ++t) {
-      const int s = (issued_before + t) % kFusedStages;
-      if (!mbar_wait_bounded(my_bars + 8 * s, ((issued_before + t) / kFusedStages) & 1, tp.wait_limit_ns)) { ok = false; break; }
+      if (!mbar_wait_bounded(my_bars + 8 * s, parity, tp.wait_limit_ns)) { ok = false; break; }
       bal_step<1, D>(st, my_ring + s * kFusedStage, k_off, v_off, qb, fabsf(scale_signed), lo + t * 2 * kPage, lo, hi, i, j);
       __syncwarp();  // all reads of the stage fed MMAs above: hand it back to TMA
       const int tn = t + kFusedStages;
@@ -206,19 +204,21 @@ __device__ __forceinline__ void suffix_pieces(const KernelParams& p, const TmaPa
           ids_next = fetch(tn + 16);
         }
         if (lane == 0) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        fire(tn);
+        fire(tn, s);
       }
+      if (++s == kFusedStages) { s = 0; parity ^= 1; }
     }
     if (!ok) {
       // a copy never landed: record it; give the copies still in flight a bounded chance to land
       if (lane == 0) {
         atomicExch(tp.status, kErrTmaTimeout);
-        for (int u = t + 1; u < min(n, t + kFusedStages); ++u)
-          mbar_wait_bounded(my_bars + 8 * ((issued_before + u) % kFusedStages), ((issued_before + u) / kFusedStages) & 1, tp.wait_limit_ns);
+        for (int u = t + 1; u < min(n, t + kFusedStages); ++u) {
+          if (++s == kFusedStages) { s = 0; parity ^= 1; }
+          mbar_wait_bounded(my_bars + 8 * s, parity, tp.wait_limit_ns);
+        }
       }
       break;
     }
-    issued_before += n;
     if (lane == 0) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the next piece's copies reuse the ring
 #pragma unroll
     for (int c = 0; c < 2; ++c) {
