@@ -147,6 +147,7 @@ __device__ __forceinline__ int split_size_of(const KernelParams& p, int kv0) {
 // and the slots of their pieces: behind the prefix chunks' slots, or all of the row's.
 struct OwnTokens {
   int kv0, live, slot0, slots;
+  bool cut_off;  // the request has more tokens than the caller's bounds say
 };
 __device__ __forceinline__ OwnTokens own_tokens(const KernelParams& p, int b) {
   OwnTokens x;
@@ -155,9 +156,9 @@ __device__ __forceinline__ OwnTokens own_tokens(const KernelParams& p, int b) {
   const bool alone = p.row_kv_start != nullptr && x.kv0 == 0;
   x.slot0 = alone ? 0 : p.slot_offset;
   x.slots = alone ? p.slot_offset + p.fused_splits : p.fused_splits;
-  // (no further than the caller's bounds, which the block table covers)
-  const int64_t most = alone ? (int64_t)p.bt_cols * kPage : (int64_t)p.fused_splits * p.split_size;
-  x.live = (int)min((int64_t)max(p.seq_lens[b] - x.kv0, 0), most);
+  const int seq_len = p.seq_lens[b];
+  x.live = own_length(seq_len, x.kv0, p.bt_cols, alone ? 0 : p.fused_splits, p.split_size);
+  x.cut_off = seq_len - x.kv0 > x.live;
   return x;
 }
 __device__ __forceinline__ SuffixCut own_cut(const OwnTokens& x) {

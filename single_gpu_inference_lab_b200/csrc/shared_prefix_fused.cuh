@@ -131,6 +131,8 @@ __device__ __forceinline__ void suffix_pieces(const KernelParams& p, const TmaPa
       const int r = (round < in_none ? round : round - in_none) * 32 + lane;
       if (r < B) {
         own = own_tokens(p, r);
+        // a request that has more tokens than the caller's bounds say is reported, not silently cut
+        if (own.cut_off && first == 0 && p.row_kv_start != nullptr) atomicExch(tp.status, kErrSuffixBound);
         if (in_none == 0 || (own.kv0 == 0) == (round < in_none)) cut = own_cut(own);
       }
       incl = cut.pieces;
@@ -150,8 +152,6 @@ __device__ __forceinline__ void suffix_pieces(const KernelParams& p, const TmaPa
     const int slot = __shfl_sync(0xffffffffu, own.slot0, at) + part;
     const int lo = kv0 + part * pairs * 2 * kPage;
     const int hi = min(lo + pairs * 2 * kPage, end);
-    // a request that has more tokens than the caller's bound says is reported, not silently cut
-    if (part == 0 && kvh == 0 && lane == 0 && p.row_kv_start != nullptr && p.seq_lens[b] > end) atomicExch(tp.status, kErrSuffixBound);
 
     const int page_first = lo / kPage, page_last = (hi - 1) / kPage;
     const int n = (page_last - page_first + 2) / 2;
