@@ -530,28 +530,22 @@ int launch_fused(const pfd_decode_args& a, const pfd::KernelParams& kp, const Fu
   return check_launch("fused shared-prefix kernel");
 }
 
-// Calls that the fused kernel takes.  Its four warps per SM for the requests' own tokens have the dense tiles' time
-// for them: some 9.5 us a round of tiles, against 2.5 us and 1.2 us a page pair of the longest piece, or of the
-// average warp's share.  Where the own tokens take clearly longer, the split-KV kernel's twelve warps per SM
-// behind the dense pass win, and its splits are shared by four warps each.  The host knows bounds only: requests
-// have half of theirs on average, and in groups behind unequal prefixes all of them fewer.  us, fused / two
-// kernels, three layers, 16 + 2 heads, batch x prefix + own tokens up to:
-//   64 x 4096 + 1024: 57.4 / 61.5   128 x 4096 + 1024: 104 / 127   128 x 8192 + 512: 145 / 178   16 x 8192 + 1024: 49.5 / 50.4
-//   40 x 4096 + 1000 (grouped): 68.2 / 71.6   90 x 5120 .. 7680 + 512, 30 in none: 172 / 219
-//   64 x 256 + 2048: 75.0 / 52.4   64 x 2048 + 2560: 105 / 76.7   16 x 256 + 8192: 70.4 / 51.7   128 x 1024 + 4096: 191 / 123
-//   64 x 512 + 4000, 30 in none: 155 / 101   24 x 1024 + 16000, 8 in none: 152 / 129
+// Calls that the fused kernel can take, and is faster on (fused_pays).
 bool fused_eligible(const pfd_decode_args& a, int prefix_chunks, int num_splits, int own_bound, bool grouped) {
   if (prefix_chunks <= 0 || a.head_dim != 128 || !tma_eligible(a)) return false;
   if (g_suffix_form.load(std::memory_order_relaxed) >= 0) return false;  // a form of the two-kernel passes is asked for
   const int group = a.num_q_heads / a.num_kv_heads;
   if (group > 8 || a.batch > pfd::kGroupedMaxBatch) return false;
-  const int64_t sms = t_device->sms;
-  const int64_t tiles = ((int64_t)a.batch * group + pfd::kPrefixRows - 1) / pfd::kPrefixRows * prefix_chunks * a.num_kv_heads;
-  const int64_t rounds = (tiles + sms - 1) / sms;
-  const int64_t pairs = ((int64_t)own_bound + 31) / 32;
-  const double longest = static_cast<double>((pairs + num_splits - 1) / num_splits) * (grouped ? 0.5 : 1.0);
-  const double share = 0.5 * static_cast<double>(a.batch * pairs * a.num_kv_heads) / static_cast<double>(pfd::kFusedSuffixWarps * sms);
-  return 2.5 + 1.2 * std::max(longest, share) <= 12.4 * static_cast<double>(rounds);
+  pfd::FusedShape s{};
+  s.batch = a.batch;
+  s.group = group;
+  s.kv_heads = a.num_kv_heads;
+  s.chunks = prefix_chunks;
+  s.slots = num_splits;
+  s.own = own_bound;
+  s.alone = grouped && !(a.flags & PFD_FLAG_ALL_IN_GROUPS) ? a.max_seq_len : 0;
+  s.grouped = grouped;
+  return pfd::fused_pays(s, t_device->sms);
 }
 
 template <int D, bool QBF16>

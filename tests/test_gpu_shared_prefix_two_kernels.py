@@ -1,0 +1,83 @@
+"""Grouped shared-prefix decode by the dense pass and the split-KV pass behind it: what the fused kernel does not take by
+itself, or is told not to.  The launches of a call (2 with the fused kernel, 3 without) pin which one ran."""
+
+import pytest
+import torch
+
+from oracle import paged_decode_oracle as oracle
+
+from helpers import assert_within_gate
+
+pytestmark = pytest.mark.gpu
+
+DEV = "cuda:0"
+
+
+class Counted:
+    """The binding, with the launches of each grouped decode written down."""
+
+    def __init__(self, cabi):
+        self._cabi, self.launches = cabi, []
+
+    def __getattr__(self, name):
+        return getattr(self._cabi, name)
+
+    def shared_prefix_decode_grouped_fp8_e4m3(self, *args, **kw):
+        before = self._cabi.launch_count()
+        self._cabi.shared_prefix_decode_grouped_fp8_e4m3(*args, **kw)
+        self.launches.append(self._cabi.launch_count() - before)
+
+
+@pytest.fixture(scope="module")
+def cabi(built_libs):
+    from single_gpu_inference_lab_b200 import cabi as module
+
+    module.load()
+    return module
+
+
+def _decode(counted, batch, hq, hkv, groups_of, prefix, own, split, alone, flags=0):
+    """Groups of `groups_of` requests behind `prefix` + 16 g tokens, the rest in none with the lengths `alone`, in turn; own
+    tokens of the members as listed in turn."""
+    from single_gpu_inference_lab_b200.workloads import quantize_per_head
+
+    gen = torch.Generator().manual_seed(batch + hq)
+    pages, d, n_groups = 2500, 128, batch // groups_of
+    if flags == 0 and alone is not None:
+        n_groups = min(n_groups, (batch - 1) // groups_of)
+    kc, ks = quantize_per_head(torch.randn(pages, 16, hkv, d, generator=gen))
+    vc, vs = quantize_per_head(torch.randn(pages, 16, hkv, d, generator=gen))
+    of = [prefix + 16 * (r // groups_of) if r < n_groups * groups_of else 0 for r in range(batch)]
+    lens = torch.tensor([of[r] + own[r % len(own)] if of[r] else alone[r % len(alone)] for r in range(batch)], dtype=torch.int32)
+    longest = int(lens.max())
+    table = torch.randint(0, pages, (batch, -(-longest // 16)), generator=gen, dtype=torch.int32)
+    for g in range(n_groups):
+        shared = of[g * groups_of] // 16
+        table[g * groups_of:(g + 1) * groups_of, :shared] = table[g * groups_of, :shared]
+    q = torch.randn(batch, hq, d, generator=gen).to(torch.bfloat16)
+    exp = oracle.reference(q, kc, vc, table.long(), lens, ks, vs)
+    gq, gkc, gvc, gt, gl, gks, gvs = (t.to(DEV) for t in (q, kc, vc, table, lens, ks, vs))
+    groups, max_groups = counted.group_shared_prefixes(gt, prefix_lengths=torch.tensor(of, dtype=torch.int32, device=DEV),
+                                                       min_batch=groups_of, min_prefix_len=256, max_groups=n_groups)
+    torch.cuda.synchronize()
+    assert groups[3:5].tolist() == [n_groups, n_groups * groups_of]
+    cap = max(of)
+    slots = -(-cap // 256) + -(-max(own) // split)
+    ws = tuple(torch.full(s, float("nan"), device=DEV) for s in ((batch, hq, slots, d), (batch, hq, slots), (batch, hq, slots)))
+    for step in range(2):
+        out = torch.full_like(gq, float("nan"))
+        counted.shared_prefix_decode_grouped_fp8_e4m3(
+            gq, gkc, gvc, gt, gl, groups=groups, max_groups=max_groups, max_prefix_len=cap, max_suffix_len=max(own),
+            k_scale=gks, v_scale=gvs, max_seq_len=longest, split_size=split, output=out, workspace=ws, flags=flags)
+        torch.cuda.synchronize()
+        assert counted.device_status() == 0
+        assert_within_gate(out, exp, f"step {step}")
+
+
+@pytest.mark.parametrize("hinted", [False, True])
+def test_a_long_context_in_no_group_sends_the_call_to_the_two_kernels(cabi, hinted):
+    """One request of 6000 tokens beside 23 behind a short prefix: three launches, two if the caller (mistakenly, here) says that
+    every request is in a group; the same result."""
+    counted = Counted(cabi)
+    _decode(counted, 24, 16, 2, 23, 272, (5, 60), 64, (6000,), cabi.PFD_FLAG_ALL_IN_GROUPS if hinted else 0)
+    assert counted.launches == ([2, 2] if hinted else [3, 3])
