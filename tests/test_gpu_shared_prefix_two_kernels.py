@@ -4,6 +4,7 @@ itself, or is told not to.  The launches of a call (2 with the fused kernel, 3 w
 import pytest
 import torch
 
+import test_gpu_shared_prefix as base
 from oracle import paged_decode_oracle as oracle
 
 from helpers import assert_within_gate
@@ -36,6 +37,14 @@ def cabi(built_libs):
     return module
 
 
+@pytest.fixture
+def two_kernels(cabi):
+    """The split-KV pass behind the dense pass, whatever the library would choose; the choice is restored."""
+    cabi.set_suffix_form(0)
+    yield Counted(cabi)
+    cabi.set_suffix_form(-1)
+
+
 def _decode(counted, batch, hq, hkv, groups_of, prefix, own, split, alone, flags=0):
     """Groups of `groups_of` requests behind `prefix` + 16 g tokens, the rest in none with the lengths `alone`, in turn; own
     tokens of the members as listed in turn."""
@@ -43,8 +52,6 @@ def _decode(counted, batch, hq, hkv, groups_of, prefix, own, split, alone, flags
 
     gen = torch.Generator().manual_seed(batch + hq)
     pages, d, n_groups = 2500, 128, batch // groups_of
-    if flags == 0 and alone is not None:
-        n_groups = min(n_groups, (batch - 1) // groups_of)
     kc, ks = quantize_per_head(torch.randn(pages, 16, hkv, d, generator=gen))
     vc, vs = quantize_per_head(torch.randn(pages, 16, hkv, d, generator=gen))
     of = [prefix + 16 * (r // groups_of) if r < n_groups * groups_of else 0 for r in range(batch)]
@@ -81,3 +88,31 @@ def test_a_long_context_in_no_group_sends_the_call_to_the_two_kernels(cabi, hint
     counted = Counted(cabi)
     _decode(counted, 24, 16, 2, 23, 272, (5, 60), 64, (6000,), cabi.PFD_FLAG_ALL_IN_GROUPS if hinted else 0)
     assert counted.launches == ([2, 2] if hinted else [3, 3])
+
+
+@pytest.mark.parametrize("shape", [
+    (150, 16, 2, 8, 1500, 40),    # many requests in none: the scan takes two rounds, items are taken in several turns
+    (12, 32, 8, 8, 4000, 16),     # a few long ones: as many splits as their slots allow
+    (40, 8, 8, 0, 700, 100),      # no group at all
+    (16, 28, 4, 15, 900, 300),    # one request in none
+])
+def test_requests_in_no_group_on_the_two_kernels(two_kernels, shape):
+    base.test_requests_in_no_group_have_ctas_of_their_own(two_kernels, *shape)
+    assert two_kernels.launches == [3, 3]
+
+
+@pytest.mark.parametrize("hint", [False, True])
+def test_more_tiles_than_tile_slots_on_the_two_kernels(two_kernels, hint):
+    base.test_grouped_decode_with_more_tiles_than_tile_slots(two_kernels, hint)
+    assert two_kernels.launches == [3, 3]
+
+
+@pytest.mark.parametrize("batch,hq,hkv,groups_of,prefix,own,split,alone", [
+    (64, 32, 2, 17, 2304, (1, 64, 100), 64, (2400, 1, 300)),  # 16 heads: nine row tiles for eight slots, the ninth in a second turn
+    (100, 24, 2, 9, 272, (17, 33), 48, (500,)),               # 12 heads, eleven groups: more than are looked up at once
+    (30, 18, 2, 29, 256, (3, 90), 64, (257,)),                # 9 heads: rows of one request in two tiles
+])
+def test_more_heads_than_the_fused_kernel_takes(cabi, batch, hq, hkv, groups_of, prefix, own, split, alone):
+    counted = Counted(cabi)
+    _decode(counted, batch, hq, hkv, groups_of, prefix, own, split, alone)
+    assert counted.launches == [3, 3]
