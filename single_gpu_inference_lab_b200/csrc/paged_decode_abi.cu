@@ -325,10 +325,10 @@ constexpr int kChunkStages16 = 2;
 constexpr int kChunkWarps16 = 6;
 // Half page pairs charged for starting a sequence.  Measured on the batch-256 configuration
 // (us per step): 0 -> 53.9, 1 -> 44.2, 2 -> 43.0, 3 -> 43.3, 4 -> 44.0; the batch-64 one does not care.  A pair costs
-// less since its copies are issued with fewer instructions; us a call at 2 / 3 / 4: 256 ragged sequences without a
-// plan 51.0 / 50.7 / 50.8, 16-bit caches, batch 64 34.1 / 33.6 / 33.4, head_dim 64, batch 256 36.9 / 36.6 / 36.6, a
-// recorded step of eight layers, batch 64 150.9 / 151.2 / 152.9.
-constexpr int kChunkPieceCost = 3;
+// less since its copies are issued with fewer instructions, which does not tell 2 from 3 (us a pass at 2 / 3: head_dim 64,
+// batch 256 35.6 / 35.3; 16-bit caches, batch 64 33.9 / 33.6; 256 ragged sequences without a plan 48.8 / 48.9; recorded
+// steps, batch 64, eight layers 150.4 / 152.0, two with the producer 50.3 / 50.9).
+constexpr int kChunkPieceCost = 2;
 
 // Pieces are stored 16 bytes at a time and packed rows 8: the fixed-split grid, which may not need the workspace and
 // stores packed rows by element, takes calls whose buffers are aligned less.
