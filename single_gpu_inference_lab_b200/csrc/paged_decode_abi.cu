@@ -504,17 +504,8 @@ int launch_fused(const pfd_decode_args& a, const pfd::KernelParams& kp, const Fu
   pp.wait_limit_ns = tp.wait_limit_ns;
   pp.phase_times = g_phase_times;
   auto kernel = pfd::shared_prefix_fused_kernel<QBF16>;
-  static std::atomic<bool> configured[kMaxDevices], checked[kMaxDevices];
+  static std::atomic<bool> configured[kMaxDevices];
   if (int rc = configure_smem(configured, kernel, pfd::kFusedSmem)) return rc;
-  if (!checked[t_device->dev].load(std::memory_order_acquire)) {
-    // the warps' register shares add up to what the block is launched with, or the second half would wait for ever
-    cudaFuncAttributes attr;
-    const cudaError_t e = cudaFuncGetAttributes(&attr, kernel);
-    if (e != cudaSuccess) return fail(PFD_ERR_CUDA, "cudaFuncGetAttributes failed: %s", cudaGetErrorString(e));
-    if ((attr.numRegs + 7) / 8 * 8 != pfd::kFusedRegs)
-      return fail(PFD_ERR_CUDA, "fused shared-prefix kernel built with %d registers a thread, not %d", attr.numRegs, pfd::kFusedRegs);
-    checked[t_device->dev].store(true, std::memory_order_release);
-  }
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(t_device->sms);
   cfg.blockDim = dim3(pfd::kFusedThreads);
@@ -530,7 +521,22 @@ int launch_fused(const pfd_decode_args& a, const pfd::KernelParams& kp, const Fu
   return check_launch("fused shared-prefix kernel");
 }
 
-// Calls that the fused kernel can take, and is faster on (fused_pays).
+// Registers a thread that the fused kernel was built with, looked up once per device; 0: not known.
+template <bool QBF16>
+int fused_registers() {
+  static std::atomic<int> known[kMaxDevices];
+  std::atomic<int>& regs = known[t_device->dev];
+  if (regs.load(std::memory_order_relaxed) == 0) {
+    cudaFuncAttributes attr;
+    if (cudaFuncGetAttributes(&attr, pfd::shared_prefix_fused_kernel<QBF16>) == cudaSuccess)
+      regs.store(attr.numRegs, std::memory_order_relaxed);
+    else
+      (void)cudaGetLastError();  // (the two kernels take the call)
+  }
+  return regs.load(std::memory_order_relaxed);
+}
+
+// Calls that the fused kernel can take, and is faster on (fused_takes).
 bool fused_eligible(const pfd_decode_args& a, int prefix_chunks, int num_splits, int own_bound, bool grouped) {
   if (prefix_chunks <= 0 || a.head_dim != 128 || !tma_eligible(a)) return false;
   if (g_suffix_form.load(std::memory_order_relaxed) >= 0) return false;  // a form of the two-kernel passes is asked for
@@ -545,7 +551,7 @@ bool fused_eligible(const pfd_decode_args& a, int prefix_chunks, int num_splits,
   s.own = own_bound;
   s.alone = grouped && !(a.flags & PFD_FLAG_ALL_IN_GROUPS) ? a.max_seq_len : 0;
   s.grouped = grouped;
-  return pfd::fused_pays(s, t_device->sms);
+  return pfd::fused_takes(s, t_device->sms, a.query_dtype == PFD_DTYPE_BF16 ? fused_registers<true>() : fused_registers<false>());
 }
 
 template <int D, bool QBF16>

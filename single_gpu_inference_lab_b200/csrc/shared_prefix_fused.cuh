@@ -23,7 +23,6 @@ namespace pfd {
 constexpr int kFusedSuffixWarps = 4;
 constexpr int kFusedStages = 2;
 constexpr int kFusedThreads = kDenseThreads + 32 * kFusedSuffixWarps;
-constexpr int kFusedRegs = 96;  // a thread at launch (see above)
 constexpr uint32_t kFusedStage = 4 * kPage * 128;
 constexpr int kFusedSmem = 1024 + DenseLayout::kBytes + kFusedSuffixWarps * kFusedStages * (kFusedStage + 8) + 32;
 

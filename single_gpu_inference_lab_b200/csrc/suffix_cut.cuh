@@ -66,6 +66,15 @@ inline bool fused_pays(const FusedShape& s, int64_t sms) {
   return 2.8 * turns + 1.2 * longest + share <= allowed && 1.35 * alone <= allowed;
 }
 
+// Registers a thread that a block of the fused kernel is launched with.  Its warps hand them from one another
+// (shared_prefix_fused.cuh): launched with any other number the ones that want more would wait for ever.
+constexpr int kFusedRegs = 96;
+
+// Calls that the fused kernel takes, if the compiler gave it `built_regs` registers a thread.
+inline bool fused_takes(const FusedShape& s, int64_t sms, int built_regs) {
+  return (built_regs + 7) / 8 * 8 == kFusedRegs && fused_pays(s, sms);
+}
+
 // Own tokens of a request of `seq_len` tokens that attends from `kv0` on, all behind its prefix (`splits` > 0: as many
 // splits of `split_size`, the caller's bound on them) or its whole context (`splits` 0); never past the `cols` pages that a
 // row of the block table is known to have.  Less than it has: a broken bound, which the caller of this reports.
