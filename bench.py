@@ -62,6 +62,10 @@ ALL_WORKLOADS = ("qwen2.5-0.5b-b8", "qwen2.5-coder-3b-b64", "qwen2.5-7b-b256", "
 KERNEL_NAMES = {1: "paged_decode_fp8_partial_ldg_kernel", 2: "paged_decode_fp8_partial_tma_kernel",
                 3: "paged_decode_fp8_chunk_kernel", 4: "paged_decode_fp8_chunk_kernel<KV16>",
                 5: "paged_decode_fp8_chunk_kernel<FUSED>", 6: "paged_decode_fp8_chunk_kernel<KV16,FUSED>"}
+# by launches: the library takes prefix and suffixes in one kernel or in two, by the shape
+SHARED_PREFIX_KERNEL_NAMES = {
+    2: "shared_prefix_fused_kernel + paged_decode_merge_kernel",
+    3: "shared_prefix_dense_kernel + paged_decode_fp8_partial_tma_kernel + paged_decode_merge_kernel"}
 
 
 def parse_args():
@@ -601,10 +605,11 @@ class Case:
                 "what": "fused RoPE + FP8 append of one new token per request (its last position), then the decode call; "
                         "the decode call's flags are the run's"}
 
-    def kernel_name(self, path: int) -> str:
+    def kernel_name(self, res: dict) -> str:
+        """Kernels of a measured step; the shared-prefix step's are told apart by how many it launched."""
         if self.shared_prefix:
-            return "shared_prefix_dense_kernel + paged_decode_fp8_partial_tma_kernel + paged_decode_merge_kernel"
-        return KERNEL_NAMES.get(path, "?")
+            return SHARED_PREFIX_KERNEL_NAMES.get(res["launches_per_step"], "?")
+        return KERNEL_NAMES.get(res["path"], "?")
 
     def release(self):
         if self.xch is not None:
@@ -622,7 +627,7 @@ def short_report(case: Case, res: dict, peak: float, world_bytes: float, world: 
     out = {
         "us_per_layer_step": round(us, 3), "kv_read_gbs": round(gbs, 1),
         "step_frac_of_hbm_peak": round(gbs / (peak * world), 4),
-        "kernel": case.kernel_name(res["path"]), "kernel_us": round(res["ms_kernel"] * 1e3, 3),
+        "kernel": case.kernel_name(res), "kernel_us": round(res["ms_kernel"] * 1e3, 3),
         "kernel_frac_of_hbm_peak": round(case.kv_bytes / (res["ms_kernel"] * 1e-3) / 1e9 / peak, 4),
         "path": case.cabi.PATH_NAMES.get(res["path"], "?"), "launches_per_step": res["launches_per_step"],
         "kv_bytes_per_step_per_gpu": case.kv_bytes, "runs_us": res["runs_us"],
@@ -878,7 +883,7 @@ def main() -> int:
 
     line = None
     if rank == 0:
-        kernel_name = case.kernel_name(res["path"])
+        kernel_name = case.kernel_name(res)
         short_kernel = kernel_name.split("<")[0] if res["path"] in KERNEL_NAMES else kernel_name
         line = {
             "metric": "decode_attn_kv_read_gbs", "value": round(value, 2), "unit": "GB/s",
