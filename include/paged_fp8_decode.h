@@ -48,11 +48,12 @@ extern "C" {
                                      on B200 than the two launches, for callers that want one node  */
 #define PFD_FLAG_ALL_IN_GROUPS 128u /* grouped shared-prefix decode: the caller has read word 4 of the
                                      groups buffer and it equals the batch, i.e. no request is outside
-                                     the groups.  The split-KV pass over the short suffixes may then
-                                     run as small CTAs beside the dense prefix pass instead of behind
-                                     it.  Only a hint about speed: with a request in no group after
-                                     all the result is the same, that request's share just takes
-                                     longer                                                         */
+                                     the groups.  The choice of kernels then looks at the suffixes
+                                     alone, not at how long a request in no group could be, and where
+                                     prefix and suffixes take a kernel each, that of the suffixes may
+                                     run as small CTAs beside the other instead of behind it.  Only a
+                                     hint about speed: with a request in no group after all the result
+                                     is the same, that request's share just takes longer             */
 #define PFD_FLAG_EARLY_KV 256u /* with PFD_FLAG_EARLY_METADATA and a plan: the caller also vouches that the
                                 kernel preceding this call in the stream writes K/V only into the LAST page of
                                 each sequence (a decode step's cache append writes one token, at position
@@ -285,15 +286,19 @@ int pfd_paged_decode_fp8_e4m3_split_out_noalloc(const pfd_decode_args* args);
  * Decode step of a batch whose requests ALL share one paged prefix: block_table[b][0 ..
  * prefix_len/16) names the same physical pages for every b (the caller checks that, e.g. with
  * the grouping of find_l20_shared_prefix_groups,
- * integrations/vllm/l20_shared_prefix_decode_dispatch.py:52-76).  Three kernels:
- *   1. dense prefix pass on tcgen05 tensor cores: 128 (request, q head) rows x 256 prefix tokens
- *      per CTA, K/V converted e4m3 -> f16 on the way into shared memory, accumulators in TMEM;
+ * integrations/vllm/l20_shared_prefix_decode_dispatch.py:52-76).  Three parts:
+ *   1. the prefix, dense on tcgen05 tensor cores: tiles of 128 (request, q head) rows x 256 prefix
+ *      tokens, K/V converted e4m3 -> f16 on the way into shared memory, accumulators in TMEM;
  *      replaces _shared_paged_prefix_gqa_partial_kernel
  *      (src/l20_stack/ops/triton_decode_attention.py:704-813);
- *   2. suffix pass: the split-KV partial kernel with kv_start = prefix_len
- *      (replaces _paged_suffix_gqa_partial_kernel, :815-912);
- *   3. the LSE merge over prefix chunks and suffix splits
+ *   2. the suffixes, split-KV (replaces _paged_suffix_gqa_partial_kernel, :815-912);
+ *   3. the LSE merge over prefix chunks and suffix pieces
  *      (replaces _prefix_suffix_gqa_reduce_kernel, :652-702).
+ * Two launches where one kernel takes parts 1 and 2 (at most 8 query heads per KV head, caches that
+ * TMA can describe, suffixes that fit into the tiles' time: pfd::fused_pays in csrc/suffix_cut.cuh),
+ * three where each part has its own.  split_size bounds the suffixes' pieces: two launches cut a
+ * suffix evenly into at most ceil((max_seq_len - prefix_len) / split_size) pieces of 64 tokens or more, three into
+ * splits of split_size.
  * Needs head_dim 128, prefix_len a multiple of 16, an f32 workspace with
  * workspace_splits >= ceil(prefix_len / 256) + ceil((max_seq_len - prefix_len) / split_size),
  * and 16-byte aligned query rows.  kv_start must be 0.
@@ -369,17 +374,18 @@ int pfd_group_shared_prefixes(const int32_t* block_table, int64_t bt_stride_b, i
  * Decode step of a batch with any number of shared-prefix groups (and requests in none), all
  * decided on the device: `groups` is the buffer pfd_group_shared_prefixes() filled for this batch
  * (same batch size, same max_groups; made once per model step, read by every layer's call).  The
- * dense tensor-core pass runs per group over the group's request list, the split-KV pass covers
+ * dense tensor-core tiles run per group over the group's request list, split-KV work covers
  * every request from the end of its group's prefix (from token 0 for a request in no group), one
- * merge.  A prefix is used up to a multiple of 16 tokens and up to min(max_prefix_len,
- * max_seq_len); what lies beyond goes through the split-KV pass, so any bound is safe and a
+ * merge; two launches or three, as above.  A prefix is used up to a multiple of 16 tokens and up to
+ * min(max_prefix_len, max_seq_len); what lies beyond is split-KV work, so any bound is safe and a
  * tight one saves idle CTAs.  Every member of a group must be at least as long as the group's
  * prefix.  max_suffix_len bounds what a request IN a group has behind its prefix (0 = unknown: the
- * whole context); the split-KV grid is sized for it, ceil(max_suffix_len / split_size) splits.  A
- * request in no group covers its whole context with as many splits as all its slots allow, of 256
- * tokens or more, taken by CTAs of their own (under PFD_FLAG_ALL_IN_GROUPS, with a cache that TMA
- * cannot describe, or beside the prefix pass by pfd_set_suffix_form(1): with as many splits as the
- * others' suffixes, longer ones).  A member whose
+ * whole context) and gives it ceil(max_suffix_len / split_size) slots for its pieces.  A request in no
+ * group has all the slots of its row, the prefix chunks' too.  In two launches its context is cut evenly into as many
+ * pieces of 64 tokens or more, one warp each; max_seq_len bounds it, so that without PFD_FLAG_ALL_IN_GROUPS a max_seq_len far
+ * above the prefixes is a reason for three launches.  In three, its splits have 256 tokens or more and
+ * CTAs of their own (under PFD_FLAG_ALL_IN_GROUPS, with a cache that TMA cannot describe, or beside the
+ * prefix pass by pfd_set_suffix_form(1): as many splits as the others' suffixes, longer ones).  A member whose
  * suffix exceeds the bound would be attended only up to it (device status 5 reports it): give a true bound (max_seq_len minus
  * the smallest prefix a group can have, i.e. the min_prefix_len of the grouping call).  The
  * workspace needs ceil(min(max_prefix_len, max_seq_len) / 256) +
@@ -419,12 +425,13 @@ int pfd_device_status(int32_t* status);
 int pfd_set_wait_limit_ns(uint64_t limit_ns);
 
 /*
- * Tuning: which form the split-KV pass of the shared-prefix entry points takes.  -1 (default):
- * chosen per call -- two-warp CTAs that run on the same SMs WHILE the dense prefix pass runs when
+ * Tuning: how the shared-prefix entry points take the tokens behind the prefix.  -1 (default):
+ * chosen per call -- in one kernel with the prefix's tiles where that is faster, else in a kernel of their own:
+ * two-warp CTAs that run on the same SMs WHILE the dense prefix pass runs when
  * the SMs that pass leaves free could not absorb the suffix work meanwhile (and, with a groups
  * table, PFD_FLAG_ALL_IN_GROUPS is set), else the ordinary four-warp CTAs, which start on those
- * free SMs and take the rest after the pass; 0: always the latter; 1: always the former.
- * Process-wide, read at launch; results do not depend on it.
+ * free SMs and take the rest after the pass; 0: always the last of these; 1: always the two-warp CTAs.
+ * Process-wide, read at launch; results depend on it by rounding alone.
  */
 int pfd_set_suffix_form(int32_t form);
 
@@ -439,7 +446,9 @@ int pfd_selftest_bounded_wait(uint64_t limit_ns, uint64_t* waited_ns, void* stre
 
 /* Which kernels the calling thread's last decode call launched. */
 #define PFD_PATH_FIXED_LDG 1 /* fixed-split grid, plain 16-byte loads, + merge kernel */
-#define PFD_PATH_FIXED_TMA 2 /* fixed-split grid, TMA pipeline, + merge kernel         */
+#define PFD_PATH_FIXED_TMA 2 /* fixed-split grid, TMA pipeline, + merge kernel; of a shared-prefix call
+                                also the kernel that takes prefix and suffixes together: two
+                                launches by pfd_launch_count(), where the grid's own are three */
 #define PFD_PATH_BALANCED 3  /* balanced persistent kernel + its merge kernel            */
 #define PFD_PATH_BALANCED_KV16 4 /* the same for 16-bit caches (pfd_paged_decode_kv16_split_out) */
 #define PFD_PATH_FUSED 5       /* balanced persistent kernel alone (PFD_FLAG_SINGLE_LAUNCH)   */

@@ -278,8 +278,8 @@ def paged_decode_kv16_split_out(query, key_cache, value_cache, block_table, seq_
 
 
 def shared_prefix_decode_fp8_e4m3(query, key_cache, value_cache, block_table, seq_lens, *, prefix_len, **kw) -> None:
-    """One layer-step through ``pfd_shared_prefix_decode_fp8_e4m3``: dense tcgen05 pass over the
-    prefix every request shares, split-KV pass over the private suffixes, one merge."""
+    """One layer-step through ``pfd_shared_prefix_decode_fp8_e4m3``: dense tcgen05 tiles over the
+    prefix every request shares, split-KV work over the private suffixes, one merge."""
     args = decode_args(query, key_cache, value_cache, block_table, seq_lens, **kw)
     lib = load()
     lib.pfd_shared_prefix_decode_fp8_e4m3.argtypes = [C.POINTER(DecodeArgs), C.c_int32]
@@ -429,8 +429,8 @@ def device_status() -> int:
 
 
 def set_suffix_form(form: int) -> None:
-    """Tuning: form of the split-KV pass behind a dense prefix pass (``pfd_set_suffix_form``):
-    -1 chosen per call, 0 always after that pass, 1 always beside it."""
+    """Tuning: how a shared-prefix call takes the tokens behind the prefix (``pfd_set_suffix_form``):
+    -1 chosen per call, among them one kernel with the prefix's tiles; 0 always after the dense pass, 1 always beside it."""
     lib = load()
     lib.pfd_set_suffix_form.argtypes = [C.c_int32]
     lib.pfd_set_suffix_form.restype = C.c_int

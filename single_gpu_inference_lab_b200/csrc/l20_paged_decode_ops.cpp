@@ -286,7 +286,7 @@ int64_t plan_bytes(int64_t batch, int64_t num_kv_heads) {
 }
 
 // Decode step of a batch whose requests all share the first prefix_len tokens' pages: dense
-// tcgen05 prefix pass + split-KV suffix pass + merge (pfd_shared_prefix_decode_fp8_e4m3).
+// tcgen05 prefix tiles, split-KV suffixes, merge (pfd_shared_prefix_decode_fp8_e4m3).
 void shared_prefix_decode_fp8_e4m3(at::Tensor query, at::Tensor key_cache, at::Tensor value_cache,
                                    at::Tensor block_table, at::Tensor seq_lens, at::Tensor partial_output,
                                    at::Tensor partial_max, at::Tensor partial_sum, at::Tensor output,

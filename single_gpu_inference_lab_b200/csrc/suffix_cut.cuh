@@ -37,33 +37,43 @@ struct FusedShape {
   bool grouped;                    // prefixes may differ, so that `own` is the shortest one's
 };
 
-// Calls that the fused kernel takes from the two kernels (the dense pass, then split-KV work behind it).  Its four warps
-// per SM for own tokens, one to a piece, have the dense tiles' time for them, where the split-KV kernel's twelve share a
-// split by four and run on SMs that have no tile.  In us: the tiles allow 9 for each round of them and 12 for the part
-// of the SMs that has one in a single round; taking a piece up costs 2.8, a page pair of the longest piece 1.2, and of
-// the average warp's share 1.0 (requests have half of their bound on average, in groups behind unequal prefixes
-// less).  Apart from that, a page pair of a request in no group costs 1.35, since the slots that bound its pieces are few where
-// its context is long.
-// Measured on 1110 shapes: 16 + 2, 28 + 4, 32 + 8, 8 + 1, 8 + 8 and 32 + 16 heads, 8 .. 256 requests, prefixes of 256 .. 8192, 16 ..
-// 2048 own tokens, up to all requests in no group, of up to 65536 tokens.  The fused kernel takes 714 of them; 46 are more than
-// 2 % slower with it and 60 of the others more than 2 % faster.  us, two kernels / fused:
-//   taken: 64 x 4096 + 512, 16 + 2 heads 17.5 / 15.6, 32 + 8 43.3 / 36.2; two groups 27.2 / 17.9, and 8 requests in none 29.9 / 20.8
-//   not taken: 64 x 1024 + 512, 8 + 8 heads 18.8 / 25.7, 32 + 8 23.1 / 27.3; 16 x 2048 + 2048, 16 + 2 16.7 / 22.1;
-//     64 x 4096 + 512 and one request in no group of 16384 tokens 23.9 / 33.2, of 65536 46.8 / 103; 4 of 4096 beside 60 x 256 + 16 26.1 / 66.3
-//   taken, and slower: how many requests are in no group only the device knows.  64 x 4096 + 512, 16 + 2 heads, 32 of them in none
-//     32.2 / 34.4, 48 37.7 / 47.4, all 51.9 / 51.6; all of 32 + 8 133 / 153 (with max_prefix_len left at max_seq_len 35.3 / 33.7,
-//     41.9 / 40.6, 53.3 / 47.4 and 147 / 153)
+// Calls that the fused kernel takes from the two kernels (the dense pass, then split-KV work behind or beside it).  In
+// us, roughly: the tiles allow its four warps per SM for own tokens 9 for each round of them and 12 for the part of the SMs
+// that has one in a single round, and the two kernels need 1.5 more for each wave of split-KV CTAs; a warp's turn costs 1, a
+// page pair of the average warp's share 1, of the longest piece 1 (0.4 in groups behind unequal prefixes, where few are
+// that long), and looking through 32 requests 0.4, twice that where the ones in no group come first.
+// Where every request has a prefix, the two kernels side by side on the same SMs are as fast while a single round of
+// tiles is all there is, or hardly any own tokens: the fused kernel takes what has more.  Where some may be in no group,
+// they run one behind the other, and a page pair of such a request costs 1.35, since the slots that bound its pieces are
+// few where its context is long.
+// Measured on 5880 shapes, each on cold caches in the form that the two kernels take by themselves: 8 + 1, 8 + 8, 16 + 2, 28 + 4,
+// 32 + 8 and 32 + 16 heads, 8 .. 256 requests, prefixes of 256 .. 8192, 16 .. 2048 own tokens, one prefix, or up to four groups
+// with none to all of the requests outside.  us, two kernels / fused:
+//   one prefix, taken: 64 x 4096 + 512, 32 + 8 heads 36.6 / 36.4; 128 x 8192 + 512, 16 + 2 50.9 / 48.4; 256 x 4096 + 128, 32 + 16 130 / 87.0
+//     not taken: 64 x 4096 + 512, 16 + 2 15.6 / 16.4; 16 x 8192 + 1024, 16 + 2 14.6 / 17.4
+//     of 2400 such shapes (and groups that hold every request) 450 are taken, 58 of them more than 2 % slower so, 318 faster
+//   two groups, 64 x 4096 + 512, 16 + 2, taken: 23.3 / 19.5, with 8 requests in none 28.2 / 23.3, with 32 34.1 / 35.6
+//     256 x 4096 + 16, 28 + 4, one group and 32 in none 107 / 92.4, two and 128 173 / 181
+//     not taken: 256 x 256 + 128, 16 + 2, 32 in none 22.8 / 25.9
+//     of 2718 with less than half of the requests in none 1020 are taken, 273 slower so, 673 faster
+//   taken, and slower: 64 x 4096 + 2048, 16 + 2, two groups and 8 requests in none 35.7 / 43.5.  How many are in none only
+//     the device knows: of 372 calls with all of them in none 137 are taken, 91 slower so, 256 x 4096 + 16, 28 + 4
+//     213 / 297 the worst
 inline bool fused_pays(const FusedShape& s, int64_t sms) {
   const auto up = [](int64_t x, int64_t by) { return (x + by - 1) / by; };
   const int64_t tiles = up(s.batch * s.group, 128) * s.chunks * s.kv_heads, warps = 4 * sms;
   const int64_t pairs = up(s.own, 32), half = pairs / (2 * kSuffixPairs);
   const int64_t pieces = half < 1 ? 1 : half < s.slots ? half : s.slots;
-  const double allowed = 9.0 * static_cast<double>(up(tiles, sms)) + 12.0 * static_cast<double>(tiles) / static_cast<double>(sms);
-  const double longest = static_cast<double>(up(pairs, s.slots)) * (s.grouped ? 0.75 : 1.0);
+  const int64_t splits = s.slots < up(pairs, kSuffixPairs) ? s.slots : up(pairs, kSuffixPairs);  // (of 64 tokens or more, as measured)
+  const double waves = static_cast<double>(s.batch * s.kv_heads * splits) / static_cast<double>(3 * sms);
+  const double allowed = 9.0 * static_cast<double>(up(tiles, sms)) + 12.0 * static_cast<double>(tiles) / static_cast<double>(sms) + 1.5 * waves;
+  const double longest = static_cast<double>(up(pairs, s.slots));
   const double share = 0.5 * static_cast<double>(s.batch * pairs * s.kv_heads) / static_cast<double>(warps);
-  const double turns = static_cast<double>(up(s.batch * s.kv_heads * pieces, warps));
+  const double scan = 0.4 * static_cast<double>(up(s.batch, 32) * (s.grouped ? 2 : 1));
+  const double own = static_cast<double>(up(s.batch * s.kv_heads * pieces, warps)) + share + scan;
+  if (s.alone == 0) return tiles > sms && share >= 0.6 && own + longest <= 0.45 * allowed;
   const double alone = static_cast<double>(up(up(s.alone, 32), s.chunks + s.slots));
-  return 2.8 * turns + 1.2 * longest + share <= allowed && 1.35 * alone <= allowed;
+  return own + 0.4 * longest <= 0.5 * allowed && (alone <= 5.0 || 1.35 * alone <= 0.5 * allowed);
 }
 
 // Registers a thread that a block of the fused kernel is launched with.  Its warps hand them from one another

@@ -104,7 +104,8 @@ def l20_decode_step(meta, query, key_cache, value_cache, block_tables, seq_lens,
     capturing = torch.cuda.is_current_stream_capturing()
     if fp8 and sw["shared_prefix"] and head_dim == 128 and MIN_GROUP_BATCH <= batch <= 2048 and max_seq_len >= MIN_PREFIX_TOKENS \
             and (not capturing or sw["shared_prefix_force"]):
-        # every group the buffer has room for costs idle CTAs in each layer's dense pass: room for a few
+        # room for a few groups: in each layer, up to eight are looked up in one round trip, and where the prefix has a
+        # kernel of its own, every group that the buffer has room for can cost it idle CTAs
         max_groups = max(1, min(batch // MIN_GROUP_BATCH, MAX_GROUPS))
         groups_buffer = _persistent(("groups", query.device, batch, max_groups), lambda: torch.empty(
             torch.ops.l20_stack.prefix_groups_bytes(batch, max_groups) // 4, dtype=torch.int32, device=query.device))

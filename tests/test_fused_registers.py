@@ -13,7 +13,7 @@ CSRC = Path(__file__).resolve().parents[1] / "single_gpu_inference_lab_b200/csrc
 SHIM = """
 #include "suffix_cut.cuh"
 extern "C" int takes(int regs, int own) {
-  return pfd::fused_takes(pfd::FusedShape{64, 8, 2, 16, 4, own, 0, false}, 148, regs);
+  return pfd::fused_takes(pfd::FusedShape{128, 8, 2, 32, 2, own, 0, false}, 148, regs);
 }
 """
 

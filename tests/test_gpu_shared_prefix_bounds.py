@@ -21,16 +21,16 @@ def cabi(built_libs):
     return module
 
 
-@pytest.mark.parametrize("grouped", [True, False])
-@pytest.mark.parametrize("max_len,member,alone", [
-    (612, 640, 700),  # within the last split, behind the last page; a request in no group behind all
-    (512, 520, 520),  # no room for any token behind the prefix
+@pytest.mark.parametrize("grouped,batch,hq,hkv,prefix,max_len,member,alone", [
+    (True, 20, 16, 2, 512, 612, 640, 700),  # within the last split, behind the last page; a request in no group behind all
+    (True, 20, 16, 2, 512, 512, 520, 520),  # no room for any token behind the prefix
+    (False, 40, 32, 4, 4096, 4324, 4350, None),
 ])
-def test_a_request_longer_than_the_bound_stays_inside_its_row(cabi, grouped, max_len, member, alone):
+def test_a_request_longer_than_the_bound_stays_inside_its_row(cabi, grouped, batch, hq, hkv, prefix, max_len, member, alone):
     from single_gpu_inference_lab_b200.workloads import quantize_per_head
 
     gen = torch.Generator().manual_seed(7)
-    batch, hq, hkv, d, pages, prefix, split = 20, 16, 2, 128, 900, 512, 64
+    d, pages, split = 128, 900, 64
     cols = -(-max_len // 16)
     kc, ks = quantize_per_head(torch.randn(pages, 16, hkv, d, generator=gen))
     vc, vs = quantize_per_head(torch.randn(pages, 16, hkv, d, generator=gen))
@@ -47,7 +47,7 @@ def test_a_request_longer_than_the_bound_stays_inside_its_row(cabi, grouped, max
     exp = oracle.reference(q, kc, vc, table.long(), lens.clamp(max=cols * 16), ks, vs)
     gq, gkc, gvc, gw, gl, gks, gvs = (t.to(DEV) for t in (q, kc, vc, wide, lens, ks, vs))
     gt = gw[:, :cols]
-    suffix = 100
+    suffix = 100 if grouped else max_len - prefix
     slots = -(-prefix // 256) + -(-suffix // split)
     ws = tuple(torch.full(s, float("nan"), device=DEV) for s in ((batch, hq, slots, d), (batch, hq, slots), (batch, hq, slots)))
     out = torch.full_like(gq, float("nan"))

@@ -83,11 +83,43 @@ def _decode(counted, batch, hq, hkv, groups_of, prefix, own, split, alone, flags
 
 @pytest.mark.parametrize("hinted", [False, True])
 def test_a_long_context_in_no_group_sends_the_call_to_the_two_kernels(cabi, hinted):
-    """One request of 6000 tokens beside 23 behind a short prefix: three launches, two if the caller (mistakenly, here) says that
+    """One request of 30000 tokens beside 39 behind a prefix: three launches, two if the caller (mistakenly, here) says that
     every request is in a group; the same result."""
     counted = Counted(cabi)
-    _decode(counted, 24, 16, 2, 23, 272, (5, 60), 64, (6000,), cabi.PFD_FLAG_ALL_IN_GROUPS if hinted else 0)
+    _decode(counted, 40, 32, 4, 39, 4096, (5, 512), 128, (30000,), cabi.PFD_FLAG_ALL_IN_GROUPS if hinted else 0)
     assert counted.launches == ([2, 2] if hinted else [3, 3])
+
+
+@pytest.mark.parametrize("batch,hq,hkv,prefix,own,split,launches", [
+    (40, 32, 4, 4096, (0, 1, 31, 32, 33, 64, 65, 512), 128, 2),   # more tiles than SMs, the last row tile of 64 rows
+    (20, 64, 8, 5136, (17, 300, 301), 304, 2),                    # a last chunk of one page, one piece to a suffix
+    (32, 16, 2, 4096, (0, 1, 31, 32, 33, 64, 65, 512), 128, 3),   # fewer tiles than SMs
+    (40, 32, 4, 4096, (0, 1, 16), 64, 3),                         # hardly any own tokens
+])
+def test_one_prefix_on_either_side_of_the_rule(cabi, batch, hq, hkv, prefix, own, split, launches):
+    from single_gpu_inference_lab_b200.workloads import quantize_per_head
+
+    gen = torch.Generator().manual_seed(batch)
+    pages, d = 1500, 128
+    kc, ks = quantize_per_head(torch.randn(pages, 16, hkv, d, generator=gen))
+    vc, vs = quantize_per_head(torch.randn(pages, 16, hkv, d, generator=gen))
+    lens = torch.tensor([prefix + own[r % len(own)] for r in range(batch)], dtype=torch.int32)
+    max_len = prefix + max(own)
+    table = torch.randint(0, pages, (batch, -(-max_len // 16)), generator=gen, dtype=torch.int32)
+    table[:, :prefix // 16] = table[0, :prefix // 16]
+    q = torch.randn(batch, hq, d, generator=gen).to(torch.bfloat16)
+    exp = oracle.reference(q, kc, vc, table.long(), lens, ks, vs)
+    gq, gkc, gvc, gt, gl, gks, gvs = (t.to(DEV) for t in (q, kc, vc, table, lens, ks, vs))
+    slots = -(-prefix // 256) + -(-max(own) // split)
+    ws = tuple(torch.full(s, float("nan"), device=DEV) for s in ((batch, hq, slots, d), (batch, hq, slots), (batch, hq, slots)))
+    for step in range(2):
+        out = torch.full_like(gq, float("nan"))
+        before = cabi.launch_count()
+        cabi.shared_prefix_decode_fp8_e4m3(gq, gkc, gvc, gt, gl, prefix_len=prefix, k_scale=gks, v_scale=gvs, max_seq_len=max_len,
+                                           split_size=split, output=out, workspace=ws)
+        torch.cuda.synchronize()
+        assert cabi.launch_count() - before == launches and cabi.device_status() == 0
+        assert_within_gate(out, exp, f"step {step}")
 
 
 @pytest.mark.parametrize("shape", [
