@@ -55,9 +55,10 @@ struct FusedShape {
 //   two groups, 64 x 4096 + 512, 16 + 2, taken: 23.3 / 19.5, with 8 requests in none 28.2 / 23.3, with 32 34.1 / 35.6
 //     256 x 4096 + 16, 28 + 4, one group and 32 in none 107 / 92.4, two and 128 173 / 181
 //     not taken: 256 x 256 + 128, 16 + 2, 32 in none 22.8 / 25.9
-//     of 2718 with less than half of the requests in none 1020 are taken, 273 slower so, 673 faster
+//     one group, 64 x 4096 + 512, 16 + 2, taken: 21.8 / 18.7
+//     of 2718 with less than half of the requests in none 1109 are taken, 282 slower so, 742 faster (0.5 instead of 0.55: 1020, 273 and 673)
 //   taken, and slower: 64 x 4096 + 2048, 16 + 2, two groups and 8 requests in none 35.7 / 43.5.  How many are in none only
-//     the device knows: of 372 calls with all of them in none 137 are taken, 91 slower so, 256 x 4096 + 16, 28 + 4
+//     the device knows: of 372 calls with all of them in none 168 are taken, 95 slower so, 256 x 4096 + 16, 28 + 4
 //     213 / 297 the worst
 inline bool fused_pays(const FusedShape& s, int64_t sms) {
   const auto up = [](int64_t x, int64_t by) { return (x + by - 1) / by; };
@@ -73,7 +74,7 @@ inline bool fused_pays(const FusedShape& s, int64_t sms) {
   const double own = static_cast<double>(up(s.batch * s.kv_heads * pieces, warps)) + share + scan;
   if (s.alone == 0) return tiles > sms && share >= 0.6 && own + longest <= 0.45 * allowed;
   const double alone = static_cast<double>(up(up(s.alone, 32), s.chunks + s.slots));
-  return own + 0.4 * longest <= 0.5 * allowed && (alone <= 5.0 || 1.35 * alone <= 0.5 * allowed);
+  return own + 0.4 * longest <= 0.5 * allowed && (alone <= 5.0 || 1.35 * alone <= 0.55 * allowed);
 }
 
 // Registers a thread that a block of the fused kernel is launched with.  Its warps hand them from one another

@@ -35,7 +35,7 @@ def pays(tmp_path_factory):
 
 
 def test_a_long_context_in_no_group_is_left_to_the_two_kernels(pays):
-    """Its slots are few and a piece is one warp's: half as long as the tiles take, no longer."""
+    """Its slots are few and a piece is one warp's: hardly more than half as long as the tiles take, no longer."""
     assert pays(64, 16, 2, 5120, 512, 128, alone=5632, grouped=True)
     for context in (16384, 32768, 131072, 2**31 - 16):
         assert not pays(64, 16, 2, 5120, 512, 128, alone=context, grouped=True)
@@ -65,6 +65,7 @@ MEASURED = [
     ((128, 8, 8, 2048, 128, 64, 0), 18.4, 21.5),
     ((128, 16, 2, 8192, 512, 256, 0), 50.9, 48.4),
     ((256, 32, 16, 4096, 128, 64, 0), 130.0, 87.0),
+    ((64, 16, 2, 4096, 512, 128, 4608), 21.8, 18.7),
     ((64, 16, 2, 5120, 512, 128, 5632), 28.2, 23.3),
     ((256, 28, 4, 4096, 16, 64, 4112), 107.0, 92.4),
     ((256, 16, 2, 320, 128, 64, 448), 22.8, 25.9),
