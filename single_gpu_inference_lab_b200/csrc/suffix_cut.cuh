@@ -90,12 +90,15 @@ inline bool fused_takes(const FusedShape& s, int64_t sms, int built_regs) {
 // splits of `split_size`, the caller's bound on them) or its whole context (`splits` 0); never past the `cols` pages that a
 // row of the block table is known to have.  Less than it has: a broken bound, which the caller of this reports.
 PFD_HOST_DEVICE int own_length(int seq_len, int kv0, int cols, int splits, int split_size) {
-  const int64_t row = static_cast<int64_t>(cols) * 16 - kv0;
-  const int64_t bound = splits > 0 ? static_cast<int64_t>(splits) * split_size : row;
-  const int64_t most = bound < row ? bound : row;
-  const int64_t has = static_cast<int64_t>(seq_len) - kv0;
-  const int64_t live = has < most ? has : most;
-  return live > 0 ? static_cast<int>(live) : 0;
+  constexpr int kMost = 0x7fffffff;  // (32 bits: every warp of the fused kernel works this out for every request)
+  const int row = cols <= kMost / 16 ? cols * 16 : kMost;
+  const int len = seq_len < 0 ? 0 : seq_len < row ? seq_len : row;
+  int live = len - kv0;
+  if (splits > 0) {
+    const int64_t bound = static_cast<int64_t>(splits) * split_size;
+    live = live < bound ? live : static_cast<int>(bound);
+  }
+  return live > 0 ? live : 0;
 }
 
 }  // namespace pfd
