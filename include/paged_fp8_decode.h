@@ -295,8 +295,8 @@ int pfd_paged_decode_fp8_e4m3_split_out_noalloc(const pfd_decode_args* args);
  *   3. the LSE merge over prefix chunks and suffix pieces
  *      (replaces _prefix_suffix_gqa_reduce_kernel, :652-702).
  * Two launches where one kernel takes parts 1 and 2 (at most 8 query heads per KV head, caches that
- * TMA can describe, suffixes that fit into the tiles' time: pfd::fused_pays in csrc/suffix_cut.cuh),
- * three where each part has its own.  split_size bounds the suffixes' pieces: two launches cut a
+ * TMA can describe, more than one round of tiles, suffixes that fit into their time: pfd::fused_pays in
+ * csrc/suffix_cut.cuh), three where each part has its own.  split_size bounds the suffixes' pieces: two launches cut a
  * suffix evenly into at most ceil((max_seq_len - prefix_len) / split_size) pieces of 64 tokens or more, three into
  * splits of split_size.
  * Needs head_dim 128, prefix_len a multiple of 16, an f32 workspace with

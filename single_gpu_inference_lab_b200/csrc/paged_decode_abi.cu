@@ -278,9 +278,9 @@ int launch_partial_tma(const pfd_decode_args& a, const pfd::KernelParams& kp, di
 // on an SM that pass leaves free -- and run while it runs.  Otherwise the ordinary four-warp CTAs
 // are launched behind the dense pass; as its programmatic dependents they start, three per SM, on
 // whatever SMs the last wave of that pass leaves free, and only what those SMs do not get done
-// while the wave runs is left for afterwards.  The small form costs the dense pass 1 us and its
-// CTAs are slow (two warps, one copy in flight each), so it is taken only when the free SMs
-// cannot absorb the suffix work.  Measured in us per step (behind / beside), 16 query and 2 KV
+// while the wave runs is left for afterwards.  The small form's CTAs are slow (two warps, one copy in flight
+// each), so it is taken only when the free SMs cannot absorb the suffix work.  Measured in us per step (behind /
+// beside) with an earlier dense tile, which was 2 us slower and another 1 us at 80 registers, 16 query and 2 KV
 // heads, prefix 4096 unless noted, suffixes up to 511 behind it (batch b = 2 b dense CTAs):
 //   batch 64, splits of 128: 19.8 / 17.4   of 256: 21.7 / 19.2   of 512: 24.6 / 24.8
 //   batch 16: 14.2 / 15.1   batch 32: 15.1 / 16.0   batch 48: 15.2 / 16.9   batch 96: 29.1 / 31.5
@@ -290,7 +290,7 @@ int launch_partial_tma(const pfd_decode_args& a, const pfd::KernelParams& kp, di
 //   batch 128 with 2048 declared (128 CTAs), splits of 512: 46.0 / 44.9
 // The estimate below (a dense wave lasts 10 us, a four-warp CTA 2 us + 1 us per page pair of each
 // warp, about 65 % of the grid has work; never with more than two dense waves, each of which
-// pays the slim kernel's 1 us) decides all of these but one as measured.  A request in
+// paid the slim kernel's 1 us) decides all of these but one as measured.  A request in
 // no group attends its whole context in as many splits as the others their suffix, which two
 // warps would take several times longer over: with a groups table the small form needs the
 // caller's word that every request is in a group (PFD_FLAG_ALL_IN_GROUPS).
@@ -842,7 +842,7 @@ int launch_prefix(const pfd_decode_args& a, int prefix_len, int chunks, bool suf
   pp.wait_limit_ns = g_wait_limit_ns.load(std::memory_order_relaxed);
   pp.phase_times = g_phase_times;
   // the slim instantiation (80 registers, whole-SM carve-out) leaves room for the suffix pass's
-  // two-warp CTAs on the same SM; it is 1 us slower by itself, so the other one runs otherwise
+  // two-warp CTAs on the same SM
   auto kernel = suffix_beside ? pfd::shared_prefix_dense_kernel<QBF16, true> : pfd::shared_prefix_dense_kernel<QBF16, false>;
   constexpr int smem = 1024 + pfd::DenseLayout::kBytes + 32;
   static std::atomic<bool> configured[2][kMaxDevices];

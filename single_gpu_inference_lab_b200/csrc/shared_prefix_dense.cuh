@@ -431,12 +431,13 @@ __device__ __forceinline__ bool dense_tile(const KernelParams& p, const PrefixPa
 
 // grid = (prefix chunks, 128-row tiles, kv heads), block = 512 threads, 1 CTA per SM
 // (grouped form: see PrefixParams).  For calls that the kernel of shared_prefix_fused.cuh does not take.
-// SLIM caps the kernel at 80 registers per thread (128 otherwise; the cap costs about 1 us of the
-// pass).  Registers are handed out per SM sub-partition (16 K each): four warps of this CTA at 80
+// SLIM caps the kernel at 80 registers per thread (128 otherwise).  With the next operands staged under the products the
+// cap costs nothing any more: 10.7 us a launch either way (64 requests, 16 + 2 heads, 4096 tokens; 8 bytes of spills
+// at 80).  Registers are handed out per SM sub-partition (16 K each): four warps of this CTA at 80
 // registers leave 6144 there, one warp of up to 192 registers -- the two-warp instantiation of
 // the suffix kernel uses 165 -- and with the largest shared-memory carve-out two 18 KB CTAs of
-// that kind fit beside the 166 KB of this one: the suffix pass then runs on the same SMs WHILE
-// this pass runs instead of after it.  (At 126 registers nothing above 32 registers per thread
+// that kind fit beside the 161 KB of this one: the suffix pass then runs on the same SMs WHILE
+// this pass runs instead of after it.  (At 128 registers nothing above 32 registers per thread
 // fits beside this CTA; without the carve-out request nothing at all, whatever the registers.)
 template <bool QBF16, bool SLIM>
 __global__ void __maxnreg__(SLIM ? 80 : 128)
