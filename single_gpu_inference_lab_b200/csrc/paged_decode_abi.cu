@@ -551,7 +551,7 @@ bool fused_eligible(const pfd_decode_args& a, int prefix_chunks, int num_splits,
   s.own = own_bound;
   s.alone = grouped && !(a.flags & PFD_FLAG_ALL_IN_GROUPS) ? a.max_seq_len : 0;
   s.grouped = grouped;
-  return pfd::fused_takes(s, t_device->sms, a.query_dtype == PFD_DTYPE_BF16 ? fused_registers<true>() : fused_registers<false>());
+  return pfd::fused_takes(s, t_device->sms, a.query_dtype == PFD_DTYPE_BF16 ? fused_registers<true> : fused_registers<false>);
 }
 
 template <int D, bool QBF16>

@@ -81,9 +81,11 @@ inline bool fused_pays(const FusedShape& s, int64_t sms) {
 // (shared_prefix_fused.cuh): launched with any other number the ones that want more would wait for ever.
 constexpr int kFusedRegs = 96;
 
-// Calls that the fused kernel takes, if the compiler gave it `built_regs` registers a thread.
-inline bool fused_takes(const FusedShape& s, int64_t sms, int built_regs) {
-  return (built_regs + 7) / 8 * 8 == kFusedRegs && fused_pays(s, sms);
+// Calls that the fused kernel takes, if the compiler gave it `built_regs()` registers a thread, which is asked only of a
+// call that would take it: the answer loads the kernel.
+template <typename Registers>
+inline bool fused_takes(const FusedShape& s, int64_t sms, Registers&& built_regs) {
+  return fused_pays(s, sms) && (built_regs() + 7) / 8 * 8 == kFusedRegs;
 }
 
 // Own tokens of a request of `seq_len` tokens that attends from `kv0` on, all behind its prefix (`splits` > 0: as many
